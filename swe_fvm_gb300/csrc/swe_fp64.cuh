@@ -6,14 +6,10 @@
 // 64 cycles, and a hardware division or square root is a chain of 7-10 of them.
 // The integer pipe issues one warp instruction per cycle.  These routines
 // compute IEEE round-to-nearest-even a / b and sqrt(x) from the 53-bit integer
-// significands, with a single-precision estimate refined by two Newton steps
-// in 128-bit fixed point and an exact remainder check, so the result equals
-// the hardware instruction bit for bit.  Operands or results that are zero,
-// subnormal, infinite or NaN take the hardware instruction.
-//
-// The methods are textbook: Newton-Raphson reciprocal and reciprocal square
-// root iterations (y' = y (2 - b y), y' = y (3 - x y^2) / 2) followed by
-// correction of the truncated quotient/root with the exact remainder.
+// significands, with a single-precision estimate, one Newton step in 32-bit
+// fixed point, two 31-bit digits and an exact remainder comparison, so the
+// result equals the hardware instruction bit for bit.  Operands or results that
+// are zero, subnormal, infinite or NaN take the hardware instruction.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -46,29 +42,25 @@ constexpr unsigned long long kHid = 1ull << 52;
 __device__ __forceinline__ unsigned long long bits(double x) { return (unsigned long long)dbits(x); }
 __device__ __forceinline__ double from_bits(unsigned long long u) { return dfrom((long long)u); }
 
-// round a 63-bit truncated significand q (value in [2^62, 2^63)) to 53 bits;
-// returns the rounded significand (may be 2^53)
-__device__ __forceinline__ unsigned long long round63(unsigned long long q, bool sticky) {
-  unsigned long long mant = q >> 10;
-  const unsigned low = (unsigned)(q & 0x3FFull);
-  const bool up = (low > 0x200u) || (low == 0x200u && (sticky || (mant & 1ull)));
-  return mant + (up ? 1ull : 0ull);
-}
-
 // The hardware instructions for the rare operands, kept out of line so that
 // the common path never issues them (predicated in-line copies would cost FP64
 // pipe slots on every call).
 static __device__ __noinline__ double ddiv_hw(double a, double b) { return __ddiv_rn(a, b); }
 static __device__ __noinline__ double dsqrt_hw(double x) { return __dsqrt_rn(x); }
 
-// 64-bit fixed-point value of a float f in (0.5, 1]: f 2^shift, from its bits
-// (integer ops only: 64-bit integer <-> float conversions issue on the FP64
-// pipe, measured)
-__device__ __forceinline__ unsigned long long fixed_from_unit_float(float f, int shift) {
-  const unsigned u = __float_as_uint(f);
-  const unsigned long long m = (unsigned long long)((u & 0x7FFFFFu) | 0x800000u);  // 2^23 (1.m)
-  const int e = (int)(u >> 23) - 127;                                             // f = 1.m 2^e
-  return m << (shift - 23 + e);
+// 2^32 f for a float f in [0.5, 1), from its bits (an integer-to-float
+// conversion would do, at eight times the issue cost)
+__device__ __forceinline__ unsigned unit_fixed32(float f) { return (__float_as_uint(f) << 8) | 0x80000000u; }
+// MUFU estimates (relative error about 2^-23), held inside [0.5, 1)
+__device__ __forceinline__ unsigned rcp_seed(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return unit_fixed32(fmaxf(fminf(r, 0.99999994f), 0.5f));
+}
+__device__ __forceinline__ unsigned rsqrt_seed(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return unit_fixed32(fmaxf(fminf(r, 0.99999994f), 0.5f));
 }
 
 }  // namespace fp64detail
@@ -90,11 +82,65 @@ __device__ __forceinline__ double dneg(double x) {
   return fp64detail::from_bits(fp64detail::bits(x) ^ 0x8000000000000000ull);
 }
 
-// ddiv_rn and dsqrt_rn are called, not inlined: a flux evaluation has half a
-// dozen of them, and inlined copies of their integer sequences made the edge
-// kernel stall on instruction fetch (ncu "no instruction"); out of line the
-// 1M-cell step ran 5 % faster (k_flux 0.215 vs 0.244 ms), with the same bits.
-static __device__ __noinline__ double ddiv_rn(double a, double b) {
+// Method of ddiv_rn and dsqrt_rn.  Both keep every step within 32 x 32 -> 64
+// bit products: a 32-bit reciprocal (square root) from the MUFU estimate and
+// one Newton step (y' = y + y (1 - b y), y' = y + y (1 - x y^2) / 2), then the
+// quotient (root) as two 31-bit digits with the running remainder held modulo
+// 2^64 (it is far smaller than that), the second digit signed.  The digits
+// leave an error of a few units 4 (5) bits below the last place, so the
+// candidate m0 they give is within (-0.3, 1.3) of the true value in units of
+// the last place, and one exact comparison with m0 + 1/2 rounds it.  (A tie
+// cannot occur: a quotient or root of 53-bit significands never lies half way
+// between two of them.)
+//
+// What bounds them is issue and, on small meshes, their own latency: a flux
+// evaluation holds eight, and with the 128-bit Newton steps used before (about
+// 290 instructions, 815 cycles each) the edge kernel issued 2536 instructions
+// per warp for its 62 FP64 ones.  Measured, SSPRK2 step before -> now: 8192-cell
+// Thacker bowl 172 -> 154 us, 1M-cell dam break 976 -> 945 us (k_flux 199 ->
+// 187 us).  At this length they are inlined (out of line 0.5-1 % slower; the
+// longer form was 5 % faster out of line).
+
+// ma = significand of the dividend in [mb, 2 mb), mb = the divisor's in
+// [2^52, 2^53): ma / mb rounded to 53 bits, in [2^52, 2^53].
+__device__ __forceinline__ unsigned long long div_significand(unsigned long long ma, unsigned long long mb) {
+  using namespace fp64detail;
+  const unsigned d = (unsigned)(mb >> 21);  // top 32 bits
+  const unsigned r0 = rcp_seed(__uint_as_float(0x3F800000u | ((d >> 8) & 0x7FFFFFu)));
+  // R = 2^84 / mb to 2 units: |e| < 2^42
+  const long long e = (long long)(0x8000000000000000ull - (unsigned long long)d * r0);
+  const unsigned R = r0 + (unsigned)(__mulhi((int)(e >> 12), (int)(r0 >> 1)) >> 18);
+  // ma / mb = (q1 + q2 2^-26) 2^-30 + rem2 / (mb 2^56)
+  const unsigned q1 = __umulhi((unsigned)(ma >> 22), R);
+  const long long rem1 = (long long)((ma << 30) - (unsigned long long)q1 * mb);  // within 6 mb < 2^56
+  const int q2 = __mulhi((int)(rem1 >> 25), (int)(R >> 1));
+  const long long rem2 = (long long)(((unsigned long long)rem1 << 26) - (unsigned long long)(long long)q2 * mb);
+  const unsigned long long Q = ((unsigned long long)q1 << 26) + (unsigned long long)(long long)q2;
+  const long long part = (long long)((Q & 15ull) * mb) + rem2;  // 16 (true - m0) mb
+  return (Q >> 4) + (part > (long long)(mb << 3) ? 1ull : 0ull);
+}
+
+// M in [2^52, 2^54): sqrt(M 2^52) rounded to an integer in [2^52, 2^53].
+__device__ __forceinline__ unsigned long long sqrt_significand(unsigned long long M) {
+  using namespace fp64detail;
+  const unsigned X = (unsigned)(M >> 22);  // x = X 2^-30 in [1, 4)
+  const float f = (X >> 31) ? __uint_as_float(0x40000000u | ((X >> 8) & 0x7FFFFFu))
+                            : __uint_as_float(0x3F800000u | ((X >> 7) & 0x7FFFFFu));
+  const unsigned r0 = rsqrt_seed(f);
+  // R = 2^32 / sqrt(x) to 3 units: |e| < 2^42
+  const long long e = (long long)(0x4000000000000000ull - (unsigned long long)X * __umulhi(r0, r0));
+  const unsigned R = r0 + (unsigned)(__mulhi((int)(e >> 11), (int)(r0 >> 1)) >> 19);
+  // sqrt(M) = (s1 + s2 2^-27) 2^-4 to a few units of 2^-31
+  const unsigned s1 = __umulhi(X, R);
+  const long long rem1 = (long long)((M << 8) - (unsigned long long)s1 * s1);  // within 4 * 2 s1 < 2^34
+  const int s2 = __mulhi((int)(rem1 >> 3), (int)(R >> 1));
+  const unsigned long long S = ((unsigned long long)s1 << 27) + (unsigned long long)(long long)s2;
+  const unsigned long long m0 = S >> 5;
+  const long long rem = (long long)((M << 52) - m0 * m0);  // (true - m0)(true + m0), modulo 2^64
+  return m0 + (rem > (long long)m0 ? 1ull : 0ull);
+}
+
+static __device__ __forceinline__ double ddiv_rn(double a, double b) {
   using namespace fp64detail;
   const unsigned long long ua = bits(a), ub = bits(b);
   const unsigned ea = (unsigned)(ua >> 52) & 0x7FFu, eb = (unsigned)(ub >> 52) & 0x7FFu;
@@ -105,102 +151,26 @@ static __device__ __noinline__ double ddiv_rn(double a, double b) {
   }
   unsigned long long ma = (ua & kM52) | kHid;
   const unsigned long long mb = (ub & kM52) | kHid;
-  const unsigned long long sign = (ua ^ ub) & 0x8000000000000000ull;
-  int e = (int)ea - (int)eb;
+  int E = (int)ea - (int)eb + 1023;
   if (ma < mb) {
     ma <<= 1;
-    --e;
+    --E;
   }
-  int E = e + 1023;
   if (E < 1 || E > 2046) return ddiv_hw(a, b);
-  if (mb == kHid) return from_bits(sign | ((unsigned long long)E << 52) | (ma & kM52));  // power of two
-  // R ~ 2^116 / mb in (2^63, 2^64): float estimate from mb's leading bits
-  // (1 <= fb < 2, 1 / fb in (0.5, 1]), two Newton steps
-  const float fb = __uint_as_float(0x3F800000u | (unsigned)((mb >> 29) & 0x7FFFFFull));
-  const float rf = __frcp_rn(fb);
-  unsigned long long R = rf < 1.0f ? fixed_from_unit_float(rf, 64) : ~0ull;
-  {
-    const unsigned __int128 P = (unsigned __int128)mb * R;
-    const __int128 D = ((__int128)1 << 116) - (__int128)P;  // |D| < 2^94
-    const long long Dh = (long long)(D >> 32);
-    R += (unsigned long long)(long long)(((__int128)R * Dh) >> 84);
-  }
-  {
-    const unsigned __int128 P = (unsigned __int128)mb * R;
-    const __int128 D = ((__int128)1 << 116) - (__int128)P;  // |D| < 2^71
-    const long long Dh = (long long)(D >> 9);
-    R += (unsigned long long)(long long)(((__int128)R * Dh) >> 107);
-  }
-  // Q = floor(ma 2^62 / mb) in [2^62, 2^63), corrected with the exact remainder
-  unsigned long long Q = (unsigned long long)(((unsigned __int128)ma * R) >> 54);
-  const __int128 N = (__int128)((unsigned __int128)ma << 62);
-  __int128 rem = N - (__int128)((unsigned __int128)Q * mb);
-#pragma unroll 1
-  for (int k = 0; k < 8 && rem < 0; ++k) {
-    --Q;
-    rem += (__int128)mb;
-  }
-#pragma unroll 1
-  for (int k = 0; k < 8 && rem >= (__int128)mb; ++k) {
-    ++Q;
-    rem -= (__int128)mb;
-  }
-  if (rem < 0 || rem >= (__int128)mb || Q < (1ull << 62) || Q >= (1ull << 63)) return ddiv_hw(a, b);
-  unsigned long long mant = round63(Q, rem != 0);
-  if (mant == (1ull << 53)) {
-    mant = kHid;
-    if (++E > 2046) return ddiv_hw(a, b);
-  }
-  return from_bits(sign | ((unsigned long long)E << 52) | (mant & kM52));
+  // a significand of 2^53 carries into the exponent (and 2046 + 1 is infinity)
+  return from_bits(((ua ^ ub) & 0x8000000000000000ull) |
+                   (((unsigned long long)(unsigned)(E - 1) << 52) + div_significand(ma, mb)));
 }
 
-static __device__ __noinline__ double dsqrt_rn(double x) {
+static __device__ __forceinline__ double dsqrt_rn(double x) {
   using namespace fp64detail;
   const unsigned long long ux = bits(x);
   const unsigned ex = (unsigned)(ux >> 52) & 0x7FFu;
   if (ex - 1u >= 2046u || (ux >> 63)) return (ux << 1) == 0ull ? x : dsqrt_hw(x);  // sqrt(+-0) = +-0 (dry side)
+  // x = M 2^(e - 52) with an even e; 1023 is odd, so an even biased exponent is an odd e
   unsigned long long M = (ux & kM52) | kHid;
-  int e = (int)ex - 1023;  // x = M 2^(e - 52)
-  if (e & 1) {             // make e - 52 even
-    M <<= 1;
-    --e;
-  }
-  // R ~ 2^89 / sqrt(M) in (2^62, 2^63]: float estimate from M's leading bits
-  // (fm = M 2^-52 in [1, 4), 1 / sqrt(fm) in (0.5, 1])
-  const float fm = (M >> 53) ? __uint_as_float(0x40000000u | (unsigned)((M >> 30) & 0x7FFFFFull))
-                             : __uint_as_float(0x3F800000u | (unsigned)((M >> 29) & 0x7FFFFFull));
-  unsigned long long R = fixed_from_unit_float(rsqrtf(fm), 63);
-  {
-    const unsigned long long T = (unsigned long long)(((unsigned __int128)R * R) >> 64);  // ~ 2^114 / M
-    const unsigned __int128 U = (unsigned __int128)M * T;                                   // ~ 2^114
-    const __int128 D = ((__int128)1 << 114) - (__int128)U;  // |D| < 2^94
-    const long long Dh = (long long)(D >> 32);
-    R += (unsigned long long)(long long)(((__int128)R * Dh) >> 83);
-  }
-  {
-    const unsigned long long T = (unsigned long long)(((unsigned __int128)R * R) >> 64);
-    const unsigned __int128 U = (unsigned __int128)M * T;
-    const __int128 D = ((__int128)1 << 114) - (__int128)U;  // |D| < 2^73
-    const long long Dh = (long long)(D >> 11);
-    R += (unsigned long long)(long long)(((__int128)R * Dh) >> 104);
-  }
-  // S = floor(sqrt(M 2^72)) in [2^62, 2^63), corrected with exact squares
-  unsigned long long S = (unsigned long long)(((unsigned __int128)M * R) >> 53);
-  const unsigned __int128 N = (unsigned __int128)M << 72;
-#pragma unroll 1
-  for (int k = 0; k < 8 && (unsigned __int128)S * S > N; ++k) --S;
-#pragma unroll 1
-  for (int k = 0; k < 8 && (unsigned __int128)(S + 1) * (S + 1) <= N; ++k) ++S;
-  const unsigned __int128 S2 = (unsigned __int128)S * S;
-  if (S2 > N || (unsigned __int128)(S + 1) * (S + 1) <= N || S < (1ull << 62) || S >= (1ull << 63))
-    return dsqrt_hw(x);
-  unsigned long long mant = round63(S, S2 != N);
-  int E = 26 + (e - 52) / 2 + 1023;
-  if (mant == (1ull << 53)) {
-    mant = kHid;
-    ++E;
-  }
-  return from_bits(((unsigned long long)E << 52) | (mant & kM52));
+  if (!(ex & 1u)) M <<= 1;
+  return from_bits(((unsigned long long)((ex + 1u) / 2u + 510u) << 52) + sqrt_significand(M));
 }
 
 #endif  // __CUDACC__
