@@ -134,6 +134,41 @@ extern "C" swe_status swe_selftest_fp64(int64_t n, uint64_t seed, int64_t* div_m
 }
 
 // ---------------------------------------------------------------------------
+// The point-wise routines that replace an operation of the reference by another
+// way to the same bits, on the caller's operands (host or device build).
+namespace {
+
+// operands per result: 0 bisection (d, c, b, xmin, xmax), 1 cube root
+__host__ __device__ constexpr int pointwise_args(int kind) { return kind == 0 ? 5 : 1; }
+__host__ __device__ double pointwise(int kind, const double* a) {
+  if (kind == 0) return swe::bisection(a[0], a[1], a[2], a[3], a[4]);
+  return swe::cbrt_rn(a[0]);
+}
+__global__ void k_pointwise(int kind, int n, const double* in, double* out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = pointwise(kind, in + (size_t)i * pointwise_args(kind));
+}
+
+}  // namespace
+
+extern "C" swe_status swe_selftest_pointwise(int32_t kind, int64_t n, const double* in, double* out, int32_t device) {
+  if (kind < 0 || kind > 1 || n <= 0 || n > (1 << 26) || !in || !out) return SWE_ERR_INVALID_ARGUMENT;
+  const size_t m = pointwise_args(kind);
+  if (!device) {
+    for (int64_t i = 0; i < n; ++i) out[i] = pointwise(kind, in + i * m);
+    return SWE_OK;
+  }
+  double* d = nullptr;
+  if (cudaMalloc(&d, (m + 1) * n * sizeof(double)) != cudaSuccess) return SWE_ERR_OUT_OF_MEMORY;
+  cudaError_t e = cudaMemcpy(d, in, m * n * sizeof(double), cudaMemcpyHostToDevice);
+  k_pointwise<<<(int)((n + 127) / 128), 128>>>(kind, (int)n, d, d + m * n);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemcpy(out, d + m * n, n * sizeof(double), cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  return e == cudaSuccess ? SWE_OK : SWE_ERR_CUDA;
+}
+
+// ---------------------------------------------------------------------------
 // Self-test of the hand-written flux reverse against the forward-mode
 // Jacobian (Dual<7>) on random interface states.
 namespace {

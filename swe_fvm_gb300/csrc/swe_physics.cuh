@@ -109,12 +109,41 @@ SWE_HD void plane_gradient(double p0x, double p0y, double p0z, double p1x, doubl
   *gy = x1;
 }
 
+// Bit patterns on the host and the device.
+#if defined(__CUDA_ARCH__)
+__device__ __forceinline__ unsigned long long ubits(double x) { return (unsigned long long)dbits(x); }
+__device__ __forceinline__ double ufrom(unsigned long long u) { return dfrom((long long)u); }
+#else
+SWE_HD unsigned long long ubits(double x) {
+  union { double d; unsigned long long u; } c;
+  c.d = x;
+  return c.u;
+}
+SWE_HD double ufrom(unsigned long long u) {
+  union { double d; unsigned long long u; } c;
+  c.u = u;
+  return c.d;
+}
+#endif
+// a / b in single precision where only a correction or a starting point depends on it
+SWE_HD float quick_div(float a, float b) {
+#if defined(__CUDA_ARCH__)
+  return __fdividef(a, b);
+#else
+  return a / b;
+#endif
+}
+SWE_HD bool negative(double x) { return (ubits(x) >> 63) != 0ull; }
+SWE_HD double magnitude(double x) { return ufrom(ubits(x) & 0x7FFFFFFFFFFFFFFFull); }
+
 // (int)log2(x) for finite x > 0, truncated toward zero, from the exponent bits
 // (src/PointOperations.cpp:33).
 SWE_HD int trunc_log2(double x) {
-  int e;
-  double m = frexp(x, &e);
-  if (m == 0.5) return e - 1;
+  const unsigned long long u = ubits(x);
+  int e = (int)(u >> 52) - 1022;  // x = m 2^e, m in [0.5, 1)
+  bool half = (u << 12) == 0ull;
+  if ((u >> 52) == 0ull) half = frexp(x, &e) == 0.5;  // subnormal
+  if (half) return e - 1;
   return (e >= 1) ? e - 1 : e;
 }
 
@@ -123,9 +152,12 @@ SWE_HD int trunc_log2(double x) {
 // faithful, not correctly rounded, and the CUDA and host ones differ in the
 // last bit; this one is exact on both.  Method: x = Mx 2^E with a 53-bit
 // integer Mx; N = Mx 2^t with t in {107, 108, 109} chosen so that 3 | (E - t)
-// and N in [2^159, 2^162); Y = floor(cbrt(N)) in [2^53, 2^54) is found from a
-// library estimate corrected with exact 192-bit integer cubes; its lowest bit
-// and the remainder N - Y^3 round it to 53 bits.
+// and N in [2^159, 2^162); Y = floor(cbrt(N)) in [2^53, 2^54) is found from an
+// estimate corrected with exact 192-bit integer cubes; its lowest bit and the
+// remainder N - Y^3 round it to 53 bits.  The estimate is a single-precision
+// root and two Newton steps whose corrections are single-precision quotients
+// (2^-22 -> 2^-44 -> a few units): a library root, frexp and ldexp in its place
+// put some four thousand cycles on the chain of every thin cell.
 struct U192 {
   unsigned long long w[3];  // little-endian limbs
 };
@@ -141,72 +173,219 @@ SWE_HD U192 u192_cube(unsigned long long y) {
   r.w[2] = (unsigned long long)((mid >> 64) + (hi >> 64));
   return r;
 }
-SWE_HD int u192_cmp(const U192& a, const U192& b) {
-  for (int k = 2; k >= 0; --k) {
-    if (a.w[k] < b.w[k]) return -1;
-    if (a.w[k] > b.w[k]) return 1;
-  }
-  return 0;
+// a <= b
+SWE_HD bool u192_le(const U192& a, const U192& b) {
+  if (a.w[2] != b.w[2]) return a.w[2] < b.w[2];
+  if (a.w[1] != b.w[1]) return a.w[1] < b.w[1];
+  return a.w[0] <= b.w[0];
 }
 SWE_HD double cbrt_rn(double x) {
-  if (!(x == x) || x == 0. || isinf(x)) return x + x;  // NaN, +-0, +-inf
-  const bool neg = x < 0.;
-  double ax = neg ? -x : x;
+  if (!(x == x) || x == 0. || (ubits(x) << 1) == (0x7FFull << 53)) return x + x;  // NaN, +-0, +-inf
+  const bool neg = negative(x);
+  double ax = magnitude(x);
   int scale = 0;
   if (ax < 2.2250738585072014e-308) {  // subnormal: scale by 2^54
     ax = ax * 18014398509481984.0;
     scale = -18;
   }
-  int e;
-  const double m = frexp(ax, &e);                                  // ax = m 2^e, m in [0.5, 1)
-  const unsigned long long Mx = (unsigned long long)ldexp(m, 53);  // exact 53-bit integer
-  const int E = e - 53;                                            // ax = Mx 2^E
-  int t = 107;
-  while (((E - t) % 3 + 3) % 3 != 0) ++t;
-  // N = Mx 2^t as 192 bits
+  const unsigned long long ua = ubits(ax);
+  const unsigned long long Mx = (ua & ((1ull << 52) - 1ull)) | (1ull << 52);
+  const int E = (int)(ua >> 52) - 1075;  // ax = Mx 2^E
+  const int k = ((E - 107) % 3 + 3) % 3;  // t = 107 + k
+  // N = Mx 2^t as 192 bits (t - 64 in {43, 44, 45})
   U192 N;
+  N.w[0] = 0ull;
+  N.w[1] = Mx << (43 + k);
+  N.w[2] = Mx >> (21 - k);
+  // u = Mx 2^(k - 52) in [1, 8), exactly; c -> cbrt(u) = cbrt(N) 2^-53
+  const double u = ufrom((Mx & ((1ull << 52) - 1ull)) | ((unsigned long long)(1023 + k) << 52));
+  double c = (double)cbrtf((float)u);
+  c -= (double)quick_div((float)(c * c * c - u), (float)(3. * c * c));
   {
-    const int word = t / 64, bit = t % 64;
-    N.w[0] = N.w[1] = N.w[2] = 0ull;
-    N.w[word] = Mx << bit;
-    if (bit && word + 1 < 3) N.w[word + 1] = Mx >> (64 - bit);
+    const double p = c * c, e = fma(c, c, -p);
+    const double r = fma(p, c, -u) + e * c;  // c^3 - u
+    c -= (double)quick_div((float)r, (float)(3. * p));
   }
-  // estimate: cbrt(Mx 2^t) = cbrt(Mx) 2^(t/3)
-  const double est = ldexp(cbrt((double)Mx * ldexp(1.0, t % 3)), t / 3);
-  unsigned long long Y = (unsigned long long)est;
+  const double est = c * 9007199254740992.0;  // 2^53
+  unsigned long long Y = est >= 18014398509481983.0 ? (1ull << 54) - 1 : (unsigned long long)est;
   if (Y < (1ull << 53)) Y = 1ull << 53;
-  if (Y >= (1ull << 54)) Y = (1ull << 54) - 1;
-  for (int it = 0; it < 64 && u192_cmp(u192_cube(Y), N) > 0; ++it) --Y;
-  for (int it = 0; it < 64 && u192_cmp(u192_cube(Y + 1), N) <= 0; ++it) ++Y;
-  const bool sticky = u192_cmp(u192_cube(Y), N) != 0;
-  unsigned long long R = Y >> 1;
+  U192 q = u192_cube(Y);
+  for (int it = 0; it < 64 && !u192_le(q, N); ++it) q = u192_cube(--Y);
+  for (int it = 0; it < 64; ++it) {
+    const U192 q1 = u192_cube(Y + 1);
+    if (!u192_le(q1, N)) break;
+    ++Y;
+    q = q1;
+  }
+  const bool sticky = q.w[0] != N.w[0] || q.w[1] != N.w[1] || q.w[2] != N.w[2];
+  unsigned long long R = Y >> 1;  // in [2^52, 2^53)
   if ((Y & 1ull) && (sticky || (R & 1ull))) ++R;
-  const double r = ldexp((double)R, (E - t) / 3 + 1 + scale);
+  // R 2^s with s = (E - t) / 3 + 1 + scale: the result is normal, a carry of R
+  // to 2^53 goes into the exponent
+  const int s = (E - 107 - k) / 3 + 1 + scale;
+  const double r = ufrom(((unsigned long long)(s + 1074) << 52) + R);
   return neg ? -r : r;
 }
 
 // include/CubicPolyMath.h:13-15: x^3 + b x^2 + c x + d
 SWE_HD double cubic(double d, double c, double b, double x) { return x * x * x + b * x * x + c * x + d; }
 
-// src/PointOperations.cpp:26-40.  f(xmin) is carried between iterations
-// instead of re-evaluated: the same function of the same argument.
-SWE_HD double bisection(double d, double c, double b, double xmin, double xmax) {
-  double fmin_ = cubic(d, c, b, xmin);
-  double fmax_ = cubic(d, c, b, xmax);
-  if (signbit(fmin_) == signbit(fmax_)) return dlt(fabs(fmin_), fabs(fmax_)) ? xmin : xmax;
-  int n = 50 + trunc_log2(xmax - xmin);
-  double x = 0.;
-  bool smin_ = signbit(fmin_);
-  for (int it = 0; it <= n; it++) {
-    x = SWE_HALF(xmin + xmax);
-    double fx = cubic(d, c, b, x);
-    bool sx = signbit(fx);
-    if (smin_ != sx) {
-      xmax = x;
-    } else {
-      xmin = x;
-      smin_ = sx;
+// |a| > |b| for two magnitudes, from their bits
+SWE_HD bool above(double x, double bound) { return ubits(x) > ubits(bound); }
+
+// The reference's bisection (src/PointOperations.cpp:26-40), bit for bit.  Its
+// result is the last midpoint of a path that only the sign of the computed f
+// at each midpoint decides, and away from the root that sign is known without
+// evaluating f.  Let E bound the error of a computed value anywhere on the
+// interval, let f have one curvature there, and let lo < hi be points where the
+// computed |f| exceeds 2 E (as at the ends of the interval) with the signs of
+// f(xmin) and f(xmax).  Then the true |f| exceeds E on all of [xmin, lo] and
+// [hi, xmax]: the side on which f runs away from zero is monotone, and on the
+// other a convex (concave) f lies on the far side of the chord between two such
+// points.  (Where lo <= xmin or hi >= xmax that part is empty.)  So f is
+// evaluated only between lo and hi, some units of rounding apart: 7 to 20 of
+// the 51 evaluations, each 5 to 8 FP64 operations of 64 cycles for the warp.
+// lo and hi come from a single-precision bisection and two Newton steps; where
+// the check fails the whole path is walked.  With cbrt_rn above, SSPRK2 pass
+// before -> now: 8192-cell Thacker bowl 154 -> 132 us a step, 250k-cell coast
+// 504 -> 436 us (k_recon1 86 -> 57 us, k_recon2 47 -> 43 us).
+// The float root s in [0, 1] of ((p3 s + p2) s + p1) s + p0, whose value at 0
+// has the sign neg: 20 halvings.
+SWE_HD float unit_root(float p3, float p2, float p1, float p0, bool neg) {
+  float s = 0.f, w = 0.5f;
+  for (int it = 0; it < 20; ++it) {
+    const float sm = s + w;
+    const float f = ((p3 * sm + p2) * sm + p1) * sm + p0;
+    if ((f < 0.f) == neg) s = sm;
+    w *= 0.5f;
+  }
+  return s + w;
+}
+
+// (xmin + xmax) / 2 rounded as the reference's 0.5 (xmin + xmax).
+SWE_HD double midpoint(double xmin, double xmax) {
+  const unsigned long long A = ubits(xmin), Z = ubits(xmax);
+  const unsigned ex = (unsigned)(A >> 52);
+  if (ex == (unsigned)(Z >> 52) && (ex & 0x7FFu) > 2u && (ex & 0x7FFu) < 0x7FEu) {
+    // one sign and binade: the mean of the bit patterns, rounded to even
+    const unsigned long long h = (A & Z) + ((A ^ Z) >> 1);
+    return ufrom(h + (h & (A ^ Z) & 1ull));
+  }
+  return SWE_HALF(xmin + xmax);
+}
+
+// x^3 + c x + d on [0, 1] (PartWet2).  The quadratic term is 0 x x, whose
+// addition changes no bit of x^3 >= 0; f(0) is 0 + d and f(1) (1 + c) + d.  The
+// midpoints are dyadic, so the steps down to the last interval that holds
+// [lo, hi] are taken at once.  A lone call on GB300: 34000 -> 11200 cycles.
+SWE_HD double bisection01(double d, double c) {
+  const double fmin_ = 0. + d, fmax_ = (1. + c) + d;
+  const bool neg_min = negative(fmin_);
+  if (neg_min == negative(fmax_)) return dlt(magnitude(fmin_), magnitude(fmax_)) ? 0. : 1.;
+  constexpr int n = 50;
+  double xmin = 0., xmax = 1.;
+  double lo = 0., hi = 1.;
+  int it = 0;
+  // convex; |computed f - f| <= u (5 x^3 + 3 |c| x + |d|), held a little larger
+  const double E = 6e-16 + 3.6e-16 * magnitude(c) + 1.3e-16 * magnitude(d);
+  {
+    const float g = quick_div(1.0f, fmaxf(fabsf((float)fmin_), fabsf((float)fmax_)));
+    double x = (double)unit_root(g, 0.f, (float)c * g, (float)fmin_ * g, neg_min);
+    double slope = 0.;
+    for (int q = 0; q < 2; ++q) {
+      const double xx = x * x;
+      slope = 3. * xx + c;
+      x -= (double)quick_div((float)((xx + c) * x + d), (float)slope);
     }
+    const double gap = (double)quick_div((float)(2.6 * E), fabsf((float)slope)) + 4.5e-16;
+    const double l = x - gap, h = x + gap, E2 = 2. * E;
+    const double fl = l * l * l + c * l + d, fh = h * h * h + c * h + d;
+    const bool at0 = !dlt(0., l), at1 = !dlt(h, 1.);
+    const bool ok = (at0 || (negative(fl) == neg_min && above(magnitude(fl), E2) && above(magnitude(fmin_), E2))) &&
+                    (at1 || (negative(fh) != neg_min && above(magnitude(fh), E2) && above(magnitude(fmax_), E2))) &&
+                    dlt(l, 1.) && dlt(0., h) && above(1e280, E) && x == x;
+    if (ok && !at0) lo = l;
+    if (ok && !at1) hi = h;
+    if (ok) {
+      // floor(lo 2^62) and ceil(hi 2^62) - 1: their common leading bits are steps
+      const unsigned long long ul = ubits(lo), uh = ubits(hi);
+      const int sl = 1013 - (int)(ul >> 52), sh = 1013 - (int)(uh >> 52);
+      const unsigned long long hid = 1ull << 52, ml = (ul & (hid - 1)) | hid, mh = (uh & (hid - 1)) | hid;
+      unsigned long long fl62 = 0ull, fh62 = (1ull << 62) - 1ull;
+      if (!at0) fl62 = sl <= 0 ? ml << -sl : sl < 64 ? ml >> sl : 0ull;
+      if (!at1) fh62 = sh <= 0 ? (mh << -sh) - 1ull : sh < 53 ? (mh - 1ull) >> sh : 0ull;
+      unsigned long long diff = fl62 ^ fh62;
+      int k = 0;
+      for (int w = 32; w > 0; w >>= 1)
+        if (k + w <= 62 && (diff >> (62 - k - w)) == 0ull) k += w;
+      if (k > n) k = n;
+      const unsigned long long j = fl62 >> (62 - k);
+      const double scale = ufrom((unsigned long long)(1023 - k) << 52);  // 2^-k
+      xmin = (double)j * scale;
+      xmax = (double)(j + 1ull) * scale;
+      it = k;
+    }
+  }
+  double x = 0.;
+  for (; it <= n; it++) {
+    x = midpoint(xmin, xmax);
+    bool left;
+    if (dle(x, lo)) left = true;
+    else if (dle(hi, x)) left = false;
+    else left = negative(x * x * x + c * x + d) == neg_min;
+    if (left) xmin = x;
+    else xmax = x;
+  }
+  return x;
+}
+
+// The general form.  34000 -> 22700 cycles a call for nearly flat cells on a
+// high bed, where rounding hides the sign longest (20 evaluations).
+SWE_HD double bisection(double d, double c, double b, double xmin, double xmax) {
+  if ((ubits(b) | ubits(xmin)) == 0ull && ubits(xmax) == ubits(1.)) return bisection01(d, c);
+  const double fmin_ = cubic(d, c, b, xmin);
+  const double fmax_ = cubic(d, c, b, xmax);
+  const bool neg_min = negative(fmin_);
+  if (neg_min == negative(fmax_)) return dlt(magnitude(fmin_), magnitude(fmax_)) ? xmin : xmax;
+  const double w = xmax - xmin;
+  const int n = 50 + trunc_log2(w);
+  double lo = xmin, hi = xmax;
+  const double c0 = 3. * xmin + b, c1 = 3. * xmax + b;  // f'' / 2 at the ends
+  if (n > 8 && ((dle(0., c0) && dle(0., c1)) || (dle(c0, 0.) && dle(c1, 0.)))) {
+    // f(xmin + w s) / |f| in single precision, s in [0, 1]
+    const float fw = (float)w, fc0 = (float)c0;
+    const float g = quick_div(1.0f, fmaxf(fabsf((float)fmin_), fabsf((float)fmax_)));
+    const double s0 = xmin * (c0 + b) + c;  // f'(xmin)
+    const float p1 = (float)s0 * fw * g, p2 = fc0 * fw * fw * g, p3 = fw * fw * fw * g;
+    double x = xmin + w * (double)unit_root(p3, p2, p1, (float)fmin_ * g, neg_min);
+    double slope = 0.;
+    for (int q = 0; q < 2; ++q) {
+      const double y = x + b;
+      slope = x * (2. * y + x) + c;
+      x -= (double)quick_div((float)((x * y + c) * x + d), (float)slope);
+    }
+    // |computed f - f| <= u (5 |x|^3 + 5 |b| x^2 + 3 |c| |x| + |d|), a little larger
+    const double m = smax(magnitude(xmin), magnitude(xmax));
+    const double E = 6e-16 * (((m + magnitude(b)) * m + magnitude(c)) * m) + 1.3e-16 * magnitude(d);
+    const double gap = (double)quick_div((float)(2.6 * E), fabsf((float)slope)) + 4.5e-16 * m;
+    const double l = x - gap, h = x + gap, E2 = 2. * E;
+    const double fl = cubic(d, c, b, l), fh = cubic(d, c, b, h);
+    const bool at0 = !dlt(xmin, l), at1 = !dlt(h, xmax);
+    const bool ok = (at0 || (negative(fl) == neg_min && above(magnitude(fl), E2) && above(magnitude(fmin_), E2))) &&
+                    (at1 || (negative(fh) != neg_min && above(magnitude(fh), E2) && above(magnitude(fmax_), E2))) &&
+                    dlt(l, xmax) && dlt(xmin, h) && above(E, 1e-280) && above(1e280, E) && x == x;
+    if (ok && !at0) lo = l;
+    if (ok && !at1) hi = h;
+  }
+  double x = 0.;
+  for (int it = 0; it <= n; it++) {
+    x = midpoint(xmin, xmax);
+    bool left;
+    if (dle(x, lo)) left = true;
+    else if (dle(hi, x)) left = false;
+    else left = negative(cubic(d, c, b, x)) == neg_min;
+    if (left) xmin = x;
+    else xmax = x;
   }
   return x;
 }
