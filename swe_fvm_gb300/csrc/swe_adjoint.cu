@@ -903,6 +903,14 @@ struct AdjointState {
 
 void adjoint_state_delete(AdjointState* a) { delete a; }
 
+// The work arrays, the topology lists and the side stream stay; a run's tape is
+// of the old bed, and so are the plane adjoints.
+cudaError_t adjoint_state_new_bed(AdjointState* a, const DevMesh& m, cudaStream_t s) {
+  a->free_tape();
+  k_plane_adj_init<<<(m.C + 255) / 256, 256, 0, s>>>(m, a->aw.padj);
+  return cudaGetLastError();
+}
+
 std::string Engine::adjoint_init() {
   if (adj_) return "";
   AdjointState* a = new AdjointState();

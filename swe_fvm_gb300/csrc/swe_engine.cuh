@@ -99,7 +99,9 @@ struct DevMesh {
   const int* einst;     // [E] (batched only)
   const EdgeRec* erec;  // [E] enx, eny, etx, ety, ezm, elmin, packed
   const int4* eidx;     // [E] (eown, enb, eslotl, eslotr), packed
+  const int2* enode;    // [E] the edge's nodes
   // nodes
+  const double2* nxy;   // [N] plan position
   const double* nz;     // [N]
   const int* nptr;      // [N+1] the cells around each node (CSR) ...
   const int* ncell;     // [3C]  ... as (cell << 2) | local node index
@@ -110,6 +112,15 @@ struct DevMesh {
   // the engine's device error word (DevWork::err), for the range checks of
   // checked builds in code that sees only the mesh
   unsigned* err;
+};
+
+// The records that depend on the bathymetry, as the device computes them
+// (DevMesh's arrays of the same names).
+struct BedArrays {
+  double *bc, *fwthr, *zn, *ze, *dry, *combo, *pw1, *ezm, *nz;
+  Pw2Rec* pw2;
+  SlotRec* srec;  // ze only
+  EdgeRec* erec;  // b only
 };
 
 struct DevWork {
@@ -194,6 +205,8 @@ struct Layout {
 struct AdjWork;
 struct AdjointState;
 void adjoint_state_delete(AdjointState* a);
+// A new bed: drops the tape and rebuilds the tables that depend on it.
+cudaError_t adjoint_state_new_bed(AdjointState* a, const DevMesh& m, cudaStream_t s);
 
 class Engine {
  public:
@@ -231,10 +244,10 @@ class Engine {
   int* d_cell_to = nullptr;
   std::string set_layouts(std::vector<Layout>&& lay);
   // Replaces the node bathymetry of the instances whose pointer is not null
-  // (each in the caller's node order, N_q values), recomputes every mesh record
-  // with the same device order and re-uploads them into the same buffers (the
-  // captured step graphs stay valid); drops the adjoint's tape.  The state is
-  // kept; the caller re-primes the flux pass.
+  // (each in the caller's node order, N_q values) and recomputes the mesh
+  // records that depend on it on the device, in the same buffers (the captured
+  // step graphs stay valid); drops the adjoint's tape.  The state is kept; the
+  // caller re-primes the flux pass.
   std::string set_bathymetry(const std::vector<const double*>& z);
   // Mean ms of one graph-replayed step of `scheme` (CFL dt) over n steps after
   // one warm-up replay, run from the current state, which is then restored
@@ -367,19 +380,23 @@ class Engine {
   cudaGraphExec_t graphs_[4][3] = {};  // [scheme id][latch mode]
   Scheme custom_{};
   AdjointState* adj_ = nullptr;
-  std::vector<std::pair<void*, size_t>> mesh_arrays_;  // device mesh records in upload order
+  BedArrays bed_{};
+  // the bathymetry-dependent mesh records from the node z (device order), on
+  // the engine's stream (swe_bed.cu); nz_host must outlive the copy
+  cudaError_t compute_bed(const double* nz_host);
+  std::vector<double> host_nz() const;
   double adj_reg_depth_ = kEta1;
 };
 
-// Precompute (swe_precompute.cu): fills the host images of DevMesh arrays for
-// instance `inst` at offsets (c0, e0, n0) of the concatenated arrays.
+// Precompute (swe_precompute.cu): fills the host images of the DevMesh arrays
+// that the bathymetry does not enter for instance `inst` at offsets (c0, e0, n0) of the concatenated arrays.
 struct HostImage {
   int C, E, N, I;
   std::vector<int> cnode, cnbr, cedge, cinst, eown, enb, eslotl, eslotr, einst, inst_cell_begin, nptr, ncell;
   std::vector<unsigned char> cown;
-  std::vector<double> bc, fwthr, area, zn, ze, cek, cnxc, cnyc, dry, combo, pw1, enx, eny, etx, ety, ezm, elmin, nz,
-      inst_cfl, inst_cor;
-  std::vector<Pw2Rec> pw2;
+  std::vector<double> area, cek, cnxc, cnyc, enx, eny, etx, ety, elmin, inst_cfl, inst_cor;
+  std::vector<double2> nxy;
+  std::vector<int2> enode;
   std::vector<SlotRec> srec;
   std::vector<int2> cslot;
   std::vector<EdgeRec> erec;

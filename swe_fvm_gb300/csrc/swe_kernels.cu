@@ -702,16 +702,12 @@ std::string Engine::init(std::vector<HostInstance>&& inst, int flux, int ws, int
   img.resize((int)C, (int)E, (int)N, I);
   for (int q = 0; q < I; ++q) precompute_instance(inst[q], q, cell_off[q], edge_off[q], node_off[q], img);
 
-  // every mesh array is recorded (device pointer, bytes) in upload order, so
-  // that set_bathymetry can refill the same buffers
-  mesh_arrays_.clear();
   auto up = [&](auto& vec, auto*& dst) -> bool {
     using T = typename std::remove_reference<decltype(vec)>::type::value_type;
     T* d = dalloc<T>(vec.size());
     if (!d) return false;
     if (cudaMemcpy(d, vec.data(), vec.size() * sizeof(T), cudaMemcpyHostToDevice) != cudaSuccess) return false;
     dst = d;
-    mesh_arrays_.push_back({(void*)d, vec.size() * sizeof(T)});
     return true;
   };
   DevMesh& M = mesh_;
@@ -719,35 +715,38 @@ std::string Engine::init(std::vector<HostInstance>&& inst, int flux, int ws, int
   bool ok = true;
   const int *p_cnode, *p_cnbr, *p_cedge, *p_cinst, *p_eown, *p_enb, *p_esl, *p_esr, *p_einst, *p_icb;
   const unsigned char* p_cown;
-  const double *p_bc, *p_fw, *p_area, *p_zn, *p_ze, *p_cek, *p_cnxc, *p_cnyc, *p_dry, *p_combo, *p_pw1, *p_enx, *p_eny,
-      *p_etx, *p_ety, *p_ezm, *p_elmin, *p_nz, *p_cfl, *p_cor;
-  const Pw2Rec* p_pw2;
-  const SlotRec* p_srec;
-  const int2* p_cslot;
-  const EdgeRec* p_erec;
+  const double *p_area, *p_cek, *p_cnxc, *p_cnyc, *p_enx, *p_eny, *p_etx, *p_ety, *p_elmin, *p_cfl, *p_cor;
+  const int2 *p_cslot, *p_enode;
+  const double2* p_nxy;
   const int4* p_eidx;
   ok = ok && up(img.cnode, p_cnode) && up(img.cnbr, p_cnbr) && up(img.cedge, p_cedge) && up(img.cinst, p_cinst);
-  ok = ok && up(img.cown, p_cown) && up(img.bc, p_bc) && up(img.fwthr, p_fw) && up(img.area, p_area);
-  ok = ok && up(img.zn, p_zn) && up(img.ze, p_ze) && up(img.cek, p_cek) && up(img.cnxc, p_cnxc) && up(img.cnyc, p_cnyc);
-  ok = ok && up(img.dry, p_dry) && up(img.combo, p_combo) && up(img.pw1, p_pw1) && up(img.pw2, p_pw2);
+  ok = ok && up(img.cown, p_cown) && up(img.area, p_area);
+  ok = ok && up(img.cek, p_cek) && up(img.cnxc, p_cnxc) && up(img.cnyc, p_cnyc);
   ok = ok && up(img.eown, p_eown) && up(img.enb, p_enb) && up(img.eslotl, p_esl) && up(img.eslotr, p_esr);
   ok = ok && up(img.einst, p_einst) && up(img.enx, p_enx) && up(img.eny, p_eny) && up(img.etx, p_etx);
-  ok = ok && up(img.ety, p_ety) && up(img.ezm, p_ezm) && up(img.elmin, p_elmin) && up(img.nz, p_nz);
+  ok = ok && up(img.ety, p_ety) && up(img.elmin, p_elmin) && up(img.enode, p_enode) && up(img.nxy, p_nxy);
   ok = ok && up(img.inst_cell_begin, p_icb) && up(img.inst_cfl, p_cfl) && up(img.inst_cor, p_cor);
-  ok = ok && up(img.srec, p_srec) && up(img.cslot, p_cslot) && up(img.erec, p_erec) && up(img.eidx, p_eidx);
+  ok = ok && up(img.srec, bed_.srec) && up(img.cslot, p_cslot) && up(img.erec, bed_.erec) && up(img.eidx, p_eidx);
   const int *p_nptr, *p_ncell;
   ok = ok && up(img.nptr, p_nptr) && up(img.ncell, p_ncell);
+  bed_.bc = dalloc<double>(C); bed_.fwthr = dalloc<double>(C);
+  bed_.zn = dalloc<double>(3 * C); bed_.ze = dalloc<double>(3 * C);
+  bed_.dry = dalloc<double>(kDryStride * C); bed_.combo = dalloc<double>(8 * kComboStride * C);
+  bed_.pw1 = dalloc<double>(kPw1Stride * C); bed_.pw2 = dalloc<Pw2Rec>(C);
+  bed_.ezm = dalloc<double>(E); bed_.nz = dalloc<double>(N);
+  ok = ok && bed_.bc && bed_.fwthr && bed_.zn && bed_.ze && bed_.dry && bed_.combo && bed_.pw1 && bed_.pw2 &&
+       bed_.ezm && bed_.nz;
   if (!ok) {
     *st = 6;
     return std::string("device allocation or upload failed: ") + cudaGetErrorString(cudaGetLastError());
   }
   M.cnode = p_cnode; M.cnbr = p_cnbr; M.cedge = p_cedge; M.cinst = p_cinst; M.cown = p_cown;
-  M.bc = p_bc; M.fwthr = p_fw; M.area = p_area; M.zn = p_zn; M.ze = p_ze; M.cek = p_cek;
-  M.cnxc = p_cnxc; M.cnyc = p_cnyc; M.dry = p_dry; M.combo = p_combo; M.pw1 = p_pw1; M.pw2 = p_pw2;
+  M.bc = bed_.bc; M.fwthr = bed_.fwthr; M.area = p_area; M.zn = bed_.zn; M.ze = bed_.ze; M.cek = p_cek;
+  M.cnxc = p_cnxc; M.cnyc = p_cnyc; M.dry = bed_.dry; M.combo = bed_.combo; M.pw1 = bed_.pw1; M.pw2 = bed_.pw2;
   M.eown = p_eown; M.enb = p_enb; M.eslotl = p_esl; M.eslotr = p_esr; M.einst = p_einst;
-  M.enx = p_enx; M.eny = p_eny; M.etx = p_etx; M.ety = p_ety; M.ezm = p_ezm; M.elmin = p_elmin;
-  M.nz = p_nz; M.inst_cell_begin = p_icb; M.inst_cfl = p_cfl; M.inst_cor = p_cor;
-  M.srec = p_srec; M.cslot = p_cslot; M.erec = p_erec; M.eidx = p_eidx;
+  M.enx = p_enx; M.eny = p_eny; M.etx = p_etx; M.ety = p_ety; M.ezm = bed_.ezm; M.elmin = p_elmin;
+  M.enode = p_enode; M.nxy = p_nxy; M.nz = bed_.nz; M.inst_cell_begin = p_icb; M.inst_cfl = p_cfl; M.inst_cor = p_cor;
+  M.srec = bed_.srec; M.cslot = p_cslot; M.erec = bed_.erec; M.eidx = p_eidx;
   M.nptr = p_nptr; M.ncell = p_ncell;
 
   DevWork& Wk = work_;
@@ -804,14 +803,18 @@ std::string Engine::init(std::vector<HostInstance>&& inst, int flux, int ws, int
     return "stream creation failed";
   }
   stream_ = own_stream_;
+  host = std::move(inst);
+  const std::vector<double> nz = host_nz();
+  cudaError_t ce = compute_bed(nz.data());
   k_init_nodes<<<nblocks(N, 256), 256, 0, stream_>>>(M, Wk);
   ++launches_;
-  cudaError_t ce = cudaStreamSynchronize(stream_);
+  if (ce == cudaSuccess) ce = cudaGetLastError();
+  const cudaError_t cs = cudaStreamSynchronize(stream_);  // also on failure: the copy reads nz
+  if (ce == cudaSuccess) ce = cs;
   if (ce != cudaSuccess) {
     *st = 5;
     return std::string("CUDA error during set-up: ") + cudaGetErrorString(ce);
   }
-  host = std::move(inst);
   return "";
 }
 
@@ -1162,42 +1165,21 @@ std::string Engine::set_bathymetry(const std::vector<const double*>& z) {
     const Layout* L = q < layouts.size() ? &layouts[q] : nullptr;
     for (int64_t p = 0; p < h.N; ++p) h.geom[3 * p + 2] = z[q][(L && !L->identity()) ? L->node_from[p] : p];
   }
-  const int I = (int)host.size();
-  HostImage img;
-  img.resize(mesh_.C, mesh_.E, mesh_.N, I);
-  for (int q = 0; q < I; ++q) precompute_instance(host[q], q, cell_off[q], edge_off[q], node_off[q], img);
-  // the same arrays, in the order init uploaded them
-  size_t k = 0;
-  bool ok = true;
-  auto refill = [&](auto& vec) {
-    using T = typename std::remove_reference<decltype(vec)>::type::value_type;
-    if (!ok || k >= mesh_arrays_.size() || mesh_arrays_[k].second != vec.size() * sizeof(T)) {
-      ok = false;
-      return;
-    }
-    ok = cudaMemcpyAsync(mesh_arrays_[k].first, vec.data(), vec.size() * sizeof(T), cudaMemcpyHostToDevice,
-                         stream_) == cudaSuccess;
-    ++k;
-  };
-  refill(img.cnode); refill(img.cnbr); refill(img.cedge); refill(img.cinst);
-  refill(img.cown); refill(img.bc); refill(img.fwthr); refill(img.area);
-  refill(img.zn); refill(img.ze); refill(img.cek); refill(img.cnxc); refill(img.cnyc);
-  refill(img.dry); refill(img.combo); refill(img.pw1); refill(img.pw2);
-  refill(img.eown); refill(img.enb); refill(img.eslotl); refill(img.eslotr);
-  refill(img.einst); refill(img.enx); refill(img.eny); refill(img.etx);
-  refill(img.ety); refill(img.ezm); refill(img.elmin); refill(img.nz);
-  refill(img.inst_cell_begin); refill(img.inst_cfl); refill(img.inst_cor);
-  refill(img.srec); refill(img.cslot); refill(img.erec); refill(img.eidx);
-  refill(img.nptr); refill(img.ncell);
-  if (!ok || k != mesh_arrays_.size()) return "re-uploading the mesh records failed";
-  // the host image must outlive the asynchronous copies
-  cudaError_t e = cudaStreamSynchronize(stream_);
-  // the adjoint's tape and tables belong to the old bed
-  if (adj_) {
-    adjoint_state_delete(adj_);
-    adj_ = nullptr;
-  }
-  return e == cudaSuccess ? "" : std::string("re-uploading the mesh records: ") + cudaGetErrorString(e);
+  const std::vector<double> nz = host_nz();
+  cudaError_t e = compute_bed(nz.data());
+  // the adjoint's tape and plane tables belong to the old bed
+  if (adj_ && e == cudaSuccess) e = adjoint_state_new_bed(adj_, mesh_, stream_);
+  // nz must outlive the asynchronous copy
+  const cudaError_t es = cudaStreamSynchronize(stream_);
+  if (e == cudaSuccess) e = es;
+  return e == cudaSuccess ? "" : std::string("recomputing the mesh records: ") + cudaGetErrorString(e);
+}
+
+std::vector<double> Engine::host_nz() const {
+  std::vector<double> nz((size_t)mesh_.N);
+  for (size_t q = 0; q < host.size(); ++q)
+    for (int64_t p = 0; p < host[q].N; ++p) nz[node_off[q] + p] = host[q].geom[3 * p + 2];
+  return nz;
 }
 
 cudaError_t Engine::update_only(const Stage& st, const double* const* in, const double* const* u0,
