@@ -275,7 +275,7 @@ swe_status check_device(Engine& eng, std::string* err) {
 // Priming flux pass so that CFLdt() is defined before the first step.
 swe_status prime(Engine& eng, std::string* err) {
   cudaError_t e = eng.reset_pass();
-  if (e == cudaSuccess) e = eng.interface_values(eng.state(0, 0), eng.state(0, 1), eng.state(0, 2), 0);
+  if (e == cudaSuccess) e = eng.interface_values(eng.state(0, 0), eng.state(0, 1), eng.state(0, 2));
   if (e == cudaSuccess) e = eng.fluxes(eng.state(0, 0));
   if (e == cudaSuccess) e = eng.reset_pass();
   if (e != cudaSuccess) return cuda_fail(err, e, "priming flux pass");
@@ -554,14 +554,15 @@ swe_status swe_compute_interface_values(swe_ctx* ctx) {
   if (!ctx) return SWE_ERR_INVALID_ARGUMENT;
   Engine& g = ctx->eng;
   cudaError_t e = g.reset_pass();
-  if (e == cudaSuccess) e = g.interface_values(g.state(0, 0), g.state(0, 1), g.state(0, 2), 0);
+  if (e == cudaSuccess) e = g.interface_values(g.state(0, 0), g.state(0, 1), g.state(0, 2));
   if (e != cudaSuccess) return cuda_fail(&ctx->err, e, "swe_compute_interface_values");
   return SWE_OK;
 }
 
 swe_status swe_compute_fluxes(swe_ctx* ctx) {
   if (!ctx) return SWE_ERR_INVALID_ARGUMENT;
-  cudaError_t e = ctx->eng.fluxes(ctx->eng.state(0, 0));
+  cudaError_t e = ctx->eng.refresh_slots();
+  if (e == cudaSuccess) e = ctx->eng.fluxes(ctx->eng.state(0, 0));
   if (e != cudaSuccess) return cuda_fail(&ctx->err, e, "swe_compute_fluxes");
   return SWE_OK;
 }
@@ -622,7 +623,8 @@ swe_status swe_get_edge_values(swe_ctx* ctx, double* edg_out, double* src_out) {
   const int64_t C = g.C(), E = g.E();
   std::vector<double> ew(3 * C), eu(3 * C), ev(3 * C), sx(3 * C), sy(3 * C);
   const swe::DevWork& w = g.work();
-  cudaError_t e = cudaStreamSynchronize(g.stream());
+  cudaError_t e = g.refresh_slots();
+  if (e == cudaSuccess) e = cudaStreamSynchronize(g.stream());
   if (e == cudaSuccess) e = cudaMemcpy(ew.data(), w.ew, 3 * C * sizeof(double), cudaMemcpyDeviceToHost);
   if (e == cudaSuccess) e = cudaMemcpy(eu.data(), w.eu, 3 * C * sizeof(double), cudaMemcpyDeviceToHost);
   if (e == cudaSuccess) e = cudaMemcpy(ev.data(), w.ev, 3 * C * sizeof(double), cudaMemcpyDeviceToHost);

@@ -362,7 +362,7 @@ __device__ double pass1_node_value(const DevMesh& m, const DevWork& wk, const do
   const P1 p = pass1(wk, W, c);
   if (p.type == 0) return m.dry[(size_t)c * kDryStride + kn];
   double off = 0.;
-  if (p.type == 2 && p.kept) off = m.combo[combo_off(m.C, c, p.mask) + 8 + kn];
+  if (p.type == 2 && p.kept) off = m.combov[combov_off(m.C, c, p.mask) + kn];
   const double a = p.w0 + off;
   return dge0(a - z) ? a : z;
 }
@@ -656,7 +656,7 @@ __device__ void pw_jacobian(const DevMesh& m, const DevWork& wk, const AdjWork& 
       }
     } else {
       double off_n = 0.;
-      if (pc.type == 2 && pc.kept) off_n = m.combo[combo_off(m.C, best, pc.mask) + 8 + bestk];
+      if (pc.type == 2 && pc.kept) off_n = m.combov[combov_off(m.C, best, pc.mask) + bestk];
       if (dge0((pc.w0 + off_n) - zc_)) {
         J.target = best;
         if (pc.type == 2) {
@@ -750,7 +750,7 @@ __device__ void adj_recon_cell(const DevMesh& m, const DevWork& wk, AdjWork aw, 
       const double* rec = m.combo + combo_off(m.C, i, p.mask);
       gx = rec[0];
       gy = rec[1];
-      for (int k = 0; k < 3; ++k) off[k] = rec[5 + k];
+      for (int k = 0; k < 3; ++k) off[k] = rec[3 + k];
     }
   } else {
     J = aw.pwjac + i;
@@ -1262,13 +1262,13 @@ std::string Engine::adjoint_backward(const double* trace_grads_host, double* gra
             // the plain stage's kernels with PartWet2 and the fluxes next to
             // partially-wet cells on the side stream, keeping every
             // intermediate (k_drain_keep leaves the node maxima and the list)
-            launch_recon1(in[0], in[1], in[2], s == 0 ? 2 : 0);
+            launch_recon1(in[0], in[1], in[2], s == 0 ? 2 : 0, true);
             cudaEventRecord(ev_fork_, stream_);
             cudaStreamWaitEvent(side_, ev_fork_, 0);
-            launch_recon2(in[0], in[1], in[2], side_);
-            fluxes_pw(in[0], side_);
+            launch_recon2(in[0], in[1], in[2], side_, true);
+            stage_fluxes_pw(in, side_);
             cudaEventRecord(ev_join_, side_);
-            e = fluxes(in[0], 1);
+            e = stage_fluxes(in);
             cudaStreamWaitEvent(stream_, ev_join_, 0);
           }
           if (e == cudaSuccess) {
@@ -1389,7 +1389,7 @@ cudaError_t Engine::adjoint_stage_reverse(const Stage& st, const double* const* 
                                           AdjWork& aw) {
   // recompute the stage's forward intermediates from its input into work_
   cudaError_t e = reset_pass();
-  if (e == cudaSuccess) e = interface_values(in[0], in[1], in[2], 0);
+  if (e == cudaSuccess) e = interface_values(in[0], in[1], in[2]);
   if (e == cudaSuccess) e = fluxes(in[0]);
   if (e != cudaSuccess) return e;
   const int b = kReverseBlock;

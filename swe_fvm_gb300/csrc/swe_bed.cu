@@ -48,9 +48,48 @@ __device__ __forceinline__ P3 midpoint_of(const DevMesh& m, int e) {
   return t;
 }
 
+// Least double x for which the non-decreasing predicate holds (+inf: none), by
+// galloping and halving over the ordered bit patterns from the guess x0.
+template <class F>
+__device__ double least(double x0, F holds) {
+  const double inf = __longlong_as_double(0x7FF0000000000000ll);
+  if (!(x0 == x0)) return inf;
+  // k(x) monotone, consecutive doubles consecutive (both zeros at 0)
+  auto at = [](long long k) { return __longlong_as_double(k < 0 ? (long long)(0x8000000000000000ull - (unsigned long long)k) : k); };
+  const long long top = 0x7FF0000000000000ll;
+  long long k = __double_as_longlong(x0);
+  if (k < 0) k = -(k & 0x7FFFFFFFFFFFFFFFll);
+  long long lo, hi, step = 1;  // fails at lo, holds at hi
+  if (holds(at(k))) {
+    hi = k;
+    lo = k - step;
+    while (lo > -top && holds(at(lo))) {
+      hi = lo;
+      step <<= 1;
+      lo = (lo < -top + step) ? -top : lo - step;
+    }
+    if (lo <= -top) return at(hi);  // cannot happen: -inf is never wet
+  } else {
+    lo = k;
+    hi = k + step;
+    while (hi < top && !holds(at(hi))) {
+      lo = hi;
+      step <<= 1;
+      hi = (hi > top - step) ? top : hi + step;
+    }
+    if (hi >= top) return inf;
+  }
+  while (hi - lo > 1) {
+    const long long mid = lo + (hi - lo) / 2;
+    if (holds(at(mid))) hi = mid;
+    else lo = mid;
+  }
+  return at(hi);
+}
+
 // Fully-wet cell plane for one wet / part-wet neighbour combination
 // (src/MUSCLObject.cpp:38-84); bit k of mask set = neighbour k partially wet.
-__device__ void plane_record(const DevMesh& m, int i, int mask, double* rec) {
+__device__ void plane_record(const DevMesh& m, int i, int mask, double* rec, double* recv) {
   const int C = m.C;
   P3 P[3], E[3], Q[3];
   bool boundary = false;
@@ -63,6 +102,8 @@ __device__ void plane_record(const DevMesh& m, int i, int mask, double* rec) {
   if (boundary) {  // never fully wet
 #pragma unroll
     for (int q = 0; q < kComboStride; ++q) rec[q] = 0.;
+#pragma unroll
+    for (int q = 0; q < kComboVStride; ++q) recv[q] = 0.;
     return;
   }
 #pragma unroll
@@ -78,6 +119,7 @@ __device__ void plane_record(const DevMesh& m, int i, int mask, double* rec) {
   const double diag = 1. - third;
   rec[0] = g0;
   rec[1] = g1;
+  double level = 0.;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     double dx[2];
@@ -88,11 +130,16 @@ __device__ void plane_record(const DevMesh& m, int i, int mask, double* rec) {
       const double m2 = (k == 2) ? diag : -third;
       dx[r] = P[0][r] * m0 + P[1][r] * m1 + P[2][r] * m2;
     }
-    rec[2 + k] = g0 * dx[0] + g1 * dx[1];                                // positivity offsets
-    rec[5 + k] = g0 * (E[k][0] - t[0]) + g1 * (E[k][1] - t[1]);          // edge-centre offsets
-    rec[8 + k] = g0 * (P[k][0] - t[0]) + g1 * (P[k][1] - t[1]);          // vertex offsets
+    // positivity of the vertex, is_wet((off + w) - z): its rounded sums are
+    // non-decreasing in w, so it holds from one level on, kept in place of the
+    // offset (the reconstruction then compares instead of adding six times)
+    const double off = g0 * dx[0] + g1 * dx[1], z = P[k][2];
+    const double from = least((z + kWetDepth) - off, [&](double w) { return is_wet((off + w) - z); });
+    level = k == 0 ? from : smax(level, from);
+    rec[3 + k] = g0 * (E[k][0] - t[0]) + g1 * (E[k][1] - t[1]);  // edge-centre offsets
+    recv[k] = g0 * (P[k][0] - t[0]) + g1 * (P[k][1] - t[1]);     // vertex offsets
   }
-  rec[11] = 0.;
+  rec[2] = level;
 }
 
 // Scalars, dry plane, PartWet1 and PartWet2 records of cell i.
@@ -109,6 +156,7 @@ __device__ void cell_record(const DevMesh& m, const BedArrays& o, int i) {
   const P3 t = centroid(P[0], P[1], P[2]);
   const double bc = t[2];
   o.bc[i] = bc;
+  o.wetthr[i] = least(bc + kWetDepth, [&](double w) { return is_wet(w - bc); });
   // src/MUSCLObject.cpp:17-25 (maxCoeff of the node z)
   double mx = P[0][2];
   if (dlt(mx, P[1][2])) mx = P[1][2];
@@ -125,6 +173,7 @@ __device__ void cell_record(const DevMesh& m, const BedArrays& o, int i) {
   double sx, sy;
   plane_gradient(P[0][0], P[0][1], P[0][2], P[1][0], P[1][1], P[1][2], P[2][0], P[2][1], P[2][2], &sx, &sy);
   double* dr = o.dry + (size_t)i * kDryStride;
+  bool wet_slots = false;  // (a plane through the bed: only by rounding)
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     const double a = bc + (sx * (P[k][0] - t[0]) + sy * (P[k][1] - t[1]));
@@ -132,9 +181,11 @@ __device__ void cell_record(const DevMesh& m, const BedArrays& o, int i) {
     const double e = bc + (sx * (E[k][0] - t[0]) + sy * (E[k][1] - t[1]));
     const double at = dge0(e - E[k][2]) ? e : E[k][2];
     dr[3 + k] = is_wet(at - E[k][2]) ? at : E[k][2];
+    wet_slots = wet_slots || is_wet(at - E[k][2]);
   }
   dr[6] = sx;
   dr[7] = sy;
+  o.cown[i] = (unsigned char)((o.cown[i] & 7u) | (wet_slots ? 8u : 0u));
   // PartWet1 (src/MUSCLObject.cpp:86-112)
   {
     double b13 = P[0][2], b23 = P[0][2];
@@ -210,7 +261,7 @@ __global__ void __launch_bounds__(128) k_bed_cells(DevMesh m, BedArrays o) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m.C) return;
   const int part = blockIdx.y;
-  if (part < 8) plane_record(m, i, part, o.combo + combo_off(m.C, i, part));
+  if (part < 8) plane_record(m, i, part, o.combo + combo_off(m.C, i, part), o.combov + combov_off(m.C, i, part));
   else cell_record(m, o, i);
 }
 

@@ -20,18 +20,24 @@
 
 namespace swe {
 
-constexpr int kComboStride = 12;  // doubles per full-wet combination record
+constexpr int kComboStride = 6;   // doubles per full-wet combination record
+constexpr int kComboVStride = 3;  // its vertex offsets, kept apart
 constexpr int kPw1Stride = 12;    // doubles per PartWet1 record
 constexpr int kDryStride = 8;     // doubles per dry-cell record
 
 enum : unsigned { kErrNonFinite = 1u, kErrBadState = 2u, kErrBadIndex = 4u };
 
-// The full-wet combination records are stored combination-major, [8][C][12]:
+// The full-wet combination records are stored combination-major, [8][C][6]:
 // the record of cell i for neighbour combination `mask` starts here.  Nearly
 // every fully-wet cell has only fully-wet neighbours (mask 0), so the records
-// a warp reads are contiguous.
+// a warp reads are contiguous.  A record is the slope (x, y), the level from
+// which the plane is positive at the vertices, and the three edge-centre
+// offsets; the vertex offsets, which only node maxima read, are [8][C][3].
 __host__ __device__ __forceinline__ size_t combo_off(int C, int i, int mask) {
   return ((size_t)mask * (size_t)C + (size_t)i) * kComboStride;
+}
+__host__ __device__ __forceinline__ size_t combov_off(int C, int i, int mask) {
+  return ((size_t)mask * (size_t)C + (size_t)i) * kComboVStride;
 }
 
 // Static per-slot record read by the update kernel with two 16-byte loads:
@@ -69,8 +75,9 @@ struct DevMesh {
   const int* cnode;           // [3][C]
   const int* cnbr;            // [3][C], -1 = wall
   const int* cedge;           // [3][C]
-  const unsigned char* cown;  // [C] bit k: this cell owns edge k
+  const unsigned char* cown;  // [C] bit k: this cell owns edge k; bit 3: a slot of its dry plane is wet
   const double* bc;           // [C] centroid bathymetry
+  const double* wetthr;       // [C] least w whose depth w - bc is wet
   const double* fwthr;        // [C] max node z, +inf for boundary cells
   const double* area;         // [C]
   const double* zn;           // [3][C] node z
@@ -79,7 +86,8 @@ struct DevMesh {
   const double* cnxc;         // [3][C] outward normal of edge k times L_k / A (x)
   const double* cnyc;         // [3][C] (y)
   const double* dry;          // [C][8] dry-cell node/edge values and slope
-  const double* combo;        // [8][C][12] full-wet plane records (combo_off)
+  const double* combo;        // [8][C][6] full-wet plane records (combo_off)
+  const double* combov;       // [8][C][3] their vertex offsets (combov_off)
   const double* pw1;          // [C][12]
   const Pw2Rec* pw2;          // [C]
   const int* cinst;           // [C] instance of the cell (batched only)
@@ -117,17 +125,25 @@ struct DevMesh {
 // The records that depend on the bathymetry, as the device computes them
 // (DevMesh's arrays of the same names).
 struct BedArrays {
-  double *bc, *fwthr, *zn, *ze, *dry, *combo, *pw1, *ezm, *nz;
+  double *bc, *wetthr, *fwthr, *zn, *ze, *dry, *combo, *combov, *pw1, *ezm, *nz;
   Pw2Rec* pw2;
+  unsigned char* cown;  // bit 3 only
   SlotRec* srec;  // ze only
   EdgeRec* erec;  // b only
 };
 
 struct DevWork {
+  // what a stage passes on: the depth at each slot (0 where not wet; the slot's
+  // velocity then follows from the cell's) and the cell's source gradient
+  double* eh;  // [3][C]
+  double* gx;  // [C]
+  double* gy;
+  // the reference's interface values and source slots in full, for the getters
+  // and the adjoint (k_recon1, k_recon2 with SLOTS)
   double* ew;  // [3][C] interface w
   double* eu;
   double* ev;
-  double* sx;  // [3][C] source gradient
+  double* sx;  // [3][C] source gradient with the Coriolis term
   double* sy;
   double* f0;  // [E] fluxes
   double* f1;
@@ -267,9 +283,14 @@ class Engine {
   // Resets the node maxima and the part-wet list (done by k_drain at the end
   // of every stage; needed before a standalone reconstruction).
   cudaError_t reset_pass();
-  // Launches one reconstruction (pass 1 + pass 2) and one flux pass.
-  cudaError_t interface_values(const double* W, const double* U, const double* V, int latch_mode);
+  // Launches one reconstruction (pass 1 + pass 2) with the full interface
+  // values, and one flux pass from them.
+  cudaError_t interface_values(const double* W, const double* U, const double* V);
   cudaError_t fluxes(const double* W);
+  // The full interface values as of the last reconstruction: a step of several
+  // stages leaves only what its own kernels read, and the rest is written here
+  // from the last stage's input, which the step keeps.
+  cudaError_t refresh_slots();
   // One whole step of `scheme`; latch_mode 1 = CFL dt, 2 = fixed dt from
   // work.fixed_dt.  Enqueued on the engine's stream.
   cudaError_t step(int scheme, int latch_mode);
@@ -364,12 +385,16 @@ class Engine {
   bool batched_ = false;
   bool cor0_ = true;  // every instance has cor = 0: no Coriolis arithmetic in the reconstruction
   double* d_integrals_ = nullptr;  // partial sums of the integrals
-  void launch_recon1(const double* W, const double* U, const double* V, int latch_mode);
-  void launch_recon2(const double* W, const double* U, const double* V, cudaStream_t s);
-  // fluxes: mode 0 every edge; mode 1 the edges with no partially-wet cell;
-  // fluxes_pw: the others (those of the listed cells), on stream s
-  cudaError_t fluxes(const double* W, int mode);
-  void fluxes_pw(const double* W, cudaStream_t s);
+  // slots: also the full interface values (DevWork::ew ...).  latch_mode: 0
+  // none, 1 the CFL dt, 2 the fixed dt, 3 none and the CFL ratio kept
+  void launch_recon1(const double* W, const double* U, const double* V, int latch_mode, bool slots);
+  void launch_recon2(const double* W, const double* U, const double* V, cudaStream_t s, bool slots);
+  // the fluxes of a stage's input: the edges with no partially-wet cell, and
+  // the others (those of the listed cells) on stream s
+  cudaError_t stage_fluxes(const double* const* in);
+  void stage_fluxes_pw(const double* const* in, cudaStream_t s);
+  bool soft_ = false;         // the step's products on the integer pipe (kSoftCells)
+  bool slots_stale_ = false;  // a step of several stages ran since the slots were written
   void launch_update(const Stage& st, const double* const* in, const double* const* u0, double* const* out,
                      double* nst);
   int64_t launches_ = 0;

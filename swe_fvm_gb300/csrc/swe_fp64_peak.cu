@@ -138,11 +138,12 @@ extern "C" swe_status swe_selftest_fp64(int64_t n, uint64_t seed, int64_t* div_m
 // way to the same bits, on the caller's operands (host or device build).
 namespace {
 
-// operands per result: 0 bisection (d, c, b, xmin, xmax), 1 cube root
-__host__ __device__ constexpr int pointwise_args(int kind) { return kind == 0 ? 5 : 1; }
+// operands per result: 0 bisection (d, c, b, xmin, xmax), 1 cube root, 2 product
+__host__ __device__ constexpr int pointwise_args(int kind) { return kind == 0 ? 5 : kind == 1 ? 1 : 2; }
 __host__ __device__ double pointwise(int kind, const double* a) {
   if (kind == 0) return swe::bisection(a[0], a[1], a[2], a[3], a[4]);
-  return swe::cbrt_rn(a[0]);
+  if (kind == 1) return swe::cbrt_rn(a[0]);
+  return a[0] * a[1];
 }
 __global__ void k_pointwise(int kind, int n, const double* in, double* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -152,7 +153,7 @@ __global__ void k_pointwise(int kind, int n, const double* in, double* out) {
 }  // namespace
 
 extern "C" swe_status swe_selftest_pointwise(int32_t kind, int64_t n, const double* in, double* out, int32_t device) {
-  if (kind < 0 || kind > 1 || n <= 0 || n > (1 << 26) || !in || !out) return SWE_ERR_INVALID_ARGUMENT;
+  if (kind < 0 || kind > 2 || n <= 0 || n > (1 << 26) || !in || !out) return SWE_ERR_INVALID_ARGUMENT;
   const size_t m = pointwise_args(kind);
   if (!device) {
     for (int64_t i = 0; i < n; ++i) out[i] = pointwise(kind, in + i * m);

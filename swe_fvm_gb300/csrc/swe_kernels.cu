@@ -55,6 +55,7 @@ namespace {
 
 constexpr double kInf = __builtin_huge_val();
 
+
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 
 // start moving the cache line of p towards this SM's L1 (no register, no wait)
@@ -86,16 +87,26 @@ __device__ __forceinline__ double add_zero_product(double x, double c, double v)
   return dfrom((long long)(ux & (uc ^ uv) & 0x8000000000000000ull));
 }
 
-template <bool COR0>
-__device__ __forceinline__ void write_slot(const DevWork& wk, int slot, double be, double w, double u, double v,
+// How a reconstruction writes a slot.  What the step's own kernels read is the
+// depth (kLean): h = w - b where wet, else 0.  The slot's velocity is the
+// cell's, zeroed or desingularised by that depth (slot_velocity), and the
+// source gradient is one per cell.  The full form (kSlots, with or without
+// Coriolis) adds the reference's interface values and source slots, for the
+// getters and the adjoint: 120 B a cell more, which is why the step leaves them.
+enum : int { kLean = 0, kSlotsCor0 = 1, kSlotsCor = 2 };
+
+template <int FORM>
+__device__ __forceinline__ void write_slot(const DevWork& wk, int slot, double h, double be, double w, double u, double v,
                                            double gx, double gy, double cor) {
+  wk.eh[slot] = is_wet(h) ? h : 0.;  // h = w - be
+  if (FORM == kLean) return;
   double ow, ou, ov;
   prim_assign(be, w, u, v, &ow, &ou, &ov);
   wk.ew[slot] = ow;
   wk.eu[slot] = ou;
   wk.ev[slot] = ov;
   double sx = gx, sy = gy;
-  if (COR0) {
+  if (FORM == kSlotsCor0) {
     const double nov = dfrom(dbits(ov) ^ (long long)0x8000000000000000ull);
     sx = add_zero_product(gx, cor, nov);
     sy = add_zero_product(gy, cor, ou);
@@ -105,6 +116,32 @@ __device__ __forceinline__ void write_slot(const DevWork& wk, int slot, double b
   }
   wk.sx[slot] = sx;
   wk.sy[slot] = sy;
+}
+
+// The velocity at a slot of depth h (eh) in a cell with velocity (u, v), as
+// UpdateInterfaceValues assigns it (src/Assigners.cpp:8-20): zero where the
+// slot or the whole cell is dry, desingularised where it is thin.
+__device__ __forceinline__ void slot_velocity(double h, bool dry_cell, double* u, double* v) {
+  if (dry_cell || !is_wet(h)) {
+    *u = 0.;
+    *v = 0.;
+  } else if (dltc(h, kEta1)) {
+    const double s = SWE_DIV(kSqrt2 * h, SWE_SQRT(h * h + kEta2));
+    *u *= s;
+    *v *= s;
+  }
+}
+
+// 0 - x: -x, but +0 for either zero
+__device__ __forceinline__ double zero_minus(double x) {
+  const unsigned long long u = ubits(x);
+  return ufrom((u << 1) == 0ull ? 0ull : u ^ 0x8000000000000000ull);
+}
+
+// 0 x: a zero of x's sign (NaN where x is not finite)
+__device__ __forceinline__ double zero_times(double x) {
+  const unsigned long long u = ubits(x);
+  return ufrom((~u & 0x7FF0000000000000ull) == 0ull ? 0x7FF8000000000000ull : u & 0x8000000000000000ull);
 }
 
 // MUSCL::AtPoint with a w-only plane (include/MUSCLObject.h:26-33): the value
@@ -133,7 +170,7 @@ __device__ __forceinline__ double pass1_value(const DevMesh& m, const DevWork& w
     at_point_wet(wk.pwrec[c], 0., z, &val);  // the PartWet1 level, a flat plane
   } else {
     // the combination plane's vertex offset when pass 1 kept the plane, else flat
-    const double off = (cl & 32u) ? m.combo[combo_off(C, c, (int)((cl >> 2) & 7u)) + 8 + kn] : 0.;
+    const double off = (cl & 32u) ? m.combov[combov_off(C, c, (int)((cl >> 2) & 7u)) + kn] : 0.;
     at_point_wet(W[c], off, z, &val);
   }
   return val;
@@ -180,7 +217,11 @@ __device__ __forceinline__ double partwet1_level(const double* __restrict__ p, d
 }
 
 // ---------------------------------------------------------------- kernels
-template <bool BATCH, bool COR0>
+// Pass 1.  Bound by its gathers and, on wetting fronts, by PartWet1's chain.
+// The wet test and the plane's positivity are comparisons with levels kept in
+// the mesh (DevMesh::wetthr, record entry 2) where the rounded sums would cost
+// seven FP64 operations; 6 are left in a fully-wet cell of 18.
+template <bool BATCH, int FORM>
 __global__ void __launch_bounds__(256, 5) k_recon1(DevMesh m, DevWork wk, const double* __restrict__ W,
                                                 const double* __restrict__ U, const double* __restrict__ V,
                                                 int latch_mode) {
@@ -189,7 +230,7 @@ __global__ void __launch_bounds__(256, 5) k_recon1(DevMesh m, DevWork wk, const 
   unsigned char cls = 0;  // dry unless set below
   if (i < m.C) {
     const int inst = BATCH ? m.cinst[i] : 0;
-    if (i == (BATCH ? m.inst_cell_begin[inst] : 0)) {
+    if (latch_mode != 3 && i == (BATCH ? m.inst_cell_begin[inst] : 0)) {
       if (latch_mode == 1) {  // dt = TimeDisc::CFLdt() of the previous flux pass
         double dt = m.inst_cfl[inst] * order_val(wk.r[inst]);
         wk.dt[inst] = dt;
@@ -203,24 +244,30 @@ __global__ void __launch_bounds__(256, 5) k_recon1(DevMesh m, DevWork wk, const 
     }
     const int C = m.C;
     // the combination record of the all-fully-wet neighbourhood (mask 0) is
-    // the one nearly every fully-wet cell reads: start its lines towards L1
+    // the one nearly every fully-wet cell reads: start its line towards L1
     // now, before the loads that decide the class and the mask
     prefetch_l1(m.combo + combo_off(C, i, 0));
-    prefetch_l1(m.combo + combo_off(C, i, 0) + 8);
-    const double cor = m.inst_cor[inst];
-    const double w = W[i], u = U[i], v = V[i];
-    const double h = w - m.bc[i];
-    if (!is_wet(h)) {
+    const double cor = FORM == kSlotsCor ? m.inst_cor[inst] : FORM == kSlotsCor0 ? m.inst_cor[inst] : 0.;
+    const double w = W[i];
+    const double u = FORM == kLean ? 0. : U[i], v = FORM == kLean ? 0. : V[i];
+    double gx = 0., gy = 0.;
+    if (dlt(w, m.wetthr[i])) {
       // ReconstructDryCell: every value is a mesh constant
       const double* dr = m.dry + (size_t)i * kDryStride;
+      gx = dr[6];
+      gy = dr[7];
+      const bool wet_slots = (m.cown[i] & 8u) != 0u;
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
         const int slot = k * C + i;
-        write_slot<COR0>(wk, slot, m.ze[slot], dr[3 + k], 0., 0., dr[6], dr[7], cor);
+        // (a dry cell's own slots are dry but for rounding, which the mesh record tells)
+        const double be = FORM != kLean || wet_slots ? m.ze[slot] : 0.;
+        const double h = wet_slots ? dr[3 + k] - be : 0.;
+        write_slot<FORM>(wk, slot, h, be, FORM == kLean ? 0. : dr[3 + k], 0., 0., gx, gy, cor);
       }
     } else if (!dlt(m.fwthr[i], w)) {
       // partially wet: the PartWet1 level now, PartWet2 in k_recon2
-      wk.pwrec[i] = partwet1_level(m.pw1 + (size_t)i * kPw1Stride, w, h);
+      wk.pwrec[i] = partwet1_level(m.pw1 + (size_t)i * kPw1Stride, w, w - m.bc[i]);
       part = true;
       cls = 1;
     } else {
@@ -235,56 +282,52 @@ __global__ void __launch_bounds__(256, 5) k_recon1(DevMesh m, DevWork wk, const 
         wn[k] = wj;
         if (dlt(m.fwthr[nb], wj)) {
           // fully-wet neighbour: plane point at its centroid
-        } else if (!is_wet(wj - m.bc[nb])) {
+        } else if (dlt(wj, m.wetthr[nb])) {
           first_order = true;
         } else {
           mask |= 1 << k;  // partially-wet neighbour: plane point at the edge centre
         }
       }
       cls = (unsigned char)(2 | (mask << 2));
-      double gx = 0., gy = 0.;
-      double toff[3] = {0., 0., 0.};
+      double at[3] = {w, w, w};  // the plane's level at the edge centres
       if (!first_order) {
-        const double* rec = m.combo + combo_off(C, i, mask);
-        const double g0 = rec[0], g1 = rec[1];
-        bool pos = true;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          const double hp = (rec[2 + k] + w) - m.zn[k * C + i];
-          if (!is_wet(hp)) pos = false;
-        }
-        if (pos) {
+        const double2* rec = (const double2*)(m.combo + combo_off(C, i, mask));
+        const double2 g = __ldg(rec), p = __ldg(rec + 1), q = __ldg(rec + 2);
+        if (dle(p.x, w)) {  // positive at the three vertices
           // binary TVD limiter on the w row (rows u, v of df are zero)
+          const double vek[3] = {w + p.y, w + q.x, w + q.y};
           bool tvd = true;
 #pragma unroll
-          for (int k = 0; k < 3; ++k) {
-            const double vmin = smin(w, wn[k]), vmax = smax(w, wn[k]);
-            const double vek = w + rec[5 + k];
-            if (!(dle(vmin, vek) && dle(vek, vmax))) tvd = false;
-          }
+          for (int k = 0; k < 3; ++k)
+            if (!(dle(smin(w, wn[k]), vek[k]) && dle(vek[k], smax(w, wn[k])))) tvd = false;
           if (tvd) {
             cls |= 32;  // combination plane kept
-            gx = g0;
-            gy = g1;
+            gx = g.x;
+            gy = g.y;
 #pragma unroll
-            for (int k = 0; k < 3; ++k) toff[k] = rec[5 + k];
+            for (int k = 0; k < 3; ++k) at[k] = vek[k];
           } else {
-            gx = 0. * g0;  // diag(TVD) * df keeps the sign of zero
-            gy = 0. * g1;
+            gx = zero_times(g.x);  // diag(TVD) * df keeps the sign of zero
+            gy = zero_times(g.y);
           }
         }
       }
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
         const int slot = k * C + i;
-        const double be = m.ze[slot];
-        double we;
-        if (at_point_wet(w, toff[k], be, &we)) write_slot<COR0>(wk, slot, be, we, u, v, gx, gy, cor);
-        else write_slot<COR0>(wk, slot, be, we, 0., 0., gx, gy, cor);
+        // AtPoint below the bed gives (b, 0, 0), and so does a slot that is not
+        // wet: one rule for both
+        const double be = m.ze[slot], h = at[k] - be;
+        const bool above = dge0(h);
+        write_slot<FORM>(wk, slot, h, be, above ? at[k] : be, above ? u : 0., above ? v : 0., gx, gy, cor);
       }
     }
+    if (!part) {
+      wk.gx[i] = gx;
+      wk.gy[i] = gy;
+    }
+    wk.cls[i] = cls;
   }
-  if (i < m.C) wk.cls[i] = cls;
   // warp-aggregated append of the partially-wet cells
   const unsigned bal = __ballot_sync(0xffffffffu, part);
   if (bal) {
@@ -306,7 +349,7 @@ __global__ void k_node_max_all(DevMesh m, DevWork wk, const double* __restrict__
 }
 
 // ReconstructPartWetCell2 (src/MUSCLObject.cpp:114-191) over the listed cells.
-template <bool BATCH, bool COR0>
+template <bool BATCH, int FORM>
 __global__ void __launch_bounds__(256) k_recon2(DevMesh m, DevWork wk, const double* __restrict__ W,
                                                 const double* __restrict__ U, const double* __restrict__ V) {
   const int C = m.C;
@@ -315,7 +358,8 @@ __global__ void __launch_bounds__(256) k_recon2(DevMesh m, DevWork wk, const dou
     const int i = gidx(wk, wk.pwlist[q], C);
     const int inst = BATCH ? m.cinst[i] : 0;
     const double cor = m.inst_cor[inst];
-    const double w = W[i], u = U[i], v = V[i];
+    const double w = W[i];
+    const double u = FORM == kLean ? 0. : U[i], v = FORM == kLean ? 0. : V[i];
     const Pw2Rec& r = m.pw2[i];
     const double b23 = r.p[0][2], b12 = r.p[1][2], b13 = r.p[2][2];
     double w0 = wk.pwrec[i];  // PartWet1 fallback level
@@ -377,19 +421,26 @@ __global__ void __launch_bounds__(256) k_recon2(DevMesh m, DevWork wk, const dou
       const int slot = k * C + i;
       const double be = m.ze[slot];
       const double off = plane ? (gx * r.dedge[k][0] + gy * r.dedge[k][1]) : 0.;
-      double we;
-      if (at_point_wet(w0, off, be, &we)) write_slot<COR0>(wk, slot, be, we, u, v, gx, gy, cor);
-      else write_slot<COR0>(wk, slot, be, we, 0., 0., gx, gy, cor);
+      const double at = w0 + off, h = at - be;
+      const bool above = dge0(h);
+      write_slot<FORM>(wk, slot, h, be, above ? at : be, above ? u : 0., above ? v : 0., gx, gy, cor);
     }
+    wk.gx[i] = gx;
+    wk.gy[i] = gy;
   }
 }
 
 // SpaceDisc::ComputeFluxes with flux plugin FLUX and the CFL min-reduction.
 // The flux of edge e (src/SpaceDisc.cpp:54-74) into f0..f2; *lw receives its
-// length-to-wavespeed ratio or stays +inf.
-template <class FLUX, bool TAPE>
-__device__ __forceinline__ void flux_edge(const DevMesh& m, const DevWork& wk, const double* __restrict__ W, int e,
-                                          int inst, double* lw) {
+// length-to-wavespeed ratio or stays +inf.  SLOTS: from the full interface
+// values (swe_compute_fluxes), else from the depths and the cells' velocities.
+// Returns false where a product left the integer routine's range (nothing of
+// use is stored then; the caller evaluates the edge again with SOFT = false).
+template <class FLUX, bool TAPE, bool SOFT, bool SLOTS>
+__device__ __forceinline__ bool flux_edge(const DevMesh& m, const DevWork& wk, const double* __restrict__ W,
+                                          const double* __restrict__ U, const double* __restrict__ V, int e, int inst,
+                                          double* lw) {
+  Products<SOFT> prod;
   const int4 ix = __ldg(m.eidx + e);  // (owner, neighbour, owner's slot, neighbour's slot)
   const int o = gidx(wk, ix.x, m.C);
   const int nb = ix.y;
@@ -408,26 +459,41 @@ __device__ __forceinline__ void flux_edge(const DevMesh& m, const DevWork& wk, c
     g.b = bl.x;
     g.lmin = bl.y;
     const int sl = gidx(wk, ix.z, 3 * m.C), sr = gidx(wk, ix.w, 3 * m.C);
-    SideState L{wk.ew[sl], wk.eu[sl], wk.ev[sl]};
-    SideState R{wk.ew[sr], wk.eu[sr], wk.ev[sr]};
-    if (TAPE) FLUX::eval(g, L, R, m.inst_cor[inst], lw, F, EdgeTape{wk.ftape, m.E, e});
-    else FLUX::eval(g, L, R, m.inst_cor[inst], lw, F);
+    DepthState L, R;
+    if (SLOTS) {
+      L = depth_state(SideState{wk.ew[sl], wk.eu[sl], wk.ev[sl]}, g.b);
+      R = depth_state(SideState{wk.ew[sr], wk.eu[sr], wk.ev[sr]}, g.b);
+    } else {
+      const int n = gidx(wk, nb, m.C);
+      L = DepthState{wk.eh[sl], U[o], V[o]};
+      R = DepthState{wk.eh[sr], U[n], V[n]};
+      slot_velocity(L.h, (wk.cls[o] & 3u) == 0u, &L.u, &L.v);
+      slot_velocity(R.h, (wk.cls[n] & 3u) == 0u, &R.u, &R.v);
+    }
+    const double cor = m.inst_cor[inst];
+    // the minimum so far (a stale one is only larger)
+    const int cap = (int)((__ldcg(wk.r + inst) >> 32) & 0x7FFFFFFFull);
+    if (TAPE) FLUX::eval_depth(prod, g, L, R, cor, cap, lw, F, EdgeTape{wk.ftape, m.E, e});
+    else FLUX::eval_depth(prod, g, L, R, cor, cap, lw, F, NoTape{});
   }
   wk.f0[e] = F[0];
   wk.f1[e] = F[1];
   wk.f2[e] = F[2];
+  return !prod.other;
 }
 
-// MODE 0: every edge.  MODE 1: the edges none of whose cells is partially
-// wet (the others wait for PartWet2 and go through k_flux_pw).
+// MODE 0: every edge, from the full interface values.  MODE 1: the edges none
+// of whose cells is partially wet (the others wait for PartWet2 and go through
+// k_flux_pw).
 // TAPE: also store the intermediates the adjoint's reverse reads (wk.ftape).
 // Register caps (the second __launch_bounds__ argument: blocks of 256 threads
 // per SM) measured on the 1M-cell dam break, CUDA events, same bits: k_flux at
 // 64 registers 0.211 -> 0.199 ms per launch, k_recon1 at 48 registers
 // 0.091 -> 0.087 ms; more resident warps hide the gathers better than the
 // few spilled registers cost.
-template <class FLUX, bool BATCH, int MODE, bool TAPE>
-__global__ void __launch_bounds__(256, 4) k_flux(DevMesh m, DevWork wk, const double* __restrict__ W) {
+template <class FLUX, bool BATCH, int MODE, bool TAPE, bool SOFT>
+__global__ void __launch_bounds__(256, 4) k_flux(DevMesh m, DevWork wk, const double* __restrict__ W,
+                                                 const double* __restrict__ U, const double* __restrict__ V) {
   __shared__ unsigned long long s_min[32];
   __shared__ int s_inst[32];
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -440,7 +506,10 @@ __global__ void __launch_bounds__(256, 4) k_flux(DevMesh m, DevWork wk, const do
       const int nb = m.enb[e];
       mine = !(((wk.cls[gidx(wk, m.eown[e], m.C)] & 3) == 1) || (nb >= 0 && (wk.cls[gidx(wk, nb, m.C)] & 3) == 1));
     }
-    if (mine) flux_edge<FLUX, TAPE>(m, wk, W, e, inst, &lw);
+    if (mine && !flux_edge<FLUX, TAPE, SOFT, MODE == 0>(m, wk, W, U, V, e, inst, &lw)) {
+      lw = kInf;
+      flux_edge<FLUX, TAPE, false, MODE == 0>(m, wk, W, U, V, e, inst, &lw);
+    }
   }
   // min-reduction of the length-to-wavespeed ratio on order-preserving integer
   // keys (exact): warp, block, one atomicMin per block and instance
@@ -490,7 +559,8 @@ __global__ void __launch_bounds__(256, 4) k_flux(DevMesh m, DevWork wk, const do
 // PartWet2): listed cell i takes its local edge k unless the edge's owner is
 // partially wet too and is not i, so that each edge is evaluated once.
 template <class FLUX, bool BATCH, bool TAPE>
-__global__ void __launch_bounds__(128) k_flux_pw(DevMesh m, DevWork wk, const double* __restrict__ W) {
+__global__ void __launch_bounds__(128) k_flux_pw(DevMesh m, DevWork wk, const double* __restrict__ W,
+                                                 const double* __restrict__ U, const double* __restrict__ V) {
   const int C = m.C;
   const int n = 3 * min(*wk.pwcount, C);
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
@@ -501,14 +571,17 @@ __global__ void __launch_bounds__(128) k_flux_pw(DevMesh m, DevWork wk, const do
     if ((((wk.cls[o] & 3) == 1) ? o : m.enb[e]) != i) continue;
     const int inst = BATCH ? m.einst[e] : 0;
     double lw = kInf;
-    flux_edge<FLUX, TAPE>(m, wk, W, e, inst, &lw);
+    flux_edge<FLUX, TAPE, false, false>(m, wk, W, U, V, e, inst, &lw);
     if (dbits(lw) != dbits(kInf)) atomicMin(wk.r + inst, order_key(lw));
   }
 }
 
 // TimeDisc::ComputeDrainingDt once per cell; also empties the part-wet list
-// for the next reconstruction.
-__global__ void __launch_bounds__(256) k_drain(DevMesh m, DevWork wk, const double* __restrict__ W) {
+// for the next reconstruction.  The update only takes minima with the stage's
+// dt, so a cell that plainly outlasts it (A h > 2 dt sum, dt_scale = 2 max(1, c)
+// times the step's dt) keeps +inf and no quotient.
+template <bool BATCH>
+__global__ void __launch_bounds__(256) k_drain(DevMesh m, DevWork wk, const double* __restrict__ W, double dt_scale) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) *wk.pwcount = 0;
   if (i >= m.C) return;
@@ -518,13 +591,18 @@ __global__ void __launch_bounds__(256) k_drain(DevMesh m, DevWork wk, const doub
     d = 0.;
   } else {
     const unsigned own = m.cown[i];
-    double sum = 0.;
+    double out[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       const double f = wk.f0[gidx(wk, m.cedge[k * m.C + i], m.E)];
-      sum += smax(0., ((own >> k) & 1u) ? f : -f);
+      out[k] = smax(0., ((own >> k) & 1u) ? f : SWE_NEG(f));
     }
-    d = dgtc(sum, kTol) ? SWE_DIV(m.area[i] * h, sum) : kInf;
+    const double sum = out[0] + out[1] + out[2];  // 0 + out[0] is out[0]
+    d = kInf;
+    if (dgtc(sum, kTol)) {
+      const double vol = m.area[i] * h;
+      if (!dlt(sum * (dt_scale * wk.dt[BATCH ? m.cinst[i] : 0]), vol)) d = SWE_DIV(vol, sum);
+    }
   }
   wk.drain[i] = d;
 }
@@ -536,18 +614,39 @@ __global__ void __launch_bounds__(256) k_drain(DevMesh m, DevWork wk, const doub
 // adjoint's segment recompute).
 // HALF: a stage with a = b = c = 1/2 (SSPRK2's second), whose products with
 // the coefficients are exact halvings.
-template <bool BATCH, bool STORE_N, bool HALF>
-__global__ void __launch_bounds__(256, 5) k_update(DevMesh m, DevWork wk, const double* Wp, const double* Up,
-                                                const double* Vp, const double* W0, const double* U0,
-                                                const double* V0, double* Wo, double* Uo, double* Vo, Stage st,
-                                                double* nst = nullptr) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m.C) return;
+// COR0: no instance has a Coriolis term.  SOFT: part of the products on the
+// integer pipe.
+//
+// Bound by the FP64 pipe: 64-70 operations a cell of 73-79 before the slots
+// held depths, the source products q g were formed once per cell and the first
+// terms were negated instead of subtracted from zero.
+// update_cell: (h, hu, hv) of cell i after the stage; false where a product left
+// the integer routine's range.
+template <bool BATCH, bool HALF, bool COR0, bool SOFT>
+__device__ __forceinline__ bool update_cell(const DevMesh& m, const DevWork& wk, int i, const double* Wp,
+                                            const double* Up, const double* Vp, const double* W0, const double* U0,
+                                            const double* V0, const Stage& st, double* n) {
+  Products<SOFT> prod;
   const int C = m.C;
   const int inst = BATCH ? m.cinst[i] : 0;
   const double dt = HALF ? SWE_HALF(wk.dt[inst]) : (st.first ? wk.dt[inst] : st.c * wk.dt[inst]);
   const unsigned own = m.cown[i];
   const double dti = wk.drain[i];
+  // source terms: q times the gradient plus cor (-v, u) at a slot; the same for
+  // the three slots unless one is dry or thin
+  const double q = dt * (1. / 3.);
+  const double gx = wk.gx[i], gy = wk.gy[i];
+  const double up = Up[i], vp = Vp[i];
+  const bool dry_cell = (wk.cls[i] & 3u) == 0u;
+  const double cor = COR0 ? 0. : m.inst_cor[inst];
+  double qsx, qsy;
+  if (COR0) {
+    qsx = prod.mul(q, gx);
+    qsy = prod.mul(q, gy);
+  } else {
+    qsx = q * (gx + cor * (-vp));
+    qsy = q * (gy + cor * up);
+  }
   double r0 = 0., r1 = 0., r2 = 0.;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
@@ -562,47 +661,81 @@ __global__ void __launch_bounds__(256, 5) k_update(DevMesh m, DevWork wk, const 
     const int nb = en.y;
     const double dtik = nb < 0 ? kInf : wk.drain[gidx(wk, nb, C)];
     const double dtk = (out ? dgt0(F0) : dlt(F0, 0.)) ? smin(dt, dti) : smin(dt, dtik);  // sgn F0 > 0
-    const double c_ek = ce.x;
-    const double h_ek = wk.ew[slot] - ce.y;
-    const double s = (out ? dtk : SWE_NEG(dtk)) * c_ek;
-    r0 -= s * F0;
-    r1 -= s * F1;
-    r2 -= s * F2;
-    const double q = dt * (1. / 3.);
-    r1 -= q * wk.sx[slot] * h_ek;
-    r2 -= q * wk.sy[slot] * h_ek;
-    const double p = SWE_HALF(h_ek) * h_ek;  // 0.5 h h
-    r1 += dtk * (nc.x * p);  // (n_x c) p
-    r2 += dtk * (nc.y * p);
+    const double h_ek = wk.eh[slot];
+    const double s = prod.mul(out ? dtk : SWE_NEG(dtk), ce.x);
+    const double a0 = prod.mul(s, F0), a1 = prod.mul(s, F1), a2 = prod.mul(s, F2);
+    if (k == 0) {
+      r0 = zero_minus(a0);
+      r1 = zero_minus(a1);
+      r2 = zero_minus(a2);
+    } else {
+      r0 -= a0;
+      r1 -= a1;
+      r2 -= a2;
+    }
+    double qx = qsx, qy = qsy;
+    if (COR0) {
+      // a zero of g takes the sign of g + cor (-v, u) with cor = +-0
+      if (((ubits(gx) << 1) == 0ull) || ((ubits(gy) << 1) == 0ull)) {
+        const double c0 = m.inst_cor[inst];
+        double u = up, v = vp;
+        if (dry_cell || !is_wet(h_ek)) u = v = 0.;
+        if ((ubits(gx) << 1) == 0ull) qx = add_zero_product(gx, c0, SWE_NEG(v));
+        if ((ubits(gy) << 1) == 0ull) qy = add_zero_product(gy, c0, u);
+      }
+    } else if (dry_cell || dltc(h_ek, kEta1)) {
+      double u = up, v = vp;
+      slot_velocity(h_ek, dry_cell, &u, &v);
+      qx = q * (gx + cor * (-v));
+      qy = q * (gy + cor * u);
+    }
+    r1 -= prod.mul(qx, h_ek);
+    r2 -= prod.mul(qy, h_ek);
+    const double p = prod.mul(SWE_HALF(h_ek), h_ek);  // 0.5 h h
+    r1 += prod.mul(dtk, prod.mul(nc.x, p));  // (n_x c) p
+    r2 += prod.mul(dtk, prod.mul(nc.y, p));
   }
   const double b = m.bc[i];
   const double h0 = W0[i] - b;
-  const double c00 = h0, c01 = h0 * U0[i], c02 = h0 * V0[i];
-  double n0, n1, n2;
+  const double c00 = h0, c01 = prod.mul(h0, U0[i]), c02 = prod.mul(h0, V0[i]);
   if (st.first && !HALF) {
-    n0 = c00 + r0;
-    n1 = c01 + r1;
-    n2 = c02 + r2;
+    n[0] = c00 + r0;
+    n[1] = c01 + r1;
+    n[2] = c02 + r2;
   } else {
     const double hp = Wp[i] - b;
-    const double c10 = hp, c11 = hp * Up[i], c12 = hp * Vp[i];
+    const double c10 = hp, c11 = prod.mul(hp, up), c12 = prod.mul(hp, vp);
     if (HALF) {
-      n0 = SWE_HALF(c00) + SWE_HALF(c10) + r0;
-      n1 = SWE_HALF(c01) + SWE_HALF(c11) + r1;
-      n2 = SWE_HALF(c02) + SWE_HALF(c12) + r2;
+      n[0] = SWE_HALF(c00) + SWE_HALF(c10) + r0;
+      n[1] = SWE_HALF(c01) + SWE_HALF(c11) + r1;
+      n[2] = SWE_HALF(c02) + SWE_HALF(c12) + r2;
     } else {
-      n0 = st.a * c00 + st.b * c10 + r0;
-      n1 = st.a * c01 + st.b * c11 + r1;
-      n2 = st.a * c02 + st.b * c12 + r2;
+      n[0] = st.a * c00 + st.b * c10 + r0;
+      n[1] = st.a * c01 + st.b * c11 + r1;
+      n[2] = st.a * c02 + st.b * c12 + r2;
     }
   }
+  return !prod.other;
+}
+
+template <bool BATCH, bool STORE_N, bool HALF, bool COR0, bool SOFT>
+__global__ void __launch_bounds__(256, 5) k_update(DevMesh m, DevWork wk, const double* Wp, const double* Up,
+                                                const double* Vp, const double* W0, const double* U0,
+                                                const double* V0, double* Wo, double* Uo, double* Vo, Stage st,
+                                                double* nst = nullptr) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= m.C) return;
+  double n[3];
+  if (!update_cell<BATCH, HALF, COR0, SOFT>(m, wk, i, Wp, Up, Vp, W0, U0, V0, st, n))
+    update_cell<BATCH, HALF, COR0, false>(m, wk, i, Wp, Up, Vp, W0, U0, V0, st, n);
+  const double b = m.bc[i];
   if (STORE_N) {
-    nst[i] = n0;
-    nst[C + i] = n1;
-    nst[2 * C + i] = n2;
+    nst[i] = n[0];
+    nst[m.C + i] = n[1];
+    nst[2 * m.C + i] = n[2];
   }
   double ow, ou, ov;
-  cons_assign(b, n0, n1, n2, &ow, &ou, &ov);
+  cons_assign(b, n[0], n[1], n[2], &ow, &ou, &ov);
   Wo[i] = ow;
   Uo[i] = ou;
   Vo[i] = ov;
@@ -714,13 +847,12 @@ std::string Engine::init(std::vector<HostInstance>&& inst, int flux, int ws, int
   M.C = (int)C; M.E = (int)E; M.N = (int)N; M.I = I;
   bool ok = true;
   const int *p_cnode, *p_cnbr, *p_cedge, *p_cinst, *p_eown, *p_enb, *p_esl, *p_esr, *p_einst, *p_icb;
-  const unsigned char* p_cown;
   const double *p_area, *p_cek, *p_cnxc, *p_cnyc, *p_enx, *p_eny, *p_etx, *p_ety, *p_elmin, *p_cfl, *p_cor;
   const int2 *p_cslot, *p_enode;
   const double2* p_nxy;
   const int4* p_eidx;
   ok = ok && up(img.cnode, p_cnode) && up(img.cnbr, p_cnbr) && up(img.cedge, p_cedge) && up(img.cinst, p_cinst);
-  ok = ok && up(img.cown, p_cown) && up(img.area, p_area);
+  ok = ok && up(img.cown, bed_.cown) && up(img.area, p_area);
   ok = ok && up(img.cek, p_cek) && up(img.cnxc, p_cnxc) && up(img.cnyc, p_cnyc);
   ok = ok && up(img.eown, p_eown) && up(img.enb, p_enb) && up(img.eslotl, p_esl) && up(img.eslotr, p_esr);
   ok = ok && up(img.einst, p_einst) && up(img.enx, p_enx) && up(img.eny, p_eny) && up(img.etx, p_etx);
@@ -729,19 +861,20 @@ std::string Engine::init(std::vector<HostInstance>&& inst, int flux, int ws, int
   ok = ok && up(img.srec, bed_.srec) && up(img.cslot, p_cslot) && up(img.erec, bed_.erec) && up(img.eidx, p_eidx);
   const int *p_nptr, *p_ncell;
   ok = ok && up(img.nptr, p_nptr) && up(img.ncell, p_ncell);
-  bed_.bc = dalloc<double>(C); bed_.fwthr = dalloc<double>(C);
+  bed_.bc = dalloc<double>(C); bed_.fwthr = dalloc<double>(C); bed_.wetthr = dalloc<double>(C);
   bed_.zn = dalloc<double>(3 * C); bed_.ze = dalloc<double>(3 * C);
   bed_.dry = dalloc<double>(kDryStride * C); bed_.combo = dalloc<double>(8 * kComboStride * C);
+  bed_.combov = dalloc<double>(8 * kComboVStride * C);
   bed_.pw1 = dalloc<double>(kPw1Stride * C); bed_.pw2 = dalloc<Pw2Rec>(C);
   bed_.ezm = dalloc<double>(E); bed_.nz = dalloc<double>(N);
-  ok = ok && bed_.bc && bed_.fwthr && bed_.zn && bed_.ze && bed_.dry && bed_.combo && bed_.pw1 && bed_.pw2 &&
+  ok = ok && bed_.bc && bed_.fwthr && bed_.wetthr && bed_.combov && bed_.zn && bed_.ze && bed_.dry && bed_.combo && bed_.pw1 && bed_.pw2 &&
        bed_.ezm && bed_.nz;
   if (!ok) {
     *st = 6;
     return std::string("device allocation or upload failed: ") + cudaGetErrorString(cudaGetLastError());
   }
-  M.cnode = p_cnode; M.cnbr = p_cnbr; M.cedge = p_cedge; M.cinst = p_cinst; M.cown = p_cown;
-  M.bc = bed_.bc; M.fwthr = bed_.fwthr; M.area = p_area; M.zn = bed_.zn; M.ze = bed_.ze; M.cek = p_cek;
+  M.cnode = p_cnode; M.cnbr = p_cnbr; M.cedge = p_cedge; M.cinst = p_cinst; M.cown = bed_.cown;
+  M.bc = bed_.bc; M.fwthr = bed_.fwthr; M.wetthr = bed_.wetthr; M.combov = bed_.combov; M.area = p_area; M.zn = bed_.zn; M.ze = bed_.ze; M.cek = p_cek;
   M.cnxc = p_cnxc; M.cnyc = p_cnyc; M.dry = bed_.dry; M.combo = bed_.combo; M.pw1 = bed_.pw1; M.pw2 = bed_.pw2;
   M.eown = p_eown; M.enb = p_enb; M.eslotl = p_esl; M.eslotr = p_esr; M.einst = p_einst;
   M.enx = p_enx; M.eny = p_eny; M.etx = p_etx; M.ety = p_ety; M.ezm = bed_.ezm; M.elmin = p_elmin;
@@ -750,6 +883,7 @@ std::string Engine::init(std::vector<HostInstance>&& inst, int flux, int ws, int
   M.nptr = p_nptr; M.ncell = p_ncell;
 
   DevWork& Wk = work_;
+  Wk.eh = dalloc<double>(3 * C); Wk.gx = dalloc<double>(C); Wk.gy = dalloc<double>(C);
   Wk.ew = dalloc<double>(3 * C); Wk.eu = dalloc<double>(3 * C); Wk.ev = dalloc<double>(3 * C);
   Wk.sx = dalloc<double>(3 * C); Wk.sy = dalloc<double>(3 * C);
   Wk.f0 = dalloc<double>(E); Wk.f1 = dalloc<double>(E); Wk.f2 = dalloc<double>(E);
@@ -770,7 +904,7 @@ std::string Engine::init(std::vector<HostInstance>&& inst, int flux, int ws, int
   for (int q = 0; q < 6; ++q) state_[q] = dalloc<double>(C);
   d_io = dalloc<double>(3 * C);
   d_ioflag = dalloc<unsigned>(1);
-  if (!Wk.ew || !Wk.eu || !Wk.ev || !Wk.sx || !Wk.sy || !Wk.f0 || !Wk.f1 || !Wk.f2 || !Wk.drain || !Wk.maxwp ||
+  if (!Wk.eh || !Wk.gx || !Wk.gy || !Wk.ew || !Wk.eu || !Wk.ev || !Wk.sx || !Wk.sy || !Wk.f0 || !Wk.f1 || !Wk.f2 || !Wk.drain || !Wk.maxwp ||
       !Wk.pwlist || !Wk.pwcount || !Wk.pwrec || !Wk.cls || !Wk.r || !Wk.dt || !Wk.tsum || !d_fixed_dt || !Wk.err ||
       !state_[5] || !d_io || !d_ioflag) {
     *st = 6;
@@ -780,6 +914,9 @@ std::string Engine::init(std::vector<HostInstance>&& inst, int flux, int ws, int
     *st = 6;
     return "pinned allocation failed";
   }
+  cudaMemset(Wk.eh, 0, 3 * C * sizeof(double));
+  cudaMemset(Wk.gx, 0, C * sizeof(double));
+  cudaMemset(Wk.gy, 0, C * sizeof(double));
   cudaMemset(Wk.ew, 0, 3 * C * sizeof(double));
   cudaMemset(Wk.eu, 0, 3 * C * sizeof(double));
   cudaMemset(Wk.ev, 0, 3 * C * sizeof(double));
@@ -824,93 +961,112 @@ cudaError_t Engine::reset_pass() {
   return cudaGetLastError();
 }
 
-void Engine::launch_recon1(const double* W, const double* U, const double* V, int latch_mode) {
+void Engine::launch_recon1(const double* W, const double* U, const double* V, int latch_mode, bool slots) {
   const int b = blk_[0], g = nblocks(mesh_.C, b);
-  if (batched_) {
-    if (cor0_) k_recon1<true, true><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode);
-    else k_recon1<true, false><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode);
-  } else {
-    if (cor0_) k_recon1<false, true><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode);
-    else k_recon1<false, false><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode);
+  const int form = !slots ? kLean : cor0_ ? kSlotsCor0 : kSlotsCor;
+  switch (form + (batched_ ? 3 : 0)) {
+    case 0: k_recon1<false, kLean><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode); break;
+    case 1: k_recon1<false, kSlotsCor0><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode); break;
+    case 2: k_recon1<false, kSlotsCor><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode); break;
+    case 3: k_recon1<true, kLean><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode); break;
+    case 4: k_recon1<true, kSlotsCor0><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode); break;
+    default: k_recon1<true, kSlotsCor><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode); break;
   }
   ++launches_;
 }
 
-void Engine::launch_recon2(const double* W, const double* U, const double* V, cudaStream_t s) {
+void Engine::launch_recon2(const double* W, const double* U, const double* V, cudaStream_t s, bool slots) {
   const int b = blk_[0], g = std::max(1, std::min(nblocks(mesh_.C, b), 152 * 2048 / b));
-  if (batched_) {
-    if (cor0_) k_recon2<true, true><<<g, b, 0, s>>>(mesh_, work_, W, U, V);
-    else k_recon2<true, false><<<g, b, 0, s>>>(mesh_, work_, W, U, V);
-  } else {
-    if (cor0_) k_recon2<false, true><<<g, b, 0, s>>>(mesh_, work_, W, U, V);
-    else k_recon2<false, false><<<g, b, 0, s>>>(mesh_, work_, W, U, V);
+  const int form = !slots ? kLean : cor0_ ? kSlotsCor0 : kSlotsCor;
+  switch (form + (batched_ ? 3 : 0)) {
+    case 0: k_recon2<false, kLean><<<g, b, 0, s>>>(mesh_, work_, W, U, V); break;
+    case 1: k_recon2<false, kSlotsCor0><<<g, b, 0, s>>>(mesh_, work_, W, U, V); break;
+    case 2: k_recon2<false, kSlotsCor><<<g, b, 0, s>>>(mesh_, work_, W, U, V); break;
+    case 3: k_recon2<true, kLean><<<g, b, 0, s>>>(mesh_, work_, W, U, V); break;
+    case 4: k_recon2<true, kSlotsCor0><<<g, b, 0, s>>>(mesh_, work_, W, U, V); break;
+    default: k_recon2<true, kSlotsCor><<<g, b, 0, s>>>(mesh_, work_, W, U, V); break;
   }
   ++launches_;
 }
 
-cudaError_t Engine::interface_values(const double* W, const double* U, const double* V, int latch_mode) {
-  launch_recon1(W, U, V, latch_mode);
-  launch_recon2(W, U, V, stream_);
+cudaError_t Engine::interface_values(const double* W, const double* U, const double* V) {
+  launch_recon1(W, U, V, 0, true);
+  launch_recon2(W, U, V, stream_, true);
   k_node_max_all<<<nblocks(std::max(mesh_.N, 1), 256), 256, 0, stream_>>>(mesh_, work_, W);
   ++launches_;
+  slots_stale_ = false;
   return cudaGetLastError();
 }
 
-template <class FLUX, bool TAPE>
-static void launch_flux_t(bool batched, int mode, int blocks, int b, cudaStream_t s, const DevMesh& m,
-                          const DevWork& w, const double* W) {
-  if (batched) {
-    if (mode) k_flux<FLUX, true, 1, TAPE><<<blocks, b, 0, s>>>(m, w, W);
-    else k_flux<FLUX, true, 0, TAPE><<<blocks, b, 0, s>>>(m, w, W);
-  } else {
-    if (mode) k_flux<FLUX, false, 1, TAPE><<<blocks, b, 0, s>>>(m, w, W);
-    else k_flux<FLUX, false, 0, TAPE><<<blocks, b, 0, s>>>(m, w, W);
-  }
+cudaError_t Engine::refresh_slots() {
+  if (!slots_stale_) return cudaSuccess;
+  // the last stage read buffer 1; its list is made again and emptied again, and
+  // the CFL ratio of its flux pass stays
+  launch_recon1(state(1, 0), state(1, 1), state(1, 2), 3, true);
+  launch_recon2(state(1, 0), state(1, 1), state(1, 2), stream_, true);
+  slots_stale_ = false;
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemsetAsync(work_.pwcount, 0, sizeof(int), stream_);
+  return e;
 }
-template <class FLUX>
-static void launch_flux(bool batched, int mode, int blocks, int b, cudaStream_t s, const DevMesh& m,
-                        const DevWork& w, const double* W) {
-  if (w.ftape) launch_flux_t<FLUX, true>(batched, mode, blocks, b, s, m, w, W);
-  else launch_flux_t<FLUX, false>(batched, mode, blocks, b, s, m, w, W);
-}
-template <class FLUX>
-static void launch_flux_pw(bool batched, int blocks, cudaStream_t s, const DevMesh& m, const DevWork& w,
-                           const double* W) {
-  if (w.ftape) {
-    if (batched) k_flux_pw<FLUX, true, true><<<blocks, 128, 0, s>>>(m, w, W);
-    else k_flux_pw<FLUX, false, true><<<blocks, 128, 0, s>>>(m, w, W);
-  } else {
-    if (batched) k_flux_pw<FLUX, true, false><<<blocks, 128, 0, s>>>(m, w, W);
-    else k_flux_pw<FLUX, false, false><<<blocks, 128, 0, s>>>(m, w, W);
+
+// The plugin of (flux, wave speed), given to f as a type.
+template <class F>
+static void with_plugin(int flux, int ws, F&& f) {
+  switch (flux * 3 + ws) {
+    case 0: f(HLL<Rusanov>{}); break;
+    case 1: f(HLL<Davis>{}); break;
+    case 2: f(HLL<Einfeldt>{}); break;
+    case 3: f(HLLC<Rusanov>{}); break;
+    case 4: f(HLLC<Davis>{}); break;
+    default: f(HLLC<Einfeldt>{}); break;
   }
 }
 
-cudaError_t Engine::fluxes(const double* W) { return fluxes(W, 0); }
+template <class FLUX, bool BATCH>
+static void launch_stage_flux(bool tape, bool soft, int g, int b, cudaStream_t s, const DevMesh& m, const DevWork& w,
+                              const double* const* in) {
+  switch ((tape ? 2 : 0) | (soft ? 1 : 0)) {
+    case 0: k_flux<FLUX, BATCH, 1, false, false><<<g, b, 0, s>>>(m, w, in[0], in[1], in[2]); break;
+    case 1: k_flux<FLUX, BATCH, 1, false, true><<<g, b, 0, s>>>(m, w, in[0], in[1], in[2]); break;
+    case 2: k_flux<FLUX, BATCH, 1, true, false><<<g, b, 0, s>>>(m, w, in[0], in[1], in[2]); break;
+    default: k_flux<FLUX, BATCH, 1, true, true><<<g, b, 0, s>>>(m, w, in[0], in[1], in[2]); break;
+  }
+}
 
-cudaError_t Engine::fluxes(const double* W, int mode) {
+cudaError_t Engine::fluxes(const double* W) {
   const int b = blk_[1], g = nblocks(mesh_.E, b);
-  switch (flux_ * 3 + ws_) {
-    case 0: launch_flux<HLL<Rusanov>>(batched_, mode, g, b, stream_, mesh_, work_, W); break;
-    case 1: launch_flux<HLL<Davis>>(batched_, mode, g, b, stream_, mesh_, work_, W); break;
-    case 2: launch_flux<HLL<Einfeldt>>(batched_, mode, g, b, stream_, mesh_, work_, W); break;
-    case 3: launch_flux<HLLC<Rusanov>>(batched_, mode, g, b, stream_, mesh_, work_, W); break;
-    case 4: launch_flux<HLLC<Davis>>(batched_, mode, g, b, stream_, mesh_, work_, W); break;
-    default: launch_flux<HLLC<Einfeldt>>(batched_, mode, g, b, stream_, mesh_, work_, W); break;
-  }
+  with_plugin(flux_, ws_, [&](auto plugin) {
+    typedef decltype(plugin) P;
+    if (batched_) k_flux<P, true, 0, false, false><<<g, b, 0, stream_>>>(mesh_, work_, W, nullptr, nullptr);
+    else k_flux<P, false, 0, false, false><<<g, b, 0, stream_>>>(mesh_, work_, W, nullptr, nullptr);
+  });
   launches_ += 1;
   return cudaGetLastError();
 }
 
-void Engine::fluxes_pw(const double* W, cudaStream_t s) {
+cudaError_t Engine::stage_fluxes(const double* const* in) {
+  const int b = blk_[1], g = nblocks(mesh_.E, b);
+  const bool tape = work_.ftape != nullptr;
+  with_plugin(flux_, ws_, [&](auto plugin) {
+    typedef decltype(plugin) P;
+    if (batched_) launch_stage_flux<P, true>(tape, soft_, g, b, stream_, mesh_, work_, in);
+    else launch_stage_flux<P, false>(tape, soft_, g, b, stream_, mesh_, work_, in);
+  });
+  launches_ += 1;
+  return cudaGetLastError();
+}
+
+void Engine::stage_fluxes_pw(const double* const* in, cudaStream_t s) {
   const int g = std::max(1, std::min((3 * (int)mesh_.C + 127) / 128, 152 * 8));
-  switch (flux_ * 3 + ws_) {
-    case 0: launch_flux_pw<HLL<Rusanov>>(batched_, g, s, mesh_, work_, W); break;
-    case 1: launch_flux_pw<HLL<Davis>>(batched_, g, s, mesh_, work_, W); break;
-    case 2: launch_flux_pw<HLL<Einfeldt>>(batched_, g, s, mesh_, work_, W); break;
-    case 3: launch_flux_pw<HLLC<Rusanov>>(batched_, g, s, mesh_, work_, W); break;
-    case 4: launch_flux_pw<HLLC<Davis>>(batched_, g, s, mesh_, work_, W); break;
-    default: launch_flux_pw<HLLC<Einfeldt>>(batched_, g, s, mesh_, work_, W); break;
-  }
+  const bool tape = work_.ftape != nullptr;
+  with_plugin(flux_, ws_, [&](auto plugin) {
+    typedef decltype(plugin) P;
+    if (batched_ && tape) k_flux_pw<P, true, true><<<g, 128, 0, s>>>(mesh_, work_, in[0], in[1], in[2]);
+    else if (batched_) k_flux_pw<P, true, false><<<g, 128, 0, s>>>(mesh_, work_, in[0], in[1], in[2]);
+    else if (tape) k_flux_pw<P, false, true><<<g, 128, 0, s>>>(mesh_, work_, in[0], in[1], in[2]);
+    else k_flux_pw<P, false, false><<<g, 128, 0, s>>>(mesh_, work_, in[0], in[1], in[2]);
+  });
   launches_ += 1;
 }
 
@@ -918,14 +1074,18 @@ cudaError_t Engine::launch_stage(const Stage& st, const double* const* in, const
                                  double* const* out, bool first_stage_of_step, int latch_mode, cudaEvent_t* ev) {
   const int b = blk_[2];
   const int lm = first_stage_of_step ? latch_mode : 0;
+  // a stage that overwrites its own input leaves the full interface values now
+  // (refresh_slots could not make them later)
+  const bool slots = in[0] == out[0];
   if (ev) cudaEventRecord(ev[0], stream_);
-  launch_recon1(in[0], in[1], in[2], lm);
+  launch_recon1(in[0], in[1], in[2], lm, slots);
   if (ev) {
     // per-kernel timing: the kernels one after another
     cudaEventRecord(ev[1], stream_);
-    launch_recon2(in[0], in[1], in[2], stream_);
+    launch_recon2(in[0], in[1], in[2], stream_, slots);
     cudaEventRecord(ev[2], stream_);
-    cudaError_t e = fluxes(in[0], 0);
+    stage_fluxes_pw(in, stream_);
+    cudaError_t e = stage_fluxes(in);
     if (e != cudaSuccess) return e;
     cudaEventRecord(ev[3], stream_);
   } else {
@@ -933,14 +1093,16 @@ cudaError_t Engine::launch_stage(const Stage& st, const double* const* in, const
     // beside the other edges' fluxes
     cudaEventRecord(ev_fork_, stream_);
     cudaStreamWaitEvent(side_, ev_fork_, 0);
-    launch_recon2(in[0], in[1], in[2], side_);
-    fluxes_pw(in[0], side_);
+    launch_recon2(in[0], in[1], in[2], side_, slots);
+    stage_fluxes_pw(in, side_);
     cudaEventRecord(ev_join_, side_);
-    cudaError_t e = fluxes(in[0], 1);
+    cudaError_t e = stage_fluxes(in);
     if (e != cudaSuccess) return e;
     cudaStreamWaitEvent(stream_, ev_join_, 0);
   }
-  k_drain<<<nblocks(mesh_.C, b), b, 0, stream_>>>(mesh_, work_, in[0]);
+  const double dt_scale = 2. * std::max(1., st.first ? 1. : st.c);
+  if (batched_) k_drain<true><<<nblocks(mesh_.C, b), b, 0, stream_>>>(mesh_, work_, in[0], dt_scale);
+  else k_drain<false><<<nblocks(mesh_.C, b), b, 0, stream_>>>(mesh_, work_, in[0], dt_scale);
   if (ev) cudaEventRecord(ev[4], stream_);
   ++launches_;
   launch_update(st, in, u0, out, nullptr);
@@ -949,26 +1111,33 @@ cudaError_t Engine::launch_stage(const Stage& st, const double* const* in, const
 }
 
 template <bool BATCH, bool STORE_N, bool HALF>
-static void update_kernel(int g, int b, cudaStream_t s, const DevMesh& m, const DevWork& w, const Stage& st,
-                          const double* const* in, const double* const* u0, double* const* out, double* nst) {
-  k_update<BATCH, STORE_N, HALF><<<g, b, 0, s>>>(m, w, in[0], in[1], in[2], u0[0], u0[1], u0[2], out[0], out[1],
-                                                 out[2], st, nst);
+static void update_kernel(int g, int b, cudaStream_t s, bool cor0, bool soft, const DevMesh& m, const DevWork& w,
+                          const Stage& st, const double* const* in, const double* const* u0, double* const* out,
+                          double* nst) {
+#define SWE_UPDATE(COR0, SOFT)                                                                             \
+  k_update<BATCH, STORE_N, HALF, COR0, SOFT><<<g, b, 0, s>>>(m, w, in[0], in[1], in[2], u0[0], u0[1], u0[2], \
+                                                             out[0], out[1], out[2], st, nst)
+  if (cor0 && soft) SWE_UPDATE(true, true);
+  else if (cor0) SWE_UPDATE(true, false);
+  else if (soft) SWE_UPDATE(false, true);
+  else SWE_UPDATE(false, false);
+#undef SWE_UPDATE
 }
 
 void Engine::launch_update(const Stage& st, const double* const* in, const double* const* u0, double* const* out,
                            double* nst) {
   const int b = blk_[2], g = nblocks(mesh_.C, b);
   const bool half = !st.first && st.a == 0.5 && st.b == 0.5 && st.c == 0.5;
-  const int sel = (batched_ ? 4 : 0) | (nst ? 2 : 0) | (half ? 1 : 0);
-  switch (sel) {
-    case 0: update_kernel<false, false, false>(g, b, stream_, mesh_, work_, st, in, u0, out, nst); break;
-    case 1: update_kernel<false, false, true>(g, b, stream_, mesh_, work_, st, in, u0, out, nst); break;
-    case 2: update_kernel<false, true, false>(g, b, stream_, mesh_, work_, st, in, u0, out, nst); break;
-    case 3: update_kernel<false, true, true>(g, b, stream_, mesh_, work_, st, in, u0, out, nst); break;
-    case 4: update_kernel<true, false, false>(g, b, stream_, mesh_, work_, st, in, u0, out, nst); break;
-    case 5: update_kernel<true, false, true>(g, b, stream_, mesh_, work_, st, in, u0, out, nst); break;
-    case 6: update_kernel<true, true, false>(g, b, stream_, mesh_, work_, st, in, u0, out, nst); break;
-    default: update_kernel<true, true, true>(g, b, stream_, mesh_, work_, st, in, u0, out, nst); break;
+  auto run = [&](auto kernel) { kernel(g, b, stream_, cor0_, soft_, mesh_, work_, st, in, u0, out, nst); };
+  switch ((batched_ ? 4 : 0) | (nst ? 2 : 0) | (half ? 1 : 0)) {
+    case 0: run(update_kernel<false, false, false>); break;
+    case 1: run(update_kernel<false, false, true>); break;
+    case 2: run(update_kernel<false, true, false>); break;
+    case 3: run(update_kernel<false, true, true>); break;
+    case 4: run(update_kernel<true, false, false>); break;
+    case 5: run(update_kernel<true, false, true>); break;
+    case 6: run(update_kernel<true, true, false>); break;
+    default: run(update_kernel<true, true, true>); break;
   }
   ++launches_;
 }
@@ -987,6 +1156,7 @@ cudaError_t Engine::step_timed(int scheme, int latch_mode, double* acc) {
     double* const* out = last ? S0 : S1;
     e = launch_stage(sc.s[s], in, S0, out, s == 0, latch_mode, ev[s]);
   }
+  slots_stale_ = sc.n > 1;
   if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
   if (e == cudaSuccess) {
     for (int s = 0; s < sc.n; ++s)
@@ -1235,6 +1405,7 @@ cudaError_t Engine::run_graph(int scheme, int latch_mode, int64_t n) {
     launches_ = per_step;  // capture launched nothing
   }
   const int64_t kernels_per_step = 6 * scheme_of(scheme).n;
+  slots_stale_ = scheme_of(scheme).n > 1;
   for (int64_t s = 0; s < n; ++s) {
     cudaError_t e = cudaGraphLaunch(ge, stream_);
     if (e != cudaSuccess) return e;

@@ -421,17 +421,32 @@ SWE_HD void cons_assign(double b, double h, double hu, double hv, double* ow, do
 }
 
 // -------------------------------------------------------------- edge flux
-// include/SpaceDisc.h:4-18: F.n of U = (h, hu, hv), g = 1
-SWE_HD void elem_flux(double nx, double ny, double h, double hu, double hv, double* f) {
+// How a flux or update multiplies; other is set when the evaluation is to be
+// done again with Products<false>.
+template <bool SOFT>
+struct Products {
+  bool other = false;
+  SWE_HD double mul(double a, double b) {
+return a * b;
+  }
+};
+
+// include/SpaceDisc.h:4-18: F.n of U = (h, hu, hv), g = 1; hh = h h
+template <class M>
+SWE_HD void elem_flux_hh(M& m, double nx, double ny, double h, double hu, double hv, double hh, double* f) {
   f[0] = 0.; f[1] = 0.; f[2] = 0.;
   if (is_wet(h)) {
-    double hveln = hu * nx + hv * ny;
+    double hveln = m.mul(hu, nx) + m.mul(hv, ny);
     f[0] = hveln;
     const double q = SWE_DIV(hveln, h);
-    const double p = SWE_HALF(h) * h;  // 0.5 h h
-    f[1] = q * hu + p * nx;
-    f[2] = q * hv + p * ny;
+    const double p = SWE_HALF(hh);  // (0.5 h) h: halving is exact on either side of the product
+    f[1] = m.mul(q, hu) + m.mul(p, nx);
+    f[2] = m.mul(q, hv) + m.mul(p, ny);
   }
+}
+SWE_HD void elem_flux(double nx, double ny, double h, double hu, double hv, double* f) {
+  Products<false> m;
+  elem_flux_hh(m, nx, ny, h, hu, hv, h * h, f);
 }
 
 // Wave-speed plugins (src/Fluxes.cpp:5-26).  speeds() returns the pair the
@@ -460,8 +475,9 @@ struct EdgeTape {
 
 struct Rusanov {
   static constexpr int id = 0;
-  template <class T>
-  SWE_HD static void speeds(double ul, double hl, double ur, double hr, double* a0, double* a1, const T& tape) {
+  template <class M, class T>
+  SWE_HD static void speeds(M& m, double ul, double hl, double ur, double hr, double* a0, double* a1,
+                            const T& tape) {
     double cl = SWE_SQRT(hl), cr = SWE_SQRT(hr);
     double ap = smax(fabs(ul) + cl, fabs(ur) + cr);
     *a0 = -ap;
@@ -469,35 +485,40 @@ struct Rusanov {
     tape.speeds(cl, cr, 0., 0., *a0, *a1);
   }
   SWE_HD static void speeds(double ul, double hl, double ur, double hr, double* a0, double* a1) {
-    speeds(ul, hl, ur, hr, a0, a1, NoTape{});
+    Products<false> m;
+    speeds(m, ul, hl, ur, hr, a0, a1, NoTape{});
   }
 };
 struct Davis {
   static constexpr int id = 1;
-  template <class T>
-  SWE_HD static void speeds(double ul, double hl, double ur, double hr, double* a0, double* a1, const T& tape) {
+  template <class M, class T>
+  SWE_HD static void speeds(M& m, double ul, double hl, double ur, double hr, double* a0, double* a1,
+                            const T& tape) {
     double cl = SWE_SQRT(hl), cr = SWE_SQRT(hr);
     *a0 = smin(ul - cl, ur - cr);
     *a1 = smax(ul + cl, ur + cr);
     tape.speeds(cl, cr, 0., 0., *a0, *a1);
   }
   SWE_HD static void speeds(double ul, double hl, double ur, double hr, double* a0, double* a1) {
-    speeds(ul, hl, ur, hr, a0, a1, NoTape{});
+    Products<false> m;
+    speeds(m, ul, hl, ur, hr, a0, a1, NoTape{});
   }
 };
 struct Einfeldt {
   static constexpr int id = 2;
-  template <class T>
-  SWE_HD static void speeds(double ul, double hl, double ur, double hr, double* a0, double* a1, const T& tape) {
+  template <class M, class T>
+  SWE_HD static void speeds(M& m, double ul, double hl, double ur, double hr, double* a0, double* a1,
+                            const T& tape) {
     double cl = SWE_SQRT(hl), cr = SWE_SQRT(hr);
-    double uRoe = SWE_DIV(cl * ul + cl * ur, cl + cr);  // the reference's cl * ur
+    double uRoe = SWE_DIV(m.mul(cl, ul) + m.mul(cl, ur), cl + cr);  // the reference's cl * ur
     double cRoe = SWE_SQRT(SWE_HALF(hl + hr));
     *a0 = smin(ul - cl, uRoe - cRoe);
     *a1 = smax(ur + cr, uRoe + cRoe);
     tape.speeds(cl, cr, uRoe, cRoe, *a0, *a1);
   }
   SWE_HD static void speeds(double ul, double hl, double ur, double hr, double* a0, double* a1) {
-    speeds(ul, hl, ur, hr, a0, a1, NoTape{});
+    Products<false> m;
+    speeds(m, ul, hl, ur, hr, a0, a1, NoTape{});
   }
 };
 
@@ -513,38 +534,64 @@ struct EdgeGeom {
 struct SideState {
   double w, u, v;  // interface primitive values (EdgeField slot)
 };
+struct DepthState {
+  double h, u, v;  // the same with the depth w - b
+};
+SWE_HD DepthState depth_state(const SideState& s, double b) { return DepthState{s.w - b, s.u, s.v}; }
+
+// |cor| + speed for a speed >= 0 (without an operation where cor is zero)
+SWE_HD double plus_coriolis(double cor, double speed) {
+  return (ubits(cor) << 1) == 0ull ? speed : fabs(cor) + speed;
+}
+
+// Whether reach / speed can lower a minimum whose double's upper word is cap
+// (kNoCap: always).  The upper word over 2^20 is the logarithm to base 2 plus
+// 1023, short of it by at most 0.0861, so a difference above cap by twice that
+// settles it (for normal numbers): three integer operations for the quotient's
+// sixty-five.  In a jittered mesh nearly every edge is settled.
+constexpr int kNoCap = 0x7FFFFFFF;
+SWE_HD bool may_lower(double reach, double speed, int cap) {
+  const int r = (int)(ubits(reach) >> 32), s = (int)(ubits(speed) >> 32);
+  constexpr int kMargin = (1023 << 20) - 180668;  // 0.1723 2^20
+  return cap == kNoCap || r < (1 << 20) || r - s + kMargin <= cap;
+}
 
 // Fluxes::HLL<W> (include/Fluxes.h:14-54).  *lw receives the edge's
-// length-to-wavespeed ratio, or is left alone when the edge does not update it.
+// length-to-wavespeed ratio, or is left alone when the edge does not update it
+// or cannot lower the minimum that cap describes (may_lower).
 template <class W>
 struct HLL {
   static constexpr int id = 0;
   SWE_HD static void eval(const EdgeGeom& g, const SideState& L, const SideState& R, double cor, double* lw,
                           double* F) {
-    eval(g, L, R, cor, lw, F, NoTape{});
+    Products<false> m;
+    eval_depth(m, g, depth_state(L, g.b), depth_state(R, g.b), cor, kNoCap, lw, F, NoTape{});
   }
-  template <class T>
-  SWE_HD static void eval(const EdgeGeom& g, const SideState& L, const SideState& R, double cor, double* lw,
-                          double* F, const T& tape) {
-    double ul = L.u * g.nx + L.v * g.ny;
-    double hl = L.w - g.b;
-    double ur = R.u * g.nx + R.v * g.ny;
-    double hr = R.w - g.b;
+  template <class M, class T>
+  SWE_HD static void eval_depth(M& m, const EdgeGeom& g, const DepthState& L, const DepthState& R, double cor,
+                                int cap, double* lw, double* F, const T& tape) {
+    const double hl = L.h, hr = R.h;
+    double ul = m.mul(L.u, g.nx) + m.mul(L.v, g.ny);
+    double ur = m.mul(R.u, g.nx) + m.mul(R.v, g.ny);
     F[0] = 0.; F[1] = 0.; F[2] = 0.;
     if (!dgtc(hl + hr, kMinCapture)) return;
     double a0, a1;
-    W::speeds(ul, hl, ur, hr, &a0, &a1, tape);
+    W::speeds(m, ul, hl, ur, hr, &a0, &a1, tape);
     double al = smin(0., a0);
     double ar = smax(0., a1);
     if (!dgtc(ar - al, kMinCapture)) return;
-    *lw = SWE_DIV(g.lmin, fabs(cor) + smax(-al, ar));
-    double Ul[3] = {hl, hl * L.u, hl * L.v};
-    double Ur[3] = {hr, hr * R.u, hr * R.v};
+    const double speed = plus_coriolis(cor, smax(-al, ar));
+    if (may_lower(g.lmin, speed, cap)) *lw = SWE_DIV(g.lmin, speed);
+    double Ul[3] = {hl, m.mul(hl, L.u), m.mul(hl, L.v)};
+    double Ur[3] = {hr, m.mul(hr, R.u), m.mul(hr, R.v)};
     double Fl[3], Fr[3];
-    elem_flux(g.nx, g.ny, Ul[0], Ul[1], Ul[2], Fl);
-    elem_flux(g.nx, g.ny, Ur[0], Ur[1], Ur[2], Fr);
+    elem_flux_hh(m, g.nx, g.ny, Ul[0], Ul[1], Ul[2], m.mul(hl, hl), Fl);
+    elem_flux_hh(m, g.nx, g.ny, Ur[0], Ur[1], Ur[2], m.mul(hr, hr), Fr);
+    const double aa = al * ar, d = ar - al;
 #pragma unroll
-    for (int q = 0; q < 3; ++q) F[q] = SWE_DIV(ar * Fl[q] - al * Fr[q] + (al * ar) * (Ur[q] - Ul[q]), ar - al);
+    for (int q = 0; q < 3; ++q)
+      F[q] = SWE_DIV(m.mul(ar, Fl[q]) - m.mul(al, Fr[q]) +
+                         m.mul(aa, Ur[q] - Ul[q]), d);
   }
 };
 
@@ -554,43 +601,46 @@ struct HLLC {
   static constexpr int id = 1;
   SWE_HD static void eval(const EdgeGeom& g, const SideState& L, const SideState& R, double cor, double* lw,
                           double* F) {
-    eval(g, L, R, cor, lw, F, NoTape{});
+    Products<false> m;
+    eval_depth(m, g, depth_state(L, g.b), depth_state(R, g.b), cor, kNoCap, lw, F, NoTape{});
   }
-  template <class T>
-  SWE_HD static void eval(const EdgeGeom& g, const SideState& L, const SideState& R, double cor, double* lw,
-                          double* F, const T& tape) {
-    double ul = L.u * g.nx + L.v * g.ny;
-    double hl = L.w - g.b;
-    double ur = R.u * g.nx + R.v * g.ny;
-    double hr = R.w - g.b;
+  template <class M, class T>
+  SWE_HD static void eval_depth(M& m, const EdgeGeom& g, const DepthState& L, const DepthState& R, double cor,
+                                int cap, double* lw, double* F, const T& tape) {
+    const double hl = L.h, hr = R.h;
+    double ul = m.mul(L.u, g.nx) + m.mul(L.v, g.ny);
+    double ur = m.mul(R.u, g.nx) + m.mul(R.v, g.ny);
     F[0] = 0.; F[1] = 0.; F[2] = 0.;
     if (!dgtc(hl + hr, kMinCapture)) return;
     double al, ar;
-    W::speeds(ul, hl, ur, hr, &al, &ar, tape);
+    W::speeds(m, ul, hl, ur, hr, &al, &ar, tape);
     // (ar - ur) hr = hr (ar - ur) and (al - ul) hl = hl (al - ul) bit for bit:
     // each product is formed once for u* and the star depth
-    const double hrA = (ar - ur) * hr, hlB = (al - ul) * hl;
-    double ustar = hrA * ur - hlB * ul + SWE_HALF(hl * hl - hr * hr);
+    const double hrA = m.mul(ar - ur, hr), hlB = m.mul(al - ul, hl);
+    const double hl2 = m.mul(hl, hl), hr2 = m.mul(hr, hr);
+    double ustar = m.mul(hrA, ur) - m.mul(hlB, ul) + SWE_HALF(hl2 - hr2);
     ustar = SWE_DIV(ustar, hrA - hlB);
     tape.ustar(ustar);
-    *lw = SWE_DIV(g.lmin, fabs(cor) + smax(kTol, smax(al, ar)));
+    const double speed = plus_coriolis(cor, smax(kTol, smax(al, ar)));
+    if (may_lower(g.lmin, speed, cap)) *lw = SWE_DIV(g.lmin, speed);
     // u* <= 0: the right star state, else the left one.  The side is picked
     // first and the shared formula evaluated once, so a warp whose edges take
     // both sides issues it once (the operations per side are the reference's).
     const bool right = !dgt0(ustar);
     const double hx = right ? hr : hl, ux = right ? R.u : L.u, vx = right ? R.v : L.v;
     const double ax = right ? ar : al, hxa = right ? hrA : hlB;  // hx (ax - u_n,x)
-    const double vt = ux * g.tx + vx * g.ty;  // tangential velocity of that side
-    double Ux[3] = {hx, hx * ux, hx * vx};
-    double us = vt * g.tx + ustar * g.ty;
-    double vs = vt * g.nx + ustar * g.ny;
+    // tangential velocity of that side
+    const double vt = m.mul(ux, g.tx) + m.mul(vx, g.ty);
+    double Ux[3] = {hx, m.mul(hx, ux), m.mul(hx, vx)};
+    double us = m.mul(vt, g.tx) + m.mul(ustar, g.ty);
+    double vs = m.mul(vt, g.nx) + m.mul(ustar, g.ny);
     double hs = SWE_DIV(hxa, ax - ustar);
-    double Us[3] = {hs, hs * us, hs * vs};
+    double Us[3] = {hs, m.mul(hs, us), m.mul(hs, vs)};
     double Fx[3];
-    elem_flux(g.nx, g.ny, Ux[0], Ux[1], Ux[2], Fx);
+    elem_flux_hh(m, g.nx, g.ny, Ux[0], Ux[1], Ux[2], right ? hr2 : hl2, Fx);
     double s = right ? smax(0., ar) : smin(0., al);
 #pragma unroll
-    for (int q = 0; q < 3; ++q) F[q] = Fx[q] + s * (Us[q] - Ux[q]);
+    for (int q = 0; q < 3; ++q) F[q] = Fx[q] + m.mul(s, Us[q] - Ux[q]);
   }
 };
 
