@@ -192,7 +192,9 @@ swe_status swe_selftest_fp64(int64_t n, uint64_t seed, int64_t* div_mismatches, 
 /* n results of a point-wise routine on the caller's operands, by the device
  * build (device != 0) or the host build: kind 0 the reference's Bisection
  * (src/PointOperations.cpp:26-40) of x^3 + b x^2 + c x + d, operands (d, c, b,
- * xmin, xmax) per result; kind 1 the correctly rounded cube root. */
+ * xmin, xmax) per result; kind 1 the correctly rounded cube root; kind 2 the
+ * product of two operands by the device's integer routine, the NaN
+ * 0x7FF8000000000123 where it leaves them to the FP64 instruction. */
 swe_status swe_selftest_pointwise(int32_t kind, int64_t n, const double* in, double* out, int32_t device);
 
 /* Compares the hand-written reverse of the flux plugin (flux, wavespeed) with

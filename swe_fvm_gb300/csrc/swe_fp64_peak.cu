@@ -143,7 +143,13 @@ __host__ __device__ constexpr int pointwise_args(int kind) { return kind == 0 ? 
 __host__ __device__ double pointwise(int kind, const double* a) {
   if (kind == 0) return swe::bisection(a[0], a[1], a[2], a[3], a[4]);
   if (kind == 1) return swe::cbrt_rn(a[0]);
+#if defined(__CUDA_ARCH__)
+  bool other = false;
+  const double r = swe::dmul_rn(a[0], a[1], &other);
+  return other ? __longlong_as_double(0x7FF8000000000123ll) : r;
+#else
   return a[0] * a[1];
+#endif
 }
 __global__ void k_pointwise(int kind, int n, const double* in, double* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;

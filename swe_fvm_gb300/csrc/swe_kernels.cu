@@ -55,6 +55,15 @@ namespace {
 
 constexpr double kInf = __builtin_huge_val();
 
+// Meshes and batches from this many cells up (two warps per scheduler) form the
+// products of the flux and update kernels on the integer pipe (Products).
+// GB300's FP64 pipe holds a warp instruction for 64 cycles; an integer product
+// takes about 26 issue slots of other pipes, so with both at work the kernels
+// issue FP64 for the additions only: 1M-cell dam break, k_flux 180 -> 141 us,
+// k_update 147 -> 99 us, step 773 -> 617 us; 250k-cell coast 339 -> 292 us.  With
+// fewer warps the integer product is the longer chain (148 against 74 cycles):
+// 44,402 cells 139 -> 137 us, 25,088 134.7 -> 135.4 us, 12,482 132 -> 135 us a step.
+constexpr int64_t kSoftCells = 40000;
 
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 
@@ -825,6 +834,7 @@ std::string Engine::init(std::vector<HostInstance>&& inst, int flux, int ws, int
   cell_off[I] = C;
   edge_off[I] = E;
   node_off[I] = N;
+  soft_ = C >= kSoftCells;
   cor0_ = true;
   for (const auto& q : inst) cor0_ = cor0_ && q.cor == 0.;
   if (3 * C > (1ll << 31) - 1 || E > (1ll << 31) - 1 || N > (1ll << 31) - 1) {

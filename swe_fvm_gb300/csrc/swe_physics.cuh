@@ -421,13 +421,17 @@ SWE_HD void cons_assign(double b, double h, double hu, double hv, double* ow, do
 }
 
 // -------------------------------------------------------------- edge flux
-// How a flux or update multiplies; other is set when the evaluation is to be
-// done again with Products<false>.
+// How a flux or update multiplies: on the integer pipe (SOFT, the same bits;
+// dmul_rn) or on the FP64 pipe.  other is set when an operand was outside
+// dmul_rn's range: the evaluation is then to be done again with Products<false>.
 template <bool SOFT>
 struct Products {
   bool other = false;
   SWE_HD double mul(double a, double b) {
-return a * b;
+#if defined(__CUDA_ARCH__)
+    if (SOFT) return dmul_rn(a, b, &other);
+#endif
+    return a * b;
   }
 };
 

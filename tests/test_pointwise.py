@@ -1,5 +1,5 @@
-"""Routines that reach the reference's bits another way, against the oracle:
-the bisection that evaluates the cubic only where rounding can hide its sign,
+"""Routines that reach the reference's bits another way, against the oracle
+(the product against IEEE arithmetic): the integer-pipe product, the bisection that evaluates the cubic only where rounding can hide its sign,
 and the cube root from a single-precision start.  Equality is exact."""
 
 import numpy as np
@@ -74,6 +74,36 @@ def check_cbrt(device):
     got = run(1, x[:, None], device)
     want = np.array([L.oracle_cbrt_rn(v) for v in x])
     assert np.array_equal(got.view(np.int64), want.view(np.int64))
+
+
+def operands(rng, n):
+    """Products over exponents of every range, ties, powers of two, zeros, subnormals and specials."""
+    def one():
+        exp = np.where(rng.random(n) < 0.6, rng.integers(1003, 1043, n),
+                       np.where(rng.random(n) < 0.5, rng.integers(505, 1540, n), rng.integers(0, 2048, n)))
+        man = rng.integers(0, 1 << 52, n)
+        man = np.where(rng.random(n) < 0.3, man & ~((1 << 27) - 1), man)  # short ones: exact products and ties
+        man = np.where(rng.random(n) < 0.1, rng.choice([0, 1, (1 << 52) - 1, 1 << 51], n), man)
+        x = ((rng.integers(0, 2, n) << 63) | (exp << 52) | man).astype(np.int64).view(np.float64)
+        return np.where(rng.random(n) < 0.05, rng.choice([0.0, -0.0, np.inf, np.nan, 5e-324, 1.0], n), x)
+
+    return np.stack([one(), one()], 1)
+
+
+@pytest.mark.gpu
+def test_product_device(gpu):
+    """The integer product has the FP64 instruction's bits, or says that it leaves the operands to it: never for
+    zeros and exponents from 2^-510 to 2^510."""
+    a = operands(np.random.default_rng(13), 400000)
+    got = run(2, a, True).view(np.int64)
+    with np.errstate(all="ignore"):
+        want = (a[:, 0] * a[:, 1]).view(np.int64)
+    left = got == 0x7FF8000000000123
+    assert np.array_equal(got[~left], want[~left])
+    mag = np.abs(a)
+    fine = ((mag == 0) | ((mag > 2.0 ** -510) & (mag < 2.0 ** 510))).all(1)
+    assert not (left & fine).any()
+    assert fine.sum() > 100000 and left.sum() > 10000
 
 
 MAKES = [one_vertex_dry, partly_wet_level, any_cubic]
