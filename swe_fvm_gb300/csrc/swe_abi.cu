@@ -230,6 +230,7 @@ swe_status upload_prim(Engine& eng, const double* prim, int64_t c0, int64_t n, s
   // one copy of the interleaved field into the staging buffer, then a device
   // unpack that also flags non-finite values
   unsigned* flag = eng.d_ioflag;
+  eng.state_changed();
   cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(unsigned), eng.stream());
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(eng.d_io, prim, 3 * n * sizeof(double), cudaMemcpyHostToDevice, eng.stream());
@@ -277,7 +278,7 @@ swe_status prime(Engine& eng, std::string* err) {
   cudaError_t e = eng.reset_pass();
   if (e == cudaSuccess) e = eng.interface_values(eng.state(0, 0), eng.state(0, 1), eng.state(0, 2));
   if (e == cudaSuccess) e = eng.fluxes(eng.state(0, 0));
-  if (e == cudaSuccess) e = eng.reset_pass();
+  if (e == cudaSuccess) e = eng.reset_pass(false);  // the list stays for the next step
   if (e != cudaSuccess) return cuda_fail(err, e, "priming flux pass");
   return SWE_OK;
 }
@@ -609,6 +610,7 @@ swe_status swe_set_prim_device(swe_ctx* ctx, const double* in) {
   if (!ctx || !in) return SWE_ERR_INVALID_ARGUMENT;
   Engine& g = ctx->eng;
   const int n = g.C();
+  g.state_changed();
   k_unpack<<<(n + 255) / 256, 256, 0, g.stream()>>>(in, g.state(0, 0), g.state(0, 1), g.state(0, 2), n, nullptr,
                                                      g.d_cell_from);
   cudaError_t e = cudaGetLastError();
@@ -1125,6 +1127,7 @@ swe_status swe_batch_set_prim_device(swe_batch* b, int32_t q, const double* in) 
   if (!b || !in || q < 0 || q >= b->eng.I()) return SWE_ERR_INVALID_ARGUMENT;
   Engine& g = b->eng;
   const int64_t c0 = g.cell_off[q], n = g.cell_off[q + 1] - c0;
+  g.state_changed();
   k_unpack<<<(int)((n + 255) / 256), 256, 0, g.stream()>>>(in, g.state(0, 0) + c0, g.state(0, 1) + c0,
                                                             g.state(0, 2) + c0, (int)n, nullptr,
                                                             g.d_cell_from ? g.d_cell_from + c0 : nullptr);

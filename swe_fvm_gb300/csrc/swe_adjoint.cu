@@ -1156,6 +1156,7 @@ std::string Engine::adjoint_backward(const double* trace_grads_host, double* gra
   AdjointState& a = *adj_;
   AdjWork& w = a.aw;
   w.reg_depth = adj_reg_depth_;
+  state_changed();  // the recompute may go through the step's own list
   const int64_t C = mesh_.C, N = mesh_.N;
   const Scheme sc = a.sc;
   const int ns = sc.n;
@@ -1262,9 +1263,10 @@ std::string Engine::adjoint_backward(const double* trace_grads_host, double* gra
             // the plain stage's kernels with PartWet2 and the fluxes next to
             // partially-wet cells on the side stream, keeping every
             // intermediate (k_drain_keep leaves the node maxima and the list)
-            launch_recon1(in[0], in[1], in[2], s == 0 ? 2 : 0, true);
+            launch_recon1(in[0], in[1], in[2], s == 0 ? 2 : 0, true, true);
             cudaEventRecord(ev_fork_, stream_);
             cudaStreamWaitEvent(side_, ev_fork_, 0);
+            launch_partwet1(in[0], side_);
             launch_recon2(in[0], in[1], in[2], side_, true);
             stage_fluxes_pw(in, side_);
             cudaEventRecord(ev_join_, side_);
@@ -1278,6 +1280,7 @@ std::string Engine::adjoint_backward(const double* trace_grads_host, double* gra
           work_ = saved;
         } else {
           e = reset_pass();
+          if (e == cudaSuccess) e = list_partwet(in[0]);
           if (e == cudaSuccess) e = launch_stage(sc.s[s], in, u0, out, s == 0, s == 0 ? 2 : 0);
         }
         if (e != cudaSuccess) return e;

@@ -156,12 +156,12 @@ __device__ void cell_record(const DevMesh& m, const BedArrays& o, int i) {
   const P3 t = centroid(P[0], P[1], P[2]);
   const double bc = t[2];
   o.bc[i] = bc;
-  o.wetthr[i] = least(bc + kWetDepth, [&](double w) { return is_wet(w - bc); });
+  const double wet = least(bc + kWetDepth, [&](double w) { return is_wet(w - bc); });
   // src/MUSCLObject.cpp:17-25 (maxCoeff of the node z)
   double mx = P[0][2];
   if (dlt(mx, P[1][2])) mx = P[1][2];
   if (dlt(mx, P[2][2])) mx = P[2][2];
-  o.fwthr[i] = boundary ? __longlong_as_double(0x7FF0000000000000ll) : mx;
+  o.thr[i] = make_double2(wet, boundary ? __longlong_as_double(0x7FF0000000000000ll) : mx);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
     o.zn[k * C + i] = P[k][2];

@@ -77,8 +77,8 @@ struct DevMesh {
   const int* cedge;           // [3][C]
   const unsigned char* cown;  // [C] bit k: this cell owns edge k; bit 3: a slot of its dry plane is wet
   const double* bc;           // [C] centroid bathymetry
-  const double* wetthr;       // [C] least w whose depth w - bc is wet
-  const double* fwthr;        // [C] max node z, +inf for boundary cells
+  const double2* thr;         // [C] levels that class a cell: x the least w whose depth
+                              // w - bc is wet, y max node z (+inf for boundary cells)
   const double* area;         // [C]
   const double* zn;           // [3][C] node z
   const double* ze;           // [3][C] edge-centre z
@@ -125,7 +125,8 @@ struct DevMesh {
 // The records that depend on the bathymetry, as the device computes them
 // (DevMesh's arrays of the same names).
 struct BedArrays {
-  double *bc, *wetthr, *fwthr, *zn, *ze, *dry, *combo, *combov, *pw1, *ezm, *nz;
+  double *bc, *zn, *ze, *dry, *combo, *combov, *pw1, *ezm, *nz;
+  double2* thr;
   Pw2Rec* pw2;
   unsigned char* cown;  // bit 3 only
   SlotRec* srec;  // ze only
@@ -282,7 +283,11 @@ class Engine {
 
   // Resets the node maxima and the part-wet list (done by k_drain at the end
   // of every stage; needed before a standalone reconstruction).
-  cudaError_t reset_pass();
+  // list: the part-wet list too.
+  cudaError_t reset_pass(bool list = true);
+  // The state in buffer 0 was written from outside: its part-wet list is to be
+  // made before the next step (a step leaves the next one's).
+  void state_changed() { list_valid_ = false; }
   // Launches one reconstruction (pass 1 + pass 2) with the full interface
   // values, and one flux pass from them.
   cudaError_t interface_values(const double* W, const double* U, const double* V);
@@ -379,7 +384,7 @@ class Engine {
   // second stream of a stage: PartWet2 and the fluxes of the edges next to
   // partially-wet cells run on it while the other edges' fluxes run on stream_
   cudaStream_t side_ = nullptr;
-  cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr;
+  cudaEvent_t ev_fork_ = nullptr, ev_pass1_ = nullptr, ev_join_ = nullptr;
   int flux_ = 1, ws_ = 2;
   int blk_[3] = {256, 256, 256};  // reconstruction, edge flux, drain/update
   bool batched_ = false;
@@ -387,7 +392,12 @@ class Engine {
   double* d_integrals_ = nullptr;  // partial sums of the integrals
   // slots: also the full interface values (DevWork::ew ...).  latch_mode: 0
   // none, 1 the CFL dt, 2 the fixed dt, 3 none and the CFL ratio kept
-  void launch_recon1(const double* W, const double* U, const double* V, int latch_mode, bool slots);
+  void launch_recon1(const double* W, const double* U, const double* V, int latch_mode, bool slots, bool append);
+  void launch_partwet1(const double* W, cudaStream_t s);
+  int listed_blocks() const;
+  cudaError_t list_partwet(const double* W);  // empties the list and fills it from W
+  cudaError_t ensure_list();
+  bool list_valid_ = false;  // the part-wet list is that of the state in buffer 0
   void launch_recon2(const double* W, const double* U, const double* V, cudaStream_t s, bool slots);
   // the fluxes of a stage's input: the edges with no partially-wet cell, and
   // the others (those of the listed cells) on stream s

@@ -1,11 +1,12 @@
 // swe_kernels.cu -- sm_103a kernels of one Runge-Kutta stage and the engine
 // that sequences them.
 //
-// A stage (src/Solvers.cpp:5-59) is six kernels over the concatenated cells
+// A stage (src/Solvers.cpp:5-59) is seven kernels over the concatenated cells
 // and edges of every instance:
 //   k_recon1  all cells    SpaceDisc::ComputeInterfaceValues pass 1
 //                          (src/SpaceDisc.cpp:37-45), listing the partially
-//                          wet cells
+//                          wet cells (in a step the update before lists them)
+//   k_partwet1 part-wet    their pass-1 level, on a second stream beside it
 //   k_recon2  part-wet     pass 2 (src/SpaceDisc.cpp:47-51), gathering the
 //                          node maximum it reads from the pass-1 values of
 //                          the node's cells (order-independent)
@@ -30,6 +31,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <type_traits>
 
 #include "swe_engine.cuh"
 
@@ -167,33 +169,46 @@ __device__ __forceinline__ bool at_point_wet(double w0, double off, double z, do
 
 // Pass-1 AtPoint value of cell c at its local node kn, from what pass 1 left:
 // the class byte (dry / partially wet / fully wet, combination mask, plane
-// kept), the PartWet1 level of a partially-wet cell and the state.
+// kept), the PartWet1 level of a partially-wet cell and the state.  (a - z >= 0
+// is a >= z: the sign of a difference is exact.)
 __device__ __forceinline__ double pass1_value(const DevMesh& m, const DevWork& wk, const double* __restrict__ W,
                                               int c, int kn) {
   const int C = m.C;
   const unsigned cl = wk.cls[c];
-  if ((cl & 3u) == 0u) return m.dry[(size_t)c * kDryStride + kn];
+  const unsigned type = cl & 3u;
   const double z = m.zn[kn * C + c];
-  double val;
-  if ((cl & 3u) == 1u) {
-    at_point_wet(wk.pwrec[c], 0., z, &val);  // the PartWet1 level, a flat plane
-  } else {
-    // the combination plane's vertex offset when pass 1 kept the plane, else flat
-    const double off = (cl & 32u) ? m.combov[combov_off(C, c, (int)((cl >> 2) & 7u)) + kn] : 0.;
-    at_point_wet(W[c], off, z, &val);
-  }
-  return val;
+  // level (the PartWet1 level is a flat plane's), and the kept plane's offset
+  const double* from = type == 0u ? m.dry + (size_t)c * kDryStride + kn : type == 1u ? wk.pwrec + c : W + c;
+  double val = *from;
+  if (type == 2u && (cl & 32u)) val = val + m.combov[combov_off(C, c, (int)((cl >> 2) & 7u)) + kn];
+  return type == 0u || dle(z, val) ? val : z;
 }
 
 // The node maximum m_max_wp of node nd (src/MUSCLObject.cpp:13-36): the
 // largest pass-1 AtPoint value of the cells around it, starting from the
 // node's bathymetry (every AtPoint value is >= it).  A maximum is exact and
 // order-free, so gathering it where it is needed gives the value the
-// reference's accumulation over its cell loop gives.
+// reference's accumulation over its cell loop gives.  LANES = 8: the whole warp
+// calls, and each group of 8 lanes shares its node's cells.
+template <int LANES>
 __device__ __forceinline__ unsigned long long node_max_key(const DevMesh& m, const DevWork& wk,
                                                            const double* __restrict__ W, int nd) {
   unsigned long long key = order_key(m.nz[nd]);
   const int q0 = m.nptr[nd], q1 = m.nptr[nd + 1];
+  if (LANES > 1) {
+    for (int q = q0 + (int)(threadIdx.x & (LANES - 1)); q < q1; q += LANES) {
+      const int c = m.ncell[gidx(wk, q, 3 * m.C)];
+      const unsigned long long k = order_key(pass1_value(m, wk, W, gidx(wk, c >> 2, m.C), c & 3));
+      key = k > key ? k : key;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int off = LANES / 2; off; off >>= 1) {
+      const unsigned long long o = __shfl_xor_sync(0xFFFFFFFFu, key, off, LANES);
+      key = o > key ? o : key;
+    }
+    return key;
+  }
   // the first 8 cells (a triangulation node has about 6) with their loads
   // issued together, the rest one by one
   constexpr int kV = 8;
@@ -215,25 +230,61 @@ __device__ __forceinline__ unsigned long long node_max_key(const DevMesh& m, con
   return key;
 }
 
-// PartWet1 level (src/MUSCLObject.cpp:86-112)
+// PartWet1 level (src/MUSCLObject.cpp:86-112).  LANES = 8: the whole warp calls,
+// a cell to each group of 8 lanes.
+template <int LANES>
 __device__ __forceinline__ double partwet1_level(const double* __restrict__ p, double w, double h) {
-  const double b13 = p[0], b23 = p[1], b12 = p[2], bdel = p[3];
-  if (dle(b13, w)) return w;
-  if (dle(w, bdel)) return b23 + cbrt_rn(3. * h * p[6] * p[7]);
-  double cc = p[6] * (3. * h * p[8] - p[9]) - p[10];
-  (void)b12;
-  return bisection(cc, p[5], p[4], p[2], b13);
+  const double b13 = p[0], b23 = p[1], bdel = p[3];
+  const bool above_all = dle(b13, w), cube = !above_all && dle(w, bdel), bisect = !above_all && !cube;
+  double level = w;
+  if (cube) level = b23 + cbrt_rn(3. * h * p[6] * p[7]);
+  if (LANES > 1 ? __any_sync(0xFFFFFFFFu, bisect) : bisect) {
+    const double cc = p[6] * (3. * h * p[8] - p[9]) - p[10];
+    const double root = LANES > 1 ? bisection_group<false>(cc, p[5], p[4], p[2], b13, bisect)
+                                  : bisection(cc, p[5], p[4], p[2], b13);
+    if (bisect) level = root;
+  }
+  return level;
+}
+
+// Appends the lanes' partially-wet cells to the list, one atomic a warp (every
+// lane of the warp calls).
+__device__ __forceinline__ void append_listed(const DevWork& wk, int C, bool part, int i) {
+  const unsigned bal = __ballot_sync(0xffffffffu, part);
+  if (bal) {
+    const int leader = __ffs(bal) - 1;
+    int base = 0;
+    if (lane_id() == leader) base = atomicAdd(wk.pwcount, __popc(bal));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    const int slot = base + __popc(bal & ((1u << lane_id()) - 1u));
+    if (part && slot < C) wk.pwlist[slot] = i;
+  }
+}
+
+// Whether cell i with level w is partially wet (neither dry nor fully wet,
+// src/MUSCLObject.cpp:13-29).
+__device__ __forceinline__ bool partly_wet(const DevMesh& m, int i, double w) {
+  const double2 t = __ldg(m.thr + i);
+  return !dlt(w, t.x) && !dlt(t.y, w);
+}
+
+// The partially-wet cells of a state that no update left (a new state or bed).
+__global__ void __launch_bounds__(256) k_list_partwet(DevMesh m, DevWork wk, const double* __restrict__ W) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  append_listed(wk, m.C, i < m.C && partly_wet(m, i, W[i]), i);
 }
 
 // ---------------------------------------------------------------- kernels
-// Pass 1.  Bound by its gathers and, on wetting fronts, by PartWet1's chain.
+// Pass 1 but for the partly wet cells' levels (k_partwet1, beside it).  Bound by
+// its gathers.  append: list those cells (a step's are listed by the update
+// before it).
 // The wet test and the plane's positivity are comparisons with levels kept in
-// the mesh (DevMesh::wetthr, record entry 2) where the rounded sums would cost
+// the mesh (DevMesh::thr, record entry 2) where the rounded sums would cost
 // seven FP64 operations; 6 are left in a fully-wet cell of 18.
 template <bool BATCH, int FORM>
 __global__ void __launch_bounds__(256, 5) k_recon1(DevMesh m, DevWork wk, const double* __restrict__ W,
                                                 const double* __restrict__ U, const double* __restrict__ V,
-                                                int latch_mode) {
+                                                int latch_mode, bool append) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   bool part = false;
   unsigned char cls = 0;  // dry unless set below
@@ -260,7 +311,8 @@ __global__ void __launch_bounds__(256, 5) k_recon1(DevMesh m, DevWork wk, const 
     const double w = W[i];
     const double u = FORM == kLean ? 0. : U[i], v = FORM == kLean ? 0. : V[i];
     double gx = 0., gy = 0.;
-    if (dlt(w, m.wetthr[i])) {
+    const double2 level = __ldg(m.thr + i);
+    if (dlt(w, level.x)) {
       // ReconstructDryCell: every value is a mesh constant
       const double* dr = m.dry + (size_t)i * kDryStride;
       gx = dr[6];
@@ -274,9 +326,8 @@ __global__ void __launch_bounds__(256, 5) k_recon1(DevMesh m, DevWork wk, const 
         const double h = wet_slots ? dr[3 + k] - be : 0.;
         write_slot<FORM>(wk, slot, h, be, FORM == kLean ? 0. : dr[3 + k], 0., 0., gx, gy, cor);
       }
-    } else if (!dlt(m.fwthr[i], w)) {
-      // partially wet: the PartWet1 level now, PartWet2 in k_recon2
-      wk.pwrec[i] = partwet1_level(m.pw1 + (size_t)i * kPw1Stride, w, w - m.bc[i]);
+    } else if (!dlt(level.y, w)) {
+      // partially wet: listed for k_partwet1 and k_recon2
       part = true;
       cls = 1;
     } else {
@@ -289,9 +340,10 @@ __global__ void __launch_bounds__(256, 5) k_recon1(DevMesh m, DevWork wk, const 
         const int nb = gidx(wk, m.cnbr[k * C + i], C);  // never a wall: fully-wet cells are interior
         const double wj = W[nb];
         wn[k] = wj;
-        if (dlt(m.fwthr[nb], wj)) {
+        const double2 tj = __ldg(m.thr + nb);
+        if (dlt(tj.y, wj)) {
           // fully-wet neighbour: plane point at its centroid
-        } else if (dlt(wj, m.wetthr[nb])) {
+        } else if (dlt(wj, tj.x)) {
           first_order = true;
         } else {
           mask |= 1 << k;  // partially-wet neighbour: plane point at the edge centre
@@ -337,16 +389,7 @@ __global__ void __launch_bounds__(256, 5) k_recon1(DevMesh m, DevWork wk, const 
     }
     wk.cls[i] = cls;
   }
-  // warp-aggregated append of the partially-wet cells
-  const unsigned bal = __ballot_sync(0xffffffffu, part);
-  if (bal) {
-    const int leader = __ffs(bal) - 1;
-    int base = 0;
-    if (lane_id() == leader) base = atomicAdd(wk.pwcount, __popc(bal));
-    base = __shfl_sync(0xffffffffu, base, leader);
-    const int slot = base + __popc(bal & ((1u << lane_id()) - 1u));
-    if (part && slot < m.C) wk.pwlist[slot] = i;
-  }
+  if (append) append_listed(wk, m.C, part, i);
 }
 
 // Every node maximum (the reference's m_max_wp after pass 1), for the
@@ -354,89 +397,138 @@ __global__ void __launch_bounds__(256, 5) k_recon1(DevMesh m, DevWork wk, const 
 // only the nodes PartWet2 reads (k_recon2).
 __global__ void k_node_max_all(DevMesh m, DevWork wk, const double* __restrict__ W) {
   const int nd = blockIdx.x * blockDim.x + threadIdx.x;
-  if (nd < m.N) wk.maxwp[nd] = node_max_key(m, wk, W, nd);
+  if (nd < m.N) wk.maxwp[nd] = node_max_key<1>(m, wk, W, nd);
 }
 
-// ReconstructPartWetCell2 (src/MUSCLObject.cpp:114-191) over the listed cells.
-template <bool BATCH, int FORM>
-__global__ void __launch_bounds__(256) k_recon2(DevMesh m, DevWork wk, const double* __restrict__ W,
-                                                const double* __restrict__ U, const double* __restrict__ V) {
-  const int C = m.C;
-  const int n = min(*wk.pwcount, C);
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
-    const int i = gidx(wk, wk.pwlist[q], C);
-    const int inst = BATCH ? m.cinst[i] : 0;
-    const double cor = m.inst_cor[inst];
+// The partly wet cells' work is one long chain a cell (PartWet1's cube root or
+// bisection, then the node maximum's gather, PartWet2's roots or bisection and a
+// plane solve), and few cells have it: the kernels last as long as the chain.
+// With up to kGroupCells listed, 8 lanes share a cell: they gather the node's
+// cells together, take three steps of a bisection for one evaluation and a slot
+// each.  Longer lists fill the SMs with one lane a cell (8 lanes issue about
+// half of each cell's instructions each).  SSPRK2 step with 8 lanes, with one:
+// 8192-cell Thacker bowl (200 listed) 120, 126 us; 25k-cell coast (2900) 134,
+// 140 us; 250k-cell coast (14000) 306, 286 us.
+constexpr int kGroupCells = 8000;
+
+// Calls work.template operator()<LANES>(cell, own) for the listed cells: with 8
+// lanes a cell the warp goes through its four cells together (a group past the
+// end repeats the last cell and owns nothing).
+template <class F>
+__device__ __forceinline__ void for_listed(const DevMesh& m, const DevWork& wk, F&& work) {
+  const int n = min(*wk.pwcount, m.C);
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+  if (n <= kGroupCells) {
+    for (int q0 = (t >> 5) * 4; q0 < n; q0 += (nt >> 5) * 4) {
+      const int q = q0 + ((t >> 3) & 3);
+      work(std::integral_constant<int, 8>{}, gidx(wk, wk.pwlist[min(q, n - 1)], m.C), q < n);
+    }
+  } else {
+    for (int q = t; q < n; q += nt) work(std::integral_constant<int, 1>{}, gidx(wk, wk.pwlist[q], m.C), true);
+  }
+}
+
+// PartWet1 level of the listed cells.
+__global__ void __launch_bounds__(128) k_partwet1(DevMesh m, DevWork wk, const double* __restrict__ W) {
+  for_listed(m, wk, [&](auto lanes, int i, bool own) {
+    constexpr int L = decltype(lanes)::value;
     const double w = W[i];
-    const double u = FORM == kLean ? 0. : U[i], v = FORM == kLean ? 0. : V[i];
-    const Pw2Rec& r = m.pw2[i];
-    const double b23 = r.p[0][2], b12 = r.p[1][2], b13 = r.p[2][2];
-    double w0 = wk.pwrec[i];  // PartWet1 fallback level
-    double gx = 0., gy = 0.;
-    bool plane = false;
-    if (!(dlt(b13, w) || r.flat)) {
-      // the node maximum of the lowest node, gathered from its cells' pass-1
-      // values; kept in maxwp for the adjoint's reverse of this cell
-      const int lo = gidx(wk, r.lo, m.N);
-      const unsigned long long key = node_max_key(m, wk, W, lo);
-      wk.maxwp[lo] = key;
-      const double w23 = order_val(key);
-      const double h23 = w23 - b23;
-      const double ratio_b = r.ratio_b;
-      const double h_delim1 = 1. / 3. * h23 * ratio_b;
-      const double h_delim2 = SWE_DIV(1. / 3. * h23 * r.hd2f, r.d13);
-      const double hi = w - m.bc[i];
-      const double ratio_h = SWE_DIV(hi, h23);
-      // columns of the reference's `points` after all its writes: point 0 is
-      // the lowest vertex with its bathymetry (see the restatement's notes)
-      double p1x, p1y, p1z, p2x, p2y, p2z;
-      bool ok = true;
-      if (dle(hi, h_delim1)) {
-        const double k2 = SWE_SQRT(SWE_DIV(3. * ratio_h, ratio_b));
-        p1x = k2 * r.p[1][0] + (1. - k2) * r.p[0][0];
-        p1y = k2 * r.p[1][1] + (1. - k2) * r.p[0][1];
-        p1z = k2 * r.p[1][2] + (1. - k2) * r.p[0][2];
-        const double k3 = SWE_SQRT(3. * ratio_h * ratio_b);
-        p2x = k3 * r.p[2][0] + (1. - k3) * r.p[0][0];
-        p2y = k3 * r.p[2][1] + (1. - k3) * r.p[0][1];
-        p2z = k3 * r.p[2][2] + (1. - k3) * r.p[0][2];
-      } else if (dle(h_delim2, hi)) {
-        const double delta_w = 1.5 * (hi - h_delim2);
-        p1x = r.p[1][0]; p1y = r.p[1][1]; p1z = r.p[1][2];
-        p2x = r.p[2][0]; p2y = r.p[2][1]; p2z = r.p[2][2];
-        p2z += delta_w;
-      } else {
-        const double alpha = 3. * ratio_h;
-        const double beta = r.beta;
-        const double k1 = 1. - bisection(SWE_DIV(1. + beta - alpha, beta * beta), SWE_DIV(alpha - 3., beta), 0., 0., 1.);
-        if (dltc(k1, kTol)) {
-          ok = false;
-        } else {
-          const double bp1 = k1 * b13 + (1. - k1) * b12;
-          p1x = r.p[1][0]; p1y = r.p[1][1]; p1z = r.p[1][2];
-          p2x = k1 * r.p[2][0] + (1. - k1) * r.p[1][0];
-          p2y = k1 * r.p[2][1] + (1. - k1) * r.p[1][1];
-          p2z = bp1;
-        }
-      }
-      if (ok) {
-        plane_gradient(r.p[0][0], r.p[0][1], r.p[0][2], p1x, p1y, p1z, p2x, p2y, p2z, &gx, &gy);
-        w0 = w23 + (gx * r.tp0x + gy * r.tp0y);
-        plane = true;
+    const double level = partwet1_level<L>(m.pw1 + (size_t)i * kPw1Stride, w, w - m.bc[i]);
+    if (own && (threadIdx.x & (L - 1)) == 0) wk.pwrec[i] = level;
+  });
+}
+
+// ReconstructPartWetCell2 (src/MUSCLObject.cpp:114-191) of cell i by LANES lanes
+// (the whole warp calls where that is 8).
+template <bool BATCH, int FORM, int LANES>
+__device__ __forceinline__ void partwet2_cell(const DevMesh& m, const DevWork& wk, const double* __restrict__ W,
+                                              const double* __restrict__ U, const double* __restrict__ V, int i,
+                                              bool own) {
+  const int C = m.C;
+  const int lane = (int)(threadIdx.x & (LANES - 1));
+  auto any = [](bool p) { return LANES > 1 ? __any_sync(0xFFFFFFFFu, p) != 0 : p; };
+  const int inst = BATCH ? m.cinst[i] : 0;
+  const double cor = FORM == kLean ? 0. : m.inst_cor[inst];
+  const double w = W[i];
+  const double u = FORM == kLean ? 0. : U[i], v = FORM == kLean ? 0. : V[i];
+  const Pw2Rec& r = m.pw2[i];
+  const double b23 = r.p[0][2], b12 = r.p[1][2], b13 = r.p[2][2];
+  double w0 = wk.pwrec[i];  // PartWet1 fallback level
+  double gx = 0., gy = 0.;
+  bool plane = !(dlt(b13, w) || r.flat);
+  if (any(plane)) {
+    // the node maximum of the lowest node, gathered from its cells' pass-1
+    // values; kept in maxwp for the adjoint's reverse of this cell
+    const int lo = gidx(wk, r.lo, m.N);
+    const unsigned long long key = node_max_key<LANES>(m, wk, W, lo);
+    if (own && plane && lane == 0) wk.maxwp[lo] = key;
+    const double w23 = order_val(key);
+    const double h23 = w23 - b23;
+    const double ratio_b = r.ratio_b;
+    const double h_delim1 = 1. / 3. * h23 * ratio_b;
+    const double h_delim2 = SWE_DIV(1. / 3. * h23 * r.hd2f, r.d13);
+    const double hi = w - m.bc[i];
+    const double ratio_h = SWE_DIV(hi, h23);
+    // columns of the reference's `points` after all its writes: point 0 is
+    // the lowest vertex with its bathymetry (see the restatement's notes)
+    double p1x = r.p[1][0], p1y = r.p[1][1], p1z = b12;
+    double p2x = r.p[2][0], p2y = r.p[2][1], p2z = b13;
+    const bool one = plane && dle(hi, h_delim1), three = plane && !one && dle(h_delim2, hi);
+    const bool two = plane && !one && !three;  // vertices wet
+    if (one) {
+      const double k2 = SWE_SQRT(SWE_DIV(3. * ratio_h, ratio_b));
+      const double k3 = SWE_SQRT(3. * ratio_h * ratio_b);
+      const double j2 = 1. - k2, j3 = 1. - k3;
+      p1x = k2 * p1x + j2 * r.p[0][0];
+      p1y = k2 * p1y + j2 * r.p[0][1];
+      p1z = k2 * p1z + j2 * r.p[0][2];
+      p2x = k3 * p2x + j3 * r.p[0][0];
+      p2y = k3 * p2y + j3 * r.p[0][1];
+      p2z = k3 * p2z + j3 * r.p[0][2];
+    }
+    if (three) p2z += 1.5 * (hi - h_delim2);
+    if (any(two)) {
+      const double alpha = 3. * ratio_h;
+      const double beta = r.beta;
+      const double cd = SWE_DIV(1. + beta - alpha, beta * beta), cc = SWE_DIV(alpha - 3., beta);
+      const double k1 = 1. - (LANES > 1 ? bisection_group<true>(cd, cc, 0., 0., 1., two) : bisection01(cd, cc));
+      if (two) {
+        const double j1 = 1. - k1;
+        p2x = k1 * p2x + j1 * r.p[1][0];
+        p2y = k1 * p2y + j1 * r.p[1][1];
+        p2z = k1 * b13 + j1 * b12;
+        if (dltc(k1, kTol)) plane = false;
       }
     }
+    if (plane) {
+      plane_gradient(r.p[0][0], r.p[0][1], r.p[0][2], p1x, p1y, p1z, p2x, p2y, p2z, &gx, &gy);
+      w0 = w23 + (gx * r.tp0x + gy * r.tp0y);
+    }
+  }
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
+  for (int k0 = 0; k0 < (LANES > 1 ? 1 : 3); ++k0) {
+    const int k = LANES > 1 ? lane : k0;
+    if (own && k < 3) {
       const int slot = k * C + i;
       const double be = m.ze[slot];
       const double off = plane ? (gx * r.dedge[k][0] + gy * r.dedge[k][1]) : 0.;
       const double at = w0 + off, h = at - be;
-      const bool above = dge0(h);
-      write_slot<FORM>(wk, slot, h, be, above ? at : be, above ? u : 0., above ? v : 0., gx, gy, cor);
+      const bool over = dge0(h);
+      write_slot<FORM>(wk, slot, h, be, over ? at : be, over ? u : 0., over ? v : 0., gx, gy, cor);
     }
+  }
+  if (own && lane == 0) {
     wk.gx[i] = gx;
     wk.gy[i] = gy;
   }
+}
+
+template <bool BATCH, int FORM>
+__global__ void __launch_bounds__(128) k_recon2(DevMesh m, DevWork wk, const double* __restrict__ W,
+                                                const double* __restrict__ U, const double* __restrict__ V) {
+  for_listed(m, wk, [&](auto lanes, int i, bool own) {
+    partwet2_cell<BATCH, FORM, decltype(lanes)::value>(m, wk, W, U, V, i, own);
+  });
 }
 
 // SpaceDisc::ComputeFluxes with flux plugin FLUX and the CFL min-reduction.
@@ -734,6 +826,7 @@ __global__ void __launch_bounds__(256, 5) k_update(DevMesh m, DevWork wk, const 
                                                 double* nst = nullptr) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m.C) return;
+  if (!STORE_N) prefetch_l1(m.thr + i);  // for the class of the new state, at the end
   double n[3];
   if (!update_cell<BATCH, HALF, COR0, SOFT>(m, wk, i, Wp, Up, Vp, W0, U0, V0, st, n))
     update_cell<BATCH, HALF, COR0, false>(m, wk, i, Wp, Up, Vp, W0, U0, V0, st, n);
@@ -754,12 +847,19 @@ __global__ void __launch_bounds__(256, 5) k_update(DevMesh m, DevWork wk, const 
                            xv = (unsigned long long)dbits(ov) >> 52;
   if (((xw & 0x7FFull) == 0x7FFull) || ((xu & 0x7FFull) == 0x7FFull) || ((xv & 0x7FFull) == 0x7FFull))
     atomicOr(wk.err, kErrNonFinite);
+  // list the next stage's partially-wet cells, so that their PartWet1 runs beside
+  // its k_recon1 instead of after it (a plain append: one over the warp's lanes
+  // kept registers across the whole kernel, 99 -> 110 us on a million cells)
+  if (!STORE_N && partly_wet(m, i, ow)) {
+    const int slot = atomicAdd(wk.pwcount, 1);
+    if (slot < m.C) wk.pwlist[slot] = i;
+  }
 }
 
-__global__ void k_init_nodes(DevMesh m, DevWork wk) {
+__global__ void k_init_nodes(DevMesh m, DevWork wk, bool list) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < m.N) wk.maxwp[i] = order_key(m.nz[i]);
-  if (i == 0) *wk.pwcount = 0;
+  if (list && i == 0) *wk.pwcount = 0;
 }
 
 inline int nblocks(int64_t n, int b) { return (int)((n + b - 1) / b); }
@@ -776,6 +876,8 @@ T* Engine::dalloc(size_t n) {
   bytes_ += n * sizeof(T);
   return (T*)p;
 }
+template int* Engine::dalloc<int>(size_t);
+template double* Engine::dalloc<double>(size_t);
 
 void Engine::set_stream(cudaStream_t s) {
   cudaStream_t next = s ? s : own_stream_;
@@ -804,7 +906,15 @@ Engine::~Engine() {
   if (own_stream_) cudaStreamDestroy(own_stream_);
   if (side_) cudaStreamDestroy(side_);
   if (ev_fork_) cudaEventDestroy(ev_fork_);
+  if (ev_pass1_) cudaEventDestroy(ev_pass1_);
   if (ev_join_) cudaEventDestroy(ev_join_);
+}
+
+// The side stream's blocks go first wherever an SM has room: its kernels are short
+// and the stage waits for their chain.
+static int side_priority() {
+  int least = 0, greatest = 0;
+  return cudaDeviceGetStreamPriorityRange(&least, &greatest) == cudaSuccess ? greatest : 0;
 }
 
 std::string Engine::init(std::vector<HostInstance>&& inst, int flux, int ws, int block, int* st, bool batched) {
@@ -871,20 +981,20 @@ std::string Engine::init(std::vector<HostInstance>&& inst, int flux, int ws, int
   ok = ok && up(img.srec, bed_.srec) && up(img.cslot, p_cslot) && up(img.erec, bed_.erec) && up(img.eidx, p_eidx);
   const int *p_nptr, *p_ncell;
   ok = ok && up(img.nptr, p_nptr) && up(img.ncell, p_ncell);
-  bed_.bc = dalloc<double>(C); bed_.fwthr = dalloc<double>(C); bed_.wetthr = dalloc<double>(C);
+  bed_.bc = dalloc<double>(C); bed_.thr = dalloc<double2>(C);
   bed_.zn = dalloc<double>(3 * C); bed_.ze = dalloc<double>(3 * C);
   bed_.dry = dalloc<double>(kDryStride * C); bed_.combo = dalloc<double>(8 * kComboStride * C);
   bed_.combov = dalloc<double>(8 * kComboVStride * C);
   bed_.pw1 = dalloc<double>(kPw1Stride * C); bed_.pw2 = dalloc<Pw2Rec>(C);
   bed_.ezm = dalloc<double>(E); bed_.nz = dalloc<double>(N);
-  ok = ok && bed_.bc && bed_.fwthr && bed_.wetthr && bed_.combov && bed_.zn && bed_.ze && bed_.dry && bed_.combo && bed_.pw1 && bed_.pw2 &&
+  ok = ok && bed_.bc && bed_.thr && bed_.combov && bed_.zn && bed_.ze && bed_.dry && bed_.combo && bed_.pw1 && bed_.pw2 &&
        bed_.ezm && bed_.nz;
   if (!ok) {
     *st = 6;
     return std::string("device allocation or upload failed: ") + cudaGetErrorString(cudaGetLastError());
   }
   M.cnode = p_cnode; M.cnbr = p_cnbr; M.cedge = p_cedge; M.cinst = p_cinst; M.cown = bed_.cown;
-  M.bc = bed_.bc; M.fwthr = bed_.fwthr; M.wetthr = bed_.wetthr; M.combov = bed_.combov; M.area = p_area; M.zn = bed_.zn; M.ze = bed_.ze; M.cek = p_cek;
+  M.bc = bed_.bc; M.thr = bed_.thr; M.combov = bed_.combov; M.area = p_area; M.zn = bed_.zn; M.ze = bed_.ze; M.cek = p_cek;
   M.cnxc = p_cnxc; M.cnyc = p_cnyc; M.dry = bed_.dry; M.combo = bed_.combo; M.pw1 = bed_.pw1; M.pw2 = bed_.pw2;
   M.eown = p_eown; M.enb = p_enb; M.eslotl = p_esl; M.eslotr = p_esr; M.einst = p_einst;
   M.enx = p_enx; M.eny = p_eny; M.etx = p_etx; M.ety = p_ety; M.ezm = bed_.ezm; M.elmin = p_elmin;
@@ -943,8 +1053,9 @@ std::string Engine::init(std::vector<HostInstance>&& inst, int flux, int ws, int
   std::vector<unsigned long long> one(I, order_key(1.0));
   cudaMemcpy(Wk.r, one.data(), I * sizeof(unsigned long long), cudaMemcpyHostToDevice);
   if (cudaStreamCreateWithFlags(&own_stream_, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaStreamCreateWithPriority(&side_, cudaStreamNonBlocking, side_priority()) != cudaSuccess ||
       cudaEventCreateWithFlags(&ev_fork_, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&ev_pass1_, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&ev_join_, cudaEventDisableTiming) != cudaSuccess) {
     *st = 5;
     return "stream creation failed";
@@ -953,7 +1064,7 @@ std::string Engine::init(std::vector<HostInstance>&& inst, int flux, int ws, int
   host = std::move(inst);
   const std::vector<double> nz = host_nz();
   cudaError_t ce = compute_bed(nz.data());
-  k_init_nodes<<<nblocks(N, 256), 256, 0, stream_>>>(M, Wk);
+  k_init_nodes<<<nblocks(N, 256), 256, 0, stream_>>>(M, Wk, true);
   ++launches_;
   if (ce == cudaSuccess) ce = cudaGetLastError();
   const cudaError_t cs = cudaStreamSynchronize(stream_);  // also on failure: the copy reads nz
@@ -965,28 +1076,54 @@ std::string Engine::init(std::vector<HostInstance>&& inst, int flux, int ws, int
   return "";
 }
 
-cudaError_t Engine::reset_pass() {
-  k_init_nodes<<<nblocks(std::max(mesh_.N, 1), 256), 256, 0, stream_>>>(mesh_, work_);
+cudaError_t Engine::reset_pass(bool list) {
+  k_init_nodes<<<nblocks(std::max(mesh_.N, 1), 256), 256, 0, stream_>>>(mesh_, work_, list);
   launches_ += 1;
   return cudaGetLastError();
 }
 
-void Engine::launch_recon1(const double* W, const double* U, const double* V, int latch_mode, bool slots) {
+void Engine::launch_recon1(const double* W, const double* U, const double* V, int latch_mode, bool slots,
+                           bool append) {
   const int b = blk_[0], g = nblocks(mesh_.C, b);
   const int form = !slots ? kLean : cor0_ ? kSlotsCor0 : kSlotsCor;
   switch (form + (batched_ ? 3 : 0)) {
-    case 0: k_recon1<false, kLean><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode); break;
-    case 1: k_recon1<false, kSlotsCor0><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode); break;
-    case 2: k_recon1<false, kSlotsCor><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode); break;
-    case 3: k_recon1<true, kLean><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode); break;
-    case 4: k_recon1<true, kSlotsCor0><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode); break;
-    default: k_recon1<true, kSlotsCor><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode); break;
+    case 0: k_recon1<false, kLean><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode, append); break;
+    case 1: k_recon1<false, kSlotsCor0><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode, append); break;
+    case 2: k_recon1<false, kSlotsCor><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode, append); break;
+    case 3: k_recon1<true, kLean><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode, append); break;
+    case 4: k_recon1<true, kSlotsCor0><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode, append); break;
+    default: k_recon1<true, kSlotsCor><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode, append); break;
   }
   ++launches_;
 }
 
+// Blocks of the kernels over the listed cells (128 threads): one lane a cell for
+// every cell, or 8 for kGroupCells of them, at most one full device.
+int Engine::listed_blocks() const {
+  const int b = 128;
+  return std::min(std::max(nblocks(mesh_.C, b), nblocks(8ll * std::min(mesh_.C, kGroupCells), b)), 6 * 152);
+}
+
+void Engine::launch_partwet1(const double* W, cudaStream_t s) {
+  k_partwet1<<<listed_blocks(), 128, 0, s>>>(mesh_, work_, W);
+  ++launches_;
+}
+
+cudaError_t Engine::list_partwet(const double* W) {
+  cudaError_t e = cudaMemsetAsync(work_.pwcount, 0, sizeof(int), stream_);
+  k_list_partwet<<<nblocks(mesh_.C, 256), 256, 0, stream_>>>(mesh_, work_, W);
+  ++launches_;
+  return e == cudaSuccess ? cudaGetLastError() : e;
+}
+
+cudaError_t Engine::ensure_list() {
+  if (list_valid_) return cudaSuccess;
+  list_valid_ = true;
+  return list_partwet(state(0, 0));
+}
+
 void Engine::launch_recon2(const double* W, const double* U, const double* V, cudaStream_t s, bool slots) {
-  const int b = blk_[0], g = std::max(1, std::min(nblocks(mesh_.C, b), 152 * 2048 / b));
+  const int b = 128, g = listed_blocks();
   const int form = !slots ? kLean : cor0_ ? kSlotsCor0 : kSlotsCor;
   switch (form + (batched_ ? 3 : 0)) {
     case 0: k_recon2<false, kLean><<<g, b, 0, s>>>(mesh_, work_, W, U, V); break;
@@ -1000,24 +1137,27 @@ void Engine::launch_recon2(const double* W, const double* U, const double* V, cu
 }
 
 cudaError_t Engine::interface_values(const double* W, const double* U, const double* V) {
-  launch_recon1(W, U, V, 0, true);
+  launch_recon1(W, U, V, 0, true, true);
+  launch_partwet1(W, stream_);
   launch_recon2(W, U, V, stream_, true);
   k_node_max_all<<<nblocks(std::max(mesh_.N, 1), 256), 256, 0, stream_>>>(mesh_, work_, W);
   ++launches_;
   slots_stale_ = false;
+  list_valid_ = W == state(0, 0);
   return cudaGetLastError();
 }
 
 cudaError_t Engine::refresh_slots() {
   if (!slots_stale_) return cudaSuccess;
-  // the last stage read buffer 1; its list is made again and emptied again, and
-  // the CFL ratio of its flux pass stays
-  launch_recon1(state(1, 0), state(1, 1), state(1, 2), 3, true);
+  // the last stage read buffer 1; the CFL ratio of its flux pass stays
+  cudaError_t e = cudaMemsetAsync(work_.pwcount, 0, sizeof(int), stream_);
+  if (e != cudaSuccess) return e;
+  launch_recon1(state(1, 0), state(1, 1), state(1, 2), 3, true, true);
+  launch_partwet1(state(1, 0), stream_);
   launch_recon2(state(1, 0), state(1, 1), state(1, 2), stream_, true);
   slots_stale_ = false;
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaMemsetAsync(work_.pwcount, 0, sizeof(int), stream_);
-  return e;
+  list_valid_ = false;  // it is that buffer's now
+  return cudaGetLastError();
 }
 
 // The plugin of (flux, wave speed), given to f as a type.
@@ -1087,11 +1227,13 @@ cudaError_t Engine::launch_stage(const Stage& st, const double* const* in, const
   // a stage that overwrites its own input leaves the full interface values now
   // (refresh_slots could not make them later)
   const bool slots = in[0] == out[0];
-  if (ev) cudaEventRecord(ev[0], stream_);
-  launch_recon1(in[0], in[1], in[2], lm, slots);
+  // (the input's partially-wet cells are listed: by the update before, or ensure_list)
   if (ev) {
     // per-kernel timing: the kernels one after another
+    cudaEventRecord(ev[0], stream_);
+    launch_recon1(in[0], in[1], in[2], lm, slots, false);
     cudaEventRecord(ev[1], stream_);
+    launch_partwet1(in[0], stream_);
     launch_recon2(in[0], in[1], in[2], stream_, slots);
     cudaEventRecord(ev[2], stream_);
     stage_fluxes_pw(in, stream_);
@@ -1099,10 +1241,14 @@ cudaError_t Engine::launch_stage(const Stage& st, const double* const* in, const
     if (e != cudaSuccess) return e;
     cudaEventRecord(ev[3], stream_);
   } else {
-    // PartWet2 and the fluxes next to partially-wet cells on the side stream,
-    // beside the other edges' fluxes
+    // on the side stream: PartWet1 beside pass 1, then PartWet2 and the fluxes
+    // next to partially-wet cells beside the other edges' fluxes
     cudaEventRecord(ev_fork_, stream_);
     cudaStreamWaitEvent(side_, ev_fork_, 0);
+    launch_partwet1(in[0], side_);
+    launch_recon1(in[0], in[1], in[2], lm, slots, false);
+    cudaEventRecord(ev_pass1_, stream_);
+    cudaStreamWaitEvent(side_, ev_pass1_, 0);
     launch_recon2(in[0], in[1], in[2], side_, slots);
     stage_fluxes_pw(in, side_);
     cudaEventRecord(ev_join_, side_);
@@ -1159,7 +1305,7 @@ cudaError_t Engine::step_timed(int scheme, int latch_mode, double* acc) {
   cudaEvent_t ev[kMaxStages][6];
   for (auto& row : ev)
     for (auto& x : row) cudaEventCreate(&x);
-  cudaError_t e = cudaSuccess;
+  cudaError_t e = ensure_list();
   for (int s = 0; s < sc.n && e == cudaSuccess; ++s) {
     const bool last = (s == sc.n - 1);
     const double* const* in = (s == 0) ? S0 : S1;
@@ -1218,6 +1364,7 @@ cudaError_t Engine::snapshot(double* buf, bool restore) {
     r = restore ? cudaMemcpyAsync(state(0, c), buf + c * C, C * sizeof(double), cudaMemcpyDeviceToDevice, stream_)
                 : cudaMemcpyAsync(buf + c * C, state(0, c), C * sizeof(double), cudaMemcpyDeviceToDevice, stream_);
   if (restore) {
+    state_changed();
     if (r == cudaSuccess) r = cudaMemsetAsync(work_.tsum, 0, mesh_.I * sizeof(double), stream_);
     if (r == cudaSuccess) r = cudaMemsetAsync(work_.dt, 0, mesh_.I * sizeof(double), stream_);
     if (r == cudaSuccess) r = cudaMemsetAsync(work_.err, 0, sizeof(unsigned), stream_);
@@ -1345,6 +1492,7 @@ std::string Engine::set_bathymetry(const std::vector<const double*>& z) {
     const Layout* L = q < layouts.size() ? &layouts[q] : nullptr;
     for (int64_t p = 0; p < h.N; ++p) h.geom[3 * p + 2] = z[q][(L && !L->identity()) ? L->node_from[p] : p];
   }
+  state_changed();
   const std::vector<double> nz = host_nz();
   cudaError_t e = compute_bed(nz.data());
   // the adjoint's tape and plane tables belong to the old bed
@@ -1384,6 +1532,8 @@ cudaError_t Engine::step(int scheme, int latch_mode) {
 
 cudaError_t Engine::run_graph(int scheme, int latch_mode, int64_t n) {
   if (n <= 0) return cudaSuccess;
+  const cudaError_t el = ensure_list();
+  if (el != cudaSuccess) return el;
   cudaGraphExec_t& ge = graphs_[scheme][latch_mode];
   const int64_t per_step = launches_;
   if (!ge) {
@@ -1414,7 +1564,7 @@ cudaError_t Engine::run_graph(int scheme, int latch_mode, int64_t n) {
     }
     launches_ = per_step;  // capture launched nothing
   }
-  const int64_t kernels_per_step = 6 * scheme_of(scheme).n;
+  const int64_t kernels_per_step = 7 * scheme_of(scheme).n;
   slots_stale_ = scheme_of(scheme).n > 1;
   for (int64_t s = 0; s < n; ++s) {
     cudaError_t e = cudaGraphLaunch(ge, stream_);

@@ -274,73 +274,129 @@ SWE_HD double midpoint(double xmin, double xmax) {
   return SWE_HALF(xmin + xmax);
 }
 
+// Where the computed sign of f must be looked at: outside [lo, hi] it is that of
+// the nearer end.
+struct Bracket {
+  double lo, hi;
+};
+
+// Lower and upper bounds lo <= root <= hi as above for x^3 + c x + d on [0, 1]
+// (convex) with the ends' computed values fmin and fmax of opposite signs.
+// two: how the two points' computed values are had (a lane group evaluates them
+// together, with collectives: no path around the call).
+template <class Two>
+SWE_HD Bracket bracket01(double d, double c, double fmin_, double fmax_, Two&& two) {
+  const bool neg_min = negative(fmin_);
+  Bracket r{0., 1.};
+  // |computed f - f| <= u (5 x^3 + 3 |c| x + |d|), held a little larger
+  const double E = 6e-16 + 3.6e-16 * magnitude(c) + 1.3e-16 * magnitude(d);
+  const float g = quick_div(1.0f, fmaxf(fabsf((float)fmin_), fabsf((float)fmax_)));
+  double x = (double)unit_root(g, 0.f, (float)c * g, (float)fmin_ * g, neg_min);
+  double slope = 0.;
+  for (int q = 0; q < 2; ++q) {
+    const double y = fma(x, x, c);
+    slope = fma(2. * x, x, y);
+    x -= (double)quick_div((float)fma(y, x, d), (float)slope);
+  }
+  const double gap = (double)quick_div((float)(2.6 * E), fabsf((float)slope)) + 4.5e-16;
+  const double l = x - gap, h = x + gap, E2 = 2. * E;
+  double fl, fh;
+  two(l, h, &fl, &fh);
+  const bool at0 = !dlt(0., l), at1 = !dlt(h, 1.);
+  const bool ok = (at0 || (negative(fl) == neg_min && above(magnitude(fl), E2) && above(magnitude(fmin_), E2))) &&
+                  (at1 || (negative(fh) != neg_min && above(magnitude(fh), E2) && above(magnitude(fmax_), E2))) &&
+                  dlt(l, 1.) && dlt(0., h) && above(1e280, E) && x == x;
+  if (ok && !at0) r.lo = l;
+  if (ok && !at1) r.hi = h;
+  return r;
+}
+
+// The bisection of [0, 1] has dyadic midpoints, so its steps down to the last
+// interval that holds [r.lo, r.hi] are taken at once: their number (at most
+// most), and that interval.
+SWE_HD int dyadic_steps(const Bracket& r, int most, double* xmin, double* xmax) {
+  // floor(lo 2^62) and ceil(hi 2^62) - 1: their common leading bits are steps
+  const unsigned long long ul = ubits(r.lo), uh = ubits(r.hi);
+  const int sl = 1013 - (int)(ul >> 52), sh = 1013 - (int)(uh >> 52);
+  const unsigned long long hid = 1ull << 52, ml = (ul & (hid - 1)) | hid, mh = (uh & (hid - 1)) | hid;
+  unsigned long long fl = 0ull, fh = (1ull << 62) - 1ull;
+  if (ul != 0ull) fl = sl <= 0 ? ml << -sl : sl < 64 ? ml >> sl : 0ull;
+  if (uh != ubits(1.)) fh = sh <= 0 ? (mh << -sh) - 1ull : sh < 53 ? (mh - 1ull) >> sh : 0ull;
+  const unsigned long long diff = fl ^ fh;
+  int k = 0;
+  for (int w = 32; w > 0; w >>= 1)
+    if (k + w <= 62 && (diff >> (62 - k - w)) == 0ull) k += w;
+  if (k > most) k = most;
+  const unsigned long long j = fl >> (62 - k);
+  const double scale = ufrom((unsigned long long)(1023 - k) << 52);  // 2^-k
+  *xmin = (double)j * scale;
+  *xmax = (double)(j + 1ull) * scale;
+  return k;
+}
+
+// The bracket for x^3 + b x^2 + c x + d on [xmin, xmax], of width w.
+template <class Two>
+SWE_HD Bracket bracket(double d, double c, double b, double xmin, double xmax, double w, double fmin_, double fmax_,
+                       Two&& two) {
+  const bool neg_min = negative(fmin_);
+  Bracket r{xmin, xmax};
+  // f'' / 2 at the ends, rounded twice (PartWet1's is -3 b13 + 3 b13 at the upper
+  // one: a last bit of b there bends f by less than E)
+  const double c0 = 3. * xmin + b, c1 = 3. * xmax + b;
+  const bool curved = (dle(0., c0) && dle(0., c1)) || (dle(c0, 0.) && dle(c1, 0.));
+  // f(xmin + w s) / |f| in single precision, s in [0, 1]
+  const float fw = (float)w, fc0 = (float)c0;
+  const float g = quick_div(1.0f, fmaxf(fabsf((float)fmin_), fabsf((float)fmax_)));
+  const double s0 = fma(xmin, c0 + b, c);  // f'(xmin)
+  const float p1 = (float)s0 * fw * g, p2 = fc0 * fw * fw * g, p3 = fw * fw * fw * g;
+  double x = fma(w, (double)unit_root(p3, p2, p1, (float)fmin_ * g, neg_min), xmin);
+  double slope = 0.;
+  for (int q = 0; q < 2; ++q) {
+    const double y = x + b, z = fma(x, y, c);
+    slope = fma(x, y + x, z);
+    x -= (double)quick_div((float)fma(z, x, d), (float)slope);
+  }
+  // |computed f - f| <= u (5 |x|^3 + 5 |b| x^2 + 3 |c| |x| + |d|), a little larger
+  const double m = smax(magnitude(xmin), magnitude(xmax));
+  const double E = fma(6e-16, fma(m + magnitude(b), m, magnitude(c)) * m, 1.3e-16 * magnitude(d));
+  const double gap = fma(4.5e-16, m, (double)quick_div((float)(2.6 * E), fabsf((float)slope)));
+  const double l = x - gap, h = x + gap, E2 = 2. * E;
+  double fl, fh;
+  two(l, h, &fl, &fh);
+  const bool at0 = !dlt(xmin, l), at1 = !dlt(h, xmax);
+  const bool ok = (at0 || (negative(fl) == neg_min && above(magnitude(fl), E2) && above(magnitude(fmin_), E2))) &&
+                  (at1 || (negative(fh) != neg_min && above(magnitude(fh), E2) && above(magnitude(fmax_), E2))) &&
+                  dlt(l, xmax) && dlt(xmin, h) && above(E, 1e-280) && above(1e280, E) && x == x && curved;
+  if (ok && !at0) r.lo = l;
+  if (ok && !at1) r.hi = h;
+  return r;
+}
+
 // x^3 + c x + d on [0, 1] (PartWet2).  The quadratic term is 0 x x, whose
-// addition changes no bit of x^3 >= 0; f(0) is 0 + d and f(1) (1 + c) + d.  The
-// midpoints are dyadic, so the steps down to the last interval that holds
-// [lo, hi] are taken at once.  A lone call on GB300: 34000 -> 11200 cycles.
+// addition changes no bit of x^3 >= 0; f(0) is 0 + d and f(1) (1 + c) + d.
+SWE_HD double cubic01(double d, double c, double x) { return x * x * x + c * x + d; }
 SWE_HD double bisection01(double d, double c) {
   const double fmin_ = 0. + d, fmax_ = (1. + c) + d;
   const bool neg_min = negative(fmin_);
   if (neg_min == negative(fmax_)) return dlt(magnitude(fmin_), magnitude(fmax_)) ? 0. : 1.;
-  constexpr int n = 50;
-  double xmin = 0., xmax = 1.;
-  double lo = 0., hi = 1.;
-  int it = 0;
-  // convex; |computed f - f| <= u (5 x^3 + 3 |c| x + |d|), held a little larger
-  const double E = 6e-16 + 3.6e-16 * magnitude(c) + 1.3e-16 * magnitude(d);
-  {
-    const float g = quick_div(1.0f, fmaxf(fabsf((float)fmin_), fabsf((float)fmax_)));
-    double x = (double)unit_root(g, 0.f, (float)c * g, (float)fmin_ * g, neg_min);
-    double slope = 0.;
-    for (int q = 0; q < 2; ++q) {
-      const double xx = x * x;
-      slope = 3. * xx + c;
-      x -= (double)quick_div((float)((xx + c) * x + d), (float)slope);
-    }
-    const double gap = (double)quick_div((float)(2.6 * E), fabsf((float)slope)) + 4.5e-16;
-    const double l = x - gap, h = x + gap, E2 = 2. * E;
-    const double fl = l * l * l + c * l + d, fh = h * h * h + c * h + d;
-    const bool at0 = !dlt(0., l), at1 = !dlt(h, 1.);
-    const bool ok = (at0 || (negative(fl) == neg_min && above(magnitude(fl), E2) && above(magnitude(fmin_), E2))) &&
-                    (at1 || (negative(fh) != neg_min && above(magnitude(fh), E2) && above(magnitude(fmax_), E2))) &&
-                    dlt(l, 1.) && dlt(0., h) && above(1e280, E) && x == x;
-    if (ok && !at0) lo = l;
-    if (ok && !at1) hi = h;
-    if (ok) {
-      // floor(lo 2^62) and ceil(hi 2^62) - 1: their common leading bits are steps
-      const unsigned long long ul = ubits(lo), uh = ubits(hi);
-      const int sl = 1013 - (int)(ul >> 52), sh = 1013 - (int)(uh >> 52);
-      const unsigned long long hid = 1ull << 52, ml = (ul & (hid - 1)) | hid, mh = (uh & (hid - 1)) | hid;
-      unsigned long long fl62 = 0ull, fh62 = (1ull << 62) - 1ull;
-      if (!at0) fl62 = sl <= 0 ? ml << -sl : sl < 64 ? ml >> sl : 0ull;
-      if (!at1) fh62 = sh <= 0 ? (mh << -sh) - 1ull : sh < 53 ? (mh - 1ull) >> sh : 0ull;
-      unsigned long long diff = fl62 ^ fh62;
-      int k = 0;
-      for (int w = 32; w > 0; w >>= 1)
-        if (k + w <= 62 && (diff >> (62 - k - w)) == 0ull) k += w;
-      if (k > n) k = n;
-      const unsigned long long j = fl62 >> (62 - k);
-      const double scale = ufrom((unsigned long long)(1023 - k) << 52);  // 2^-k
-      xmin = (double)j * scale;
-      xmax = (double)(j + 1ull) * scale;
-      it = k;
-    }
-  }
-  double x = 0.;
-  for (; it <= n; it++) {
+  const Bracket r = bracket01(d, c, fmin_, fmax_, [&](double l, double h, double* fl, double* fh) {
+    *fl = cubic01(d, c, l);
+    *fh = cubic01(d, c, h);
+  });
+  double xmin, xmax, x = 0.;
+  for (int it = dyadic_steps(r, 50, &xmin, &xmax); it <= 50; it++) {
     x = midpoint(xmin, xmax);
     bool left;
-    if (dle(x, lo)) left = true;
-    else if (dle(hi, x)) left = false;
-    else left = negative(x * x * x + c * x + d) == neg_min;
+    if (dle(x, r.lo)) left = true;
+    else if (dle(r.hi, x)) left = false;
+    else left = negative(cubic01(d, c, x)) == neg_min;
     if (left) xmin = x;
     else xmax = x;
   }
   return x;
 }
 
-// The general form.  34000 -> 22700 cycles a call for nearly flat cells on a
-// high bed, where rounding hides the sign longest (20 evaluations).
+// The general form.
 SWE_HD double bisection(double d, double c, double b, double xmin, double xmax) {
   if ((ubits(b) | ubits(xmin)) == 0ull && ubits(xmax) == ubits(1.)) return bisection01(d, c);
   const double fmin_ = cubic(d, c, b, xmin);
@@ -349,46 +405,115 @@ SWE_HD double bisection(double d, double c, double b, double xmin, double xmax) 
   if (neg_min == negative(fmax_)) return dlt(magnitude(fmin_), magnitude(fmax_)) ? xmin : xmax;
   const double w = xmax - xmin;
   const int n = 50 + trunc_log2(w);
-  double lo = xmin, hi = xmax;
-  const double c0 = 3. * xmin + b, c1 = 3. * xmax + b;  // f'' / 2 at the ends
-  if (n > 8 && ((dle(0., c0) && dle(0., c1)) || (dle(c0, 0.) && dle(c1, 0.)))) {
-    // f(xmin + w s) / |f| in single precision, s in [0, 1]
-    const float fw = (float)w, fc0 = (float)c0;
-    const float g = quick_div(1.0f, fmaxf(fabsf((float)fmin_), fabsf((float)fmax_)));
-    const double s0 = xmin * (c0 + b) + c;  // f'(xmin)
-    const float p1 = (float)s0 * fw * g, p2 = fc0 * fw * fw * g, p3 = fw * fw * fw * g;
-    double x = xmin + w * (double)unit_root(p3, p2, p1, (float)fmin_ * g, neg_min);
-    double slope = 0.;
-    for (int q = 0; q < 2; ++q) {
-      const double y = x + b;
-      slope = x * (2. * y + x) + c;
-      x -= (double)quick_div((float)((x * y + c) * x + d), (float)slope);
-    }
-    // |computed f - f| <= u (5 |x|^3 + 5 |b| x^2 + 3 |c| |x| + |d|), a little larger
-    const double m = smax(magnitude(xmin), magnitude(xmax));
-    const double E = 6e-16 * (((m + magnitude(b)) * m + magnitude(c)) * m) + 1.3e-16 * magnitude(d);
-    const double gap = (double)quick_div((float)(2.6 * E), fabsf((float)slope)) + 4.5e-16 * m;
-    const double l = x - gap, h = x + gap, E2 = 2. * E;
-    const double fl = cubic(d, c, b, l), fh = cubic(d, c, b, h);
-    const bool at0 = !dlt(xmin, l), at1 = !dlt(h, xmax);
-    const bool ok = (at0 || (negative(fl) == neg_min && above(magnitude(fl), E2) && above(magnitude(fmin_), E2))) &&
-                    (at1 || (negative(fh) != neg_min && above(magnitude(fh), E2) && above(magnitude(fmax_), E2))) &&
-                    dlt(l, xmax) && dlt(xmin, h) && above(E, 1e-280) && above(1e280, E) && x == x;
-    if (ok && !at0) lo = l;
-    if (ok && !at1) hi = h;
-  }
+  Bracket r{xmin, xmax};
+  if (n > 8)
+    r = bracket(d, c, b, xmin, xmax, w, fmin_, fmax_, [&](double l, double h, double* fl, double* fh) {
+      *fl = cubic(d, c, b, l);
+      *fh = cubic(d, c, b, h);
+    });
   double x = 0.;
   for (int it = 0; it <= n; it++) {
     x = midpoint(xmin, xmax);
     bool left;
-    if (dle(x, lo)) left = true;
-    else if (dle(hi, x)) left = false;
+    if (dle(x, r.lo)) left = true;
+    else if (dle(r.hi, x)) left = false;
     else left = negative(cubic(d, c, b, x)) == neg_min;
     if (left) xmin = x;
     else xmax = x;
   }
   return x;
 }
+
+#if defined(__CUDACC__)
+// The same by groups of 8 lanes, four bisections a warp.  Every lane of the warp
+// calls together, the lanes of a group with the same operands, and the groups
+// that have none with active = false.  The steps that the bracket decides are
+// taken by comparison; then lane q > 0 of a group takes node q of the tree of
+// the next seven midpoints, so that a round settles three steps for one
+// evaluation.  All collectives are over the warp: with groups that run apart the
+// FP64 pipe would issue each group's operations by themselves (64 cycles each).
+template <bool UNIT>
+__device__ double bisection_group(double d, double c, double b, double xmin, double xmax, bool active) {
+  constexpr unsigned kWarp = 0xFFFFFFFFu;
+  const int q = threadIdx.x & 7;
+  auto f = [&](double x) { return UNIT ? cubic01(d, c, x) : cubic(d, c, b, x); };
+  // the computed values at two points, one in the even lanes and one in the odd
+  auto two = [&](double l, double h, double* fl, double* fh) {
+    const double v = f((q & 1) ? h : l);
+    *fl = __shfl_sync(kWarp, v, 0, 8);
+    *fh = __shfl_sync(kWarp, v, 1, 8);
+  };
+  double fmin_, fmax_;
+  if (UNIT) {
+    fmin_ = 0. + d;
+    fmax_ = (1. + c) + d;
+  } else {
+    two(xmin, xmax, &fmin_, &fmax_);
+  }
+  const bool neg_min = negative(fmin_);
+  const bool same = neg_min == negative(fmax_);
+  double x = same ? (dlt(magnitude(fmin_), magnitude(fmax_)) ? xmin : xmax) : 0.;
+  int n = 50, it = 0;
+  Bracket r;
+  if (UNIT) {
+    r = bracket01(d, c, fmin_, fmax_, two);
+    it = dyadic_steps(r, n, &xmin, &xmax);
+  } else {
+    const double w = xmax - xmin;
+    n = 50 + trunc_log2(w);
+    const Bracket found = bracket(d, c, b, xmin, xmax, w, fmin_, fmax_, two);
+    r = n > 8 ? found : Bracket{xmin, xmax};
+  }
+  if (same || !active) n = -1;
+  // steps that the bracket decides
+  auto key = [](double y) {  // ordered as the doubles are
+    const long long u = (long long)ubits(y);
+    return u < 0 ? -(u & 0x7FFFFFFFFFFFFFFFll) : u;
+  };
+  const long long klo = key(r.lo), khi = key(r.hi);
+  bool plain = it <= n;
+  while (__any_sync(kWarp, plain)) {
+    if (plain) {
+      const double mid = midpoint(xmin, xmax);
+      const long long k = key(mid);
+      if (k <= klo) xmin = x = mid;
+      else if (khi <= k) xmax = x = mid;
+      else plain = false;
+      if (plain) plain = ++it <= n;
+    }
+  }
+  const int node = q > 0 ? q : 1, depth = node > 3 ? 2 : node > 1 ? 1 : 0;
+  while (__any_sync(kWarp, it <= n)) {
+    // this lane's midpoint: down from the root by its node number's bits
+    double a = xmin, z = xmax, mid = midpoint(a, z);
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+      if (t < depth) {
+        if ((node >> (depth - 1 - t)) & 1) a = mid;
+        else z = mid;
+        mid = midpoint(a, z);
+      }
+    const long long k = key(mid);
+    const bool neg = negative(f(mid));
+    const bool right = k <= klo || (k < khi && neg == neg_min);  // the path goes on right of mid
+    const unsigned went = __ballot_sync(kWarp, right) >> (threadIdx.x & 24);
+    const int levels = min(3, n - it + 1);
+    int at = 1;
+    if (levels > 1) at = 2 * at + ((went >> at) & 1u);
+    if (levels > 2) at = 2 * at + ((went >> at) & 1u);
+    const double xn = __shfl_sync(kWarp, mid, at, 8);
+    const double an = __shfl_sync(kWarp, right ? mid : a, at, 8);
+    const double zn = __shfl_sync(kWarp, right ? z : mid, at, 8);
+    if (it <= n) {
+      x = xn;
+      xmin = an;
+      xmax = zn;
+      it += levels;
+    }
+  }
+  return x;
+}
+#endif
 
 // --------------------------------------------------------------- assigners
 // src/Assigners.cpp:8-20: PrimAssigner (edge writes)
