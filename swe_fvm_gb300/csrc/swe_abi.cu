@@ -88,6 +88,41 @@ __global__ void k_unpack(const double* __restrict__ in, double* __restrict__ W, 
   }
 }
 
+// The getters' arrays in the reference's layout and the caller's numbering, so
+// that each is one copy to the host (host loops over five arrays of 3 C values
+// took 0.5 ms of the 0.77 ms in which a program reads all fields of 18,000 cells).
+// Row 2 e + (c < n) of edge e holds the value of its cell c towards cell n
+// (EdgeIndexer::Id, include/ValueField.h:70-75); a null component is zero.
+__global__ void k_edge_rows(swe::DevMesh m, const double* a, const double* b, const double* c,
+                            const int* __restrict__ edge_caller, const int* __restrict__ cell_caller,
+                            double* __restrict__ out) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= 3 * m.C) return;
+  const int i = s % m.C, nb = m.cnbr[s];
+  const long long row =
+      2ll * edge_caller[m.cedge[s]] + (cell_caller[i] < (nb < 0 ? nb : cell_caller[nb]) ? 1 : 0);
+  out[3 * row] = a ? a[s] : 0.;
+  out[3 * row + 1] = b[s];
+  out[3 * row + 2] = c[s];
+}
+__global__ void k_flux_rows(const double* a, const double* b, const double* c, int n,
+                            const int* __restrict__ edge_caller, double* __restrict__ out) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= n) return;
+  const long long r = 3ll * edge_caller[e];
+  out[r] = a[e];
+  out[r + 1] = b[e];
+  out[r + 2] = c[e];
+}
+__global__ void k_node_rows(const unsigned long long* key, int n, const int* __restrict__ node_caller,
+                            double* __restrict__ out) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q < n) out[node_caller[q]] = swe::order_val(key[q]);
+}
+// a scalar from the launch's own arguments (an 8-byte copy from pageable memory
+// goes through the copy engine)
+__global__ void k_set_value(double* p, double v) { *p = v; }
+
 swe_status read_instance(const swe_mesh* m, const swe_params* p, HostInstance* h, std::string* why) {
   if (!m || !m->geometry || !m->edge_nodes || !m->edge_cells || !m->cell_nodes || !m->cell_edges ||
       !m->cell_neighbours) {
@@ -240,11 +275,10 @@ swe_status upload_prim(Engine& eng, const double* prim, int64_t c0, int64_t n, s
                                                                 eng.d_cell_from ? eng.d_cell_from + c0 : nullptr);
     e = cudaGetLastError();
   }
-  unsigned h = 0;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&h, flag, sizeof(unsigned), cudaMemcpyDeviceToHost, eng.stream());
+  if (e == cudaSuccess) e = cudaMemcpyAsync(eng.h_word, flag, sizeof(unsigned), cudaMemcpyDeviceToHost, eng.stream());
   if (e == cudaSuccess) e = cudaStreamSynchronize(eng.stream());
   if (e != cudaSuccess) return cuda_fail(err, e, "uploading the state");
-  if (h) return fail(err, SWE_ERR_NONFINITE, "state has a non-finite value");
+  if ((unsigned)*eng.h_word) return fail(err, SWE_ERR_NONFINITE, "state has a non-finite value");
   return SWE_OK;
 }
 
@@ -493,7 +527,8 @@ swe_status swe_step(swe_ctx* ctx, int32_t scheme, double dt) {
   SWE_GUARD_BEGIN
   if (!ctx->eng.has_scheme(scheme)) return fail(&ctx->err, SWE_ERR_INVALID_ARGUMENT, kSchemeMsg);
   if (!(dt > 0.) || !std::isfinite(dt)) return fail(&ctx->err, SWE_ERR_INVALID_ARGUMENT, "dt must be positive and finite");
-  cudaError_t e = cudaMemcpyAsync(ctx->eng.d_fixed_dt, &dt, sizeof(double), cudaMemcpyHostToDevice, ctx->eng.stream());
+  k_set_value<<<1, 1, 0, ctx->eng.stream()>>>(ctx->eng.d_fixed_dt, dt);
+  cudaError_t e = cudaGetLastError();
   // one replay of the step's CUDA graph (captured on first use)
   if (e == cudaSuccess) e = ctx->eng.run_graph(scheme, 2, 1);
   if (e != cudaSuccess) return cuda_fail(&ctx->err, e, "swe_step");
@@ -508,7 +543,8 @@ swe_status swe_run(swe_ctx* ctx, int32_t scheme, double dt, int64_t n_steps) {
   if (!ctx->eng.has_scheme(scheme)) return fail(&ctx->err, SWE_ERR_INVALID_ARGUMENT, kSchemeMsg);
   if (!(dt > 0.) || !std::isfinite(dt)) return fail(&ctx->err, SWE_ERR_INVALID_ARGUMENT, "dt must be positive and finite");
   if (n_steps < 0) return fail(&ctx->err, SWE_ERR_INVALID_ARGUMENT, "n_steps must be >= 0");
-  cudaError_t e = cudaMemcpyAsync(ctx->eng.d_fixed_dt, &dt, sizeof(double), cudaMemcpyHostToDevice, ctx->eng.stream());
+  k_set_value<<<1, 1, 0, ctx->eng.stream()>>>(ctx->eng.d_fixed_dt, dt);
+  cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = ctx->eng.run_graph(scheme, 2, n_steps);
   if (e != cudaSuccess) return cuda_fail(&ctx->err, e, "swe_run");
   return SWE_OK;
@@ -534,11 +570,12 @@ swe_status swe_run_cfl(swe_ctx* ctx, int32_t scheme, int64_t n_steps, double* t_
 
 swe_status swe_min_len_to_wavespeed(swe_ctx* ctx, double* r) {
   if (!ctx || !r) return SWE_ERR_INVALID_ARGUMENT;
-  unsigned long long k = 0;
-  cudaError_t e = cudaMemcpyAsync(&k, ctx->eng.work().r, sizeof(k), cudaMemcpyDeviceToHost, ctx->eng.stream());
+  // through pinned memory: a small copy to pageable memory takes longer than the wait
+  cudaError_t e = cudaMemcpyAsync(ctx->eng.h_word, ctx->eng.work().r, sizeof(unsigned long long),
+                                  cudaMemcpyDeviceToHost, ctx->eng.stream());
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->eng.stream());
   if (e != cudaSuccess) return cuda_fail(&ctx->err, e, "swe_min_len_to_wavespeed");
-  *r = swe::order_val(k);
+  *r = swe::order_val(*ctx->eng.h_word);
   return SWE_OK;
 }
 
@@ -622,42 +659,24 @@ swe_status swe_get_edge_values(swe_ctx* ctx, double* edg_out, double* src_out) {
   if (!ctx) return SWE_ERR_INVALID_ARGUMENT;
   SWE_GUARD_BEGIN
   Engine& g = ctx->eng;
-  const int64_t C = g.C(), E = g.E();
-  std::vector<double> ew(3 * C), eu(3 * C), ev(3 * C), sx(3 * C), sy(3 * C);
   const swe::DevWork& w = g.work();
+  const int n = 3 * g.C();
   cudaError_t e = g.refresh_slots();
+  std::string why = e == cudaSuccess ? g.field_rows() : std::string();
+  if (!why.empty()) return fail(&ctx->err, SWE_ERR_CUDA, why);
+  auto rows = [&](const double* a, const double* b, const double* c, double* out) {
+    const size_t bytes = 6 * (size_t)g.E() * sizeof(double);
+    if (e == cudaSuccess) e = cudaMemsetAsync(g.d_rows, 0, bytes, g.stream());
+    if (e != cudaSuccess) return;
+    k_edge_rows<<<(n + 255) / 256, 256, 0, g.stream()>>>(g.mesh(), a, b, c, g.d_edge_caller, g.d_cell_caller,
+                                                         g.d_rows);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(out, g.d_rows, bytes, cudaMemcpyDeviceToHost, g.stream());
+  };
+  if (edg_out) rows(w.ew, w.eu, w.ev, edg_out);
+  if (src_out) rows(nullptr, w.sx, w.sy, src_out);
   if (e == cudaSuccess) e = cudaStreamSynchronize(g.stream());
-  if (e == cudaSuccess) e = cudaMemcpy(ew.data(), w.ew, 3 * C * sizeof(double), cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess) e = cudaMemcpy(eu.data(), w.eu, 3 * C * sizeof(double), cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess) e = cudaMemcpy(ev.data(), w.ev, 3 * C * sizeof(double), cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess) e = cudaMemcpy(sx.data(), w.sx, 3 * C * sizeof(double), cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess) e = cudaMemcpy(sy.data(), w.sy, 3 * C * sizeof(double), cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return cuda_fail(&ctx->err, e, "swe_get_edge_values");
-  const HostInstance& h = g.host[0];
-  const swe::Layout& L = g.layouts[0];
-  if (edg_out) std::memset(edg_out, 0, 6 * E * sizeof(double));
-  if (src_out) std::memset(src_out, 0, 6 * E * sizeof(double));
-  for (int64_t i = 0; i < C; ++i)
-    for (int k = 0; k < 3; ++k) {
-      // the slot's edge, cell and neighbour in the caller's numbering
-      int64_t ed = h.ce[3 * i + k], nb = h.ct[3 * i + k], ci = i;
-      if (!L.identity()) {
-        ed = L.edge_from[ed];
-        nb = nb >= 0 ? L.cell_from[nb] : nb;
-        ci = L.cell_from[i];
-      }
-      const int64_t id = 2 * ed + (ci < nb ? 1 : 0);  // EdgeIndexer::Id (include/ValueField.h:70-75)
-      const int64_t s = k * C + i;
-      if (edg_out) {
-        edg_out[3 * id] = ew[s];
-        edg_out[3 * id + 1] = eu[s];
-        edg_out[3 * id + 2] = ev[s];
-      }
-      if (src_out) {
-        src_out[3 * id + 1] = sx[s];
-        src_out[3 * id + 2] = sy[s];
-      }
-    }
   return SWE_OK;
   SWE_GUARD_END(&ctx->err)
 }
@@ -666,20 +685,16 @@ swe_status swe_get_fluxes(swe_ctx* ctx, double* f_out) {
   if (!ctx || !f_out) return SWE_ERR_INVALID_ARGUMENT;
   SWE_GUARD_BEGIN
   Engine& g = ctx->eng;
-  const int64_t E = g.E();
-  std::vector<double> a(E), b(E), c(E);
-  cudaError_t e = cudaStreamSynchronize(g.stream());
-  if (e == cudaSuccess) e = cudaMemcpy(a.data(), g.work().f0, E * sizeof(double), cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess) e = cudaMemcpy(b.data(), g.work().f1, E * sizeof(double), cudaMemcpyDeviceToHost);
-  if (e == cudaSuccess) e = cudaMemcpy(c.data(), g.work().f2, E * sizeof(double), cudaMemcpyDeviceToHost);
+  const std::string why = g.field_rows();
+  if (!why.empty()) return fail(&ctx->err, SWE_ERR_CUDA, why);
+  const int n = g.E();
+  k_flux_rows<<<(n + 255) / 256, 256, 0, g.stream()>>>(g.work().f0, g.work().f1, g.work().f2, n, g.d_edge_caller,
+                                                       g.d_rows);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(f_out, g.d_rows, 3 * (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, g.stream());
+  if (e == cudaSuccess) e = cudaStreamSynchronize(g.stream());
   if (e != cudaSuccess) return cuda_fail(&ctx->err, e, "swe_get_fluxes");
-  const swe::Layout& L = g.layouts[0];
-  for (int64_t q = 0; q < E; ++q) {
-    const int64_t d = L.identity() ? q : L.edge_from[q];
-    f_out[3 * d] = a[q];
-    f_out[3 * d + 1] = b[q];
-    f_out[3 * d + 2] = c[q];
-  }
   return SWE_OK;
   SWE_GUARD_END(&ctx->err)
 }
@@ -688,14 +703,15 @@ swe_status swe_get_node_max(swe_ctx* ctx, double* max_out) {
   if (!ctx || !max_out) return SWE_ERR_INVALID_ARGUMENT;
   SWE_GUARD_BEGIN
   Engine& g = ctx->eng;
-  const int64_t N = g.N();
-  std::vector<unsigned long long> k(N);
-  cudaError_t e = cudaStreamSynchronize(g.stream());
-  if (e == cudaSuccess) e = cudaMemcpy(k.data(), g.work().maxwp, N * sizeof(k[0]), cudaMemcpyDeviceToHost);
+  const std::string why = g.field_rows();
+  if (!why.empty()) return fail(&ctx->err, SWE_ERR_CUDA, why);
+  const int n = g.N();
+  k_node_rows<<<(n + 255) / 256, 256, 0, g.stream()>>>(g.work().maxwp, n, g.d_node_caller, g.d_rows);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(max_out, g.d_rows, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, g.stream());
+  if (e == cudaSuccess) e = cudaStreamSynchronize(g.stream());
   if (e != cudaSuccess) return cuda_fail(&ctx->err, e, "swe_get_node_max");
-  std::vector<double> v(N);
-  for (int64_t q = 0; q < N; ++q) v[q] = swe::order_val(k[q]);
-  nodes_to_caller(g, v.data(), max_out);
   return SWE_OK;
   SWE_GUARD_END(&ctx->err)
 }

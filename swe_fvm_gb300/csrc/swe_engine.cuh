@@ -367,7 +367,12 @@ class Engine {
   double* d_io = nullptr;        // [3C] staging buffer for the interleaved 3 x C field
   unsigned* d_ioflag = nullptr;  // non-finite flag of the last upload
   double* d_fixed_dt = nullptr;  // [I] device dt of fixed-step runs
-  double* h_fixed_dt = nullptr;  // pinned host scalar
+  unsigned long long* h_word = nullptr;  // pinned host word for scalars read back
+  // device edge -> the caller's edge (one instance), and a staging buffer of
+  // max(6 E, N) doubles for the field getters; made by the first of them
+  int* d_edge_caller = nullptr;
+  double* d_rows = nullptr;
+  std::string field_rows();
 
  private:
   cudaError_t launch_stage(const Stage& st, const double* const* in, const double* const* u0, double* const* out,

@@ -902,7 +902,7 @@ Engine::~Engine() {
     for (auto& g : row)
       if (g) cudaGraphExecDestroy(g);
   for (void* p : allocs_) cudaFree(p);
-  if (h_fixed_dt) cudaFreeHost(h_fixed_dt);
+  if (h_word) cudaFreeHost(h_word);
   if (own_stream_) cudaStreamDestroy(own_stream_);
   if (side_) cudaStreamDestroy(side_);
   if (ev_fork_) cudaEventDestroy(ev_fork_);
@@ -1030,7 +1030,7 @@ std::string Engine::init(std::vector<HostInstance>&& inst, int flux, int ws, int
     *st = 6;
     return "device allocation failed";
   }
-  if (cudaMallocHost(&h_fixed_dt, sizeof(double)) != cudaSuccess) {
+  if (cudaMallocHost(&h_word, sizeof(*h_word)) != cudaSuccess) {
     *st = 6;
     return "pinned allocation failed";
   }
@@ -1074,6 +1074,25 @@ std::string Engine::init(std::vector<HostInstance>&& inst, int flux, int ws, int
     return std::string("CUDA error during set-up: ") + cudaGetErrorString(ce);
   }
   return "";
+}
+
+std::string Engine::field_rows() {
+  if (d_rows) return "";
+  std::string e = caller_maps();
+  if (!e.empty()) return e;
+  std::vector<int> em((size_t)mesh_.E);
+  for (size_t q = 0; q < host.size(); ++q) {
+    const Layout* L = q < layouts.size() ? &layouts[q] : nullptr;
+    const bool id = !L || L->identity();
+    for (int64_t j = 0; j < edge_off[q + 1] - edge_off[q]; ++j)
+      em[edge_off[q] + j] = (int)(edge_off[q] + (id ? j : L->edge_from[j]));
+  }
+  if (!d_edge_caller) d_edge_caller = dalloc<int>(em.size());
+  if (!d_edge_caller) return "device allocation failed";
+  if (cudaMemcpy(d_edge_caller, em.data(), em.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
+    return std::string("uploading the caller order: ") + cudaGetErrorString(cudaGetLastError());
+  d_rows = dalloc<double>(std::max(6 * (size_t)mesh_.E, (size_t)mesh_.N));
+  return d_rows ? "" : "device allocation failed";
 }
 
 cudaError_t Engine::reset_pass(bool list) {
