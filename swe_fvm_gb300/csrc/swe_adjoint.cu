@@ -58,10 +58,15 @@ __global__ void __launch_bounds__(256) k_drain_keep(DevMesh m, DevWork wk, const
   wk.drain[i] = d;
 }
 
-__global__ void k_fold_scatter(int C, double* lamp, double* lscatter) {
+// End of a stage's reverse: the adjoint of its input (with the scattered part)
+// becomes lam, and the accumulators are zero for the next one.
+__global__ void k_fold_scatter(int C, double* lamp, double* lscatter, double* lam) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < C) {
-    lamp[i] += lscatter[i];
+    lam[i] = lamp[i] + lscatter[i];
+    lam[C + i] = lamp[C + i];
+    lam[2 * C + i] = lamp[2 * C + i];
+    lamp[i] = lamp[C + i] = lamp[2 * C + i] = 0.;
     lscatter[i] = 0.;
   }
 }
@@ -875,6 +880,10 @@ struct AdjointState {
   bool taped = false;
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  // the recompute's stream, and per set of kept intermediates the events that it
+  // is filled and that the reverse is through with it
+  cudaStream_t rec = nullptr;
+  cudaEvent_t ev_rec[2] = {}, ev_rev[2] = {};
   template <class T>
   T* alloc(size_t n) {
     void* p = nullptr;
@@ -896,8 +905,9 @@ struct AdjointState {
     free_tape();
     for (void* p : allocs) cudaFree(p);
     if (side) cudaStreamDestroy(side);
-    if (ev_fork) cudaEventDestroy(ev_fork);
-    if (ev_join) cudaEventDestroy(ev_join);
+    if (rec) cudaStreamDestroy(rec);
+    for (cudaEvent_t e : {ev_fork, ev_join, ev_rec[0], ev_rec[1], ev_rev[0], ev_rev[1]})
+      if (e) cudaEventDestroy(e);
   }
 };
 
@@ -1002,7 +1012,12 @@ std::string Engine::adjoint_init() {
   }
   if (cudaStreamCreateWithFlags(&a->side, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&a->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&a->ev_join, cudaEventDisableTiming) != cudaSuccess) {
+      cudaEventCreateWithFlags(&a->ev_join, cudaEventDisableTiming) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&a->rec, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&a->ev_rec[0], cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&a->ev_rec[1], cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&a->ev_rev[0], cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&a->ev_rev[1], cudaEventDisableTiming) != cudaSuccess) {
     delete a;
     return "adjoint stream set-up failed";
   }
@@ -1167,9 +1182,24 @@ std::string Engine::adjoint_backward(const double* trace_grads_host, double* gra
   if (n_obs * a.n_gauges)
     cudaMemcpy(d_tg, trace_grads_host, n_obs * a.n_gauges * sizeof(double),
                device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice);
-  // stage-input store of one segment: [K][ns] states of 3C, plus the segment end
   const int64_t K = a.ckpt;
-  std::vector<double*> store((size_t)K * ns + 1, nullptr);
+  const int64_t nseg = (a.n_steps + K - 1) / K;
+  // per-stage forward intermediates of one segment (interface slots, fluxes,
+  // draining dt, node maxima, part-wet list) when device memory allows, and two
+  // sets of them where there is room: the recompute of the segment before then
+  // runs on a stream of its own beside a segment's reverse (both are chains of
+  // small kernels on all but the largest meshes)
+  const int64_t E = mesh_.E;
+  const size_t per_stage = ((15 * C + 10 * E + 5 * C) * sizeof(double) + N * sizeof(unsigned long long) +
+                            (C + 1) * sizeof(int) + C + 255) / 256 * 256;
+  size_t free_b = 0, total_b = 0;
+  cudaMemGetInfo(&free_b, &total_b);
+  const double one_set = ((double)per_stage + 24. * (double)C) * (double)(K * ns);
+  const bool keep = (double)per_stage * (double)(K * ns) < 0.6 * (double)free_b;
+  const int sets = keep && nseg > 1 && 2. * one_set < 0.6 * (double)free_b ? 2 : 1;
+  // stage-input store of a segment: [K][ns] states of 3C, plus the segment end
+  const size_t per_set = (size_t)K * ns + 1;
+  std::vector<double*> store(per_set * sets, nullptr);
   for (auto& p : store)
     if (cudaMalloc(&p, 3 * C * sizeof(double)) != cudaSuccess) {
       cudaFree(d_tg);
@@ -1178,26 +1208,18 @@ std::string Engine::adjoint_backward(const double* trace_grads_host, double* gra
       return "segment store allocation failed";
     }
   const int b = 256, gc = (int)((C + b - 1) / b);
-  // per-stage forward intermediates of one segment (interface slots, fluxes,
-  // draining dt, node maxima, part-wet list) when device memory allows
-  const int64_t E = mesh_.E;
-  const size_t per_stage = ((15 * C + 10 * E + 5 * C) * sizeof(double) + N * sizeof(unsigned long long) +
-                            (C + 1) * sizeof(int) + C + 255) / 256 * 256;
-  size_t free_b = 0, total_b = 0;
-  cudaMemGetInfo(&free_b, &total_b);
-  const bool keep = (double)per_stage * (double)(K * ns) < 0.6 * (double)free_b;
   std::vector<DevWork> kept;
   std::vector<double*> kept_n;  // state before ConsAssigner of each stage
   char* kept_pool = nullptr;
   if (keep) {
-    if (cudaMalloc(&kept_pool, per_stage * (size_t)(K * ns)) != cudaSuccess) {
+    if (cudaMalloc(&kept_pool, per_stage * (size_t)(sets * K * ns)) != cudaSuccess) {
       cudaFree(d_tg);
       for (auto& q : store) cudaFree(q);
       return "intermediate store allocation failed";
     }
-    kept.resize((size_t)(K * ns));
-    kept_n.resize((size_t)(K * ns));
-    for (int64_t q = 0; q < K * ns; ++q) {
+    kept.resize((size_t)(sets * K * ns));
+    kept_n.resize((size_t)(sets * K * ns));
+    for (int64_t q = 0; q < sets * K * ns; ++q) {
       char* p = kept_pool + per_stage * (size_t)q;
       DevWork wq = work_;
       auto take = [&](size_t bytes) {
@@ -1227,6 +1249,7 @@ std::string Engine::adjoint_backward(const double* trace_grads_host, double* gra
   cudaMemsetAsync(w.lam, 0, 3 * C * sizeof(double), stream_);
   cudaMemsetAsync(w.lz, 0, N * sizeof(double), stream_);
   cudaMemsetAsync(w.lscatter, 0, C * sizeof(double), stream_);
+  cudaMemsetAsync(w.lamp, 0, 3 * C * sizeof(double), stream_);
   std::vector<double> tsum_saved((size_t)I(), 0.);  // the recompute must not advance the clocks
   cudaMemcpyAsync(tsum_saved.data(), work_.tsum, I() * sizeof(double), cudaMemcpyDeviceToHost, stream_);
   cudaStreamSynchronize(stream_);
@@ -1234,18 +1257,21 @@ std::string Engine::adjoint_backward(const double* trace_grads_host, double* gra
   cudaMalloc(&lam_step, 3 * C * sizeof(double));
   cudaMemsetAsync(lam_step, 0, 3 * C * sizeof(double), stream_);
   std::string err;
-  const int64_t nseg = (a.n_steps + K - 1) / K;
   // The first step index of the current segment lives on the device, so that
   // one captured graph of a full segment's recompute and one of its reverse
   // replay for every full segment.
-  long long* d_s0 = nullptr;
-  if (cudaMalloc(&d_s0, sizeof(long long)) != cudaSuccess) err = "allocation failed";
+  long long* d_s0s = nullptr;  // one per set
+  if (cudaMalloc(&d_s0s, 2 * sizeof(long long)) != cudaSuccess) err = "allocation failed";
+  // the recompute's step dt (the reverse fetches its own into work_.dt)
+  double* d_dt_rec = nullptr;
+  if (cudaMalloc(&d_dt_rec, I() * sizeof(double)) != cudaSuccess) err = "allocation failed";
   const bool seeds = a.obs > 0 && a.n_gauges > 0;
   // recompute of steps s0 .. s0+len-1 with the recorded dt, keeping every
   // stage's forward intermediates when they fit
-  auto enqueue_recompute = [&](int64_t len) -> cudaError_t {
+  auto enqueue_recompute = [&](int64_t len, int set) -> cudaError_t {
+    const long long* d_s0 = d_s0s + set;
     for (int64_t loc = 0; loc < len; ++loc) {
-      const int64_t base = loc * ns;
+      const int64_t base = set * (int64_t)per_set + loc * ns, kb = set * K * ns + loc * ns;
       k_fetch_dt<<<(I() + 127) / 128, 128, 0, stream_>>>(d_fixed_dt, a.d_dt, d_s0, loc, I());
       double* S0p = store[base];
       const double* u0[3] = {S0p, S0p + C, S0p + 2 * C};
@@ -1257,7 +1283,8 @@ std::string Engine::adjoint_backward(const double* trace_grads_host, double* gra
         cudaError_t e;
         if (keep) {
           const DevWork saved = work_;
-          work_ = kept[base + s];
+          work_ = kept[kb + s];
+          work_.dt = d_dt_rec;
           e = reset_pass();
           if (e == cudaSuccess) {
             // the plain stage's kernels with PartWet2 and the fluxes next to
@@ -1275,7 +1302,7 @@ std::string Engine::adjoint_backward(const double* trace_grads_host, double* gra
           }
           if (e == cudaSuccess) {
             k_drain_keep<<<gc, b, 0, stream_>>>(mesh_, work_, in[0]);
-            e = update_only(sc.s[s], in, u0, out, kept_n[base + s]);
+            e = update_only(sc.s[s], in, u0, out, kept_n[kb + s]);
           }
           work_ = saved;
         } else {
@@ -1289,9 +1316,10 @@ std::string Engine::adjoint_backward(const double* trace_grads_host, double* gra
     return cudaGetLastError();
   };
   // reverse of steps s0+len-1 .. s0
-  auto enqueue_reverse = [&](int64_t len) -> cudaError_t {
+  auto enqueue_reverse = [&](int64_t len, int set) -> cudaError_t {
+    const long long* d_s0 = d_s0s + set;
     for (int64_t loc = len - 1; loc >= 0; --loc) {
-      const int64_t base = loc * ns;
+      const int64_t base = set * (int64_t)per_set + loc * ns, kb = set * K * ns + loc * ns;
       if (seeds)
         k_seed_gauges_seg<<<(a.n_gauges + 255) / 256, 256, 0, stream_>>>(lam_step, a.d_gauges, a.n_gauges, d_tg,
                                                                          d_s0, loc, a.obs);
@@ -1303,12 +1331,10 @@ std::string Engine::adjoint_backward(const double* trace_grads_host, double* gra
       for (int s = ns - 1; s >= 0; --s) {
         double* inp = store[base + s];
         const double* in[3] = {inp, inp + C, inp + 2 * C};
-        cudaMemsetAsync(w.lamp, 0, 3 * C * sizeof(double), stream_);
-        cudaError_t e = keep ? adjoint_stage_reverse_stored(sc.s[s], in, u0, w, kept[base + s], kept_n[base + s])
+        cudaError_t e = keep ? adjoint_stage_reverse_stored(sc.s[s], in, u0, w, kept[kb + s], kept_n[kb + s])
                              : adjoint_stage_reverse(sc.s[s], in, u0, w);
         if (e != cudaSuccess) return e;
-        k_fold_scatter<<<gc, b, 0, stream_>>>((int)C, w.lamp, w.lscatter);
-        cudaMemcpyAsync(w.lam, w.lamp, 3 * C * sizeof(double), cudaMemcpyDeviceToDevice, stream_);
+        k_fold_scatter<<<gc, b, 0, stream_>>>((int)C, w.lamp, w.lscatter, w.lam);
       }
       // adjoint of the step's initial state: through the first stage's input and the Shu-Osher terms
       k_add3<<<gc, b, 0, stream_>>>((int)C, w.lam, w.lam0, lam_step);
@@ -1334,29 +1360,46 @@ std::string Engine::adjoint_backward(const double* trace_grads_host, double* gra
     cudaGetLastError();
     return ge;
   };
-  cudaGraphExec_t g_rec = nullptr, g_rev = nullptr;
-  bool tried = false;
+  cudaGraphExec_t g_rec[2] = {nullptr, nullptr}, g_rev[2] = {nullptr, nullptr};
+  bool tried[2] = {false, false};
+  const cudaStream_t main = stream_, rec = sets > 1 ? a.rec : main;
+  // the recompute of segment seg into its set, after the reverse that last read
+  // that set
+  auto recompute = [&](int64_t seg) {
+    const int set = (int)(seg % sets);
+    const int64_t s0 = seg * K, len = std::min(a.n_steps, s0 + K) - s0;
+    if (sets > 1) cudaStreamWaitEvent(rec, a.ev_rev[set], 0);
+    cudaMemcpyAsync(store[per_set * set], a.checkpoints[seg], 3 * C * sizeof(double), cudaMemcpyDeviceToDevice, rec);
+    k_set_i64<<<1, 32, 0, rec>>>(d_s0s + set, s0);
+    if (len == K && !tried[set]) {
+      tried[set] = true;
+      g_rec[set] = capture([&] { return enqueue_recompute(K, set); });
+      g_rev[set] = capture([&] { return enqueue_reverse(K, set); });
+    }
+    stream_ = rec;
+    const cudaError_t e = (len == K && g_rec[set]) ? cudaGraphLaunch(g_rec[set], rec) : enqueue_recompute(len, set);
+    stream_ = main;
+    if (e != cudaSuccess) err = std::string("segment recompute: ") + cudaGetErrorString(e);
+    if (sets > 1) cudaEventRecord(a.ev_rec[set], rec);
+  };
+  if (sets > 1)
+    for (int q = 0; q < 2; ++q) cudaEventRecord(a.ev_rev[q], main);  // nothing to wait for but what came before
   for (int64_t seg = nseg - 1; seg >= 0 && err.empty(); --seg) {
-    const int64_t s0 = seg * K, s1 = std::min(a.n_steps, s0 + K), len = s1 - s0;
-    for (int q = 0; q < 3; ++q)
-      cudaMemcpyAsync(store[0] + q * C, a.checkpoints[seg] + q * C, C * sizeof(double), cudaMemcpyDeviceToDevice,
-                      stream_);
-    k_set_i64<<<1, 32, 0, stream_>>>(d_s0, s0);
-    if (len == K && !tried) {
-      tried = true;
-      g_rec = capture([&] { return enqueue_recompute(K); });
-      g_rev = capture([&] { return enqueue_reverse(K); });
-    }
-    cudaError_t e = (len == K && g_rec) ? cudaGraphLaunch(g_rec, stream_) : enqueue_recompute(len);
-    if (e != cudaSuccess) {
-      err = std::string("segment recompute: ") + cudaGetErrorString(e);
-      break;
-    }
-    e = (len == K && g_rev) ? cudaGraphLaunch(g_rev, stream_) : enqueue_reverse(len);
+    const int set = (int)(seg % sets);
+    const int64_t len = std::min(a.n_steps, (seg + 1) * K) - seg * K;
+    if (sets == 1 || seg == nseg - 1) recompute(seg);
+    if (sets > 1 && seg > 0 && err.empty()) recompute(seg - 1);
+    if (!err.empty()) break;
+    if (sets > 1) cudaStreamWaitEvent(main, a.ev_rec[set], 0);
+    const cudaError_t e = (len == K && g_rev[set]) ? cudaGraphLaunch(g_rev[set], main) : enqueue_reverse(len, set);
     if (e != cudaSuccess) err = std::string("stage reverse: ") + cudaGetErrorString(e);
+    if (sets > 1) cudaEventRecord(a.ev_rev[set], main);
   }
-  if (g_rec) cudaGraphExecDestroy(g_rec);
-  if (g_rev) cudaGraphExecDestroy(g_rev);
+  if (sets > 1) cudaStreamSynchronize(rec);  // (all of it was waited for, but on an error)
+  for (int q = 0; q < 2; ++q) {
+    if (g_rec[q]) cudaGraphExecDestroy(g_rec[q]);
+    if (g_rev[q]) cudaGraphExecDestroy(g_rev[q]);
+  }
   if (err.empty()) {
     double* d_out = store[0];
     k_interleave<<<gc, b, 0, stream_>>>(lam_step, (int)C, d_out);
@@ -1376,7 +1419,8 @@ std::string Engine::adjoint_backward(const double* trace_grads_host, double* gra
   for (auto& p : store) cudaFree(p);
   cudaFree(d_tg);
   cudaFree(lam_step);
-  cudaFree(d_s0);
+  cudaFree(d_s0s);
+  cudaFree(d_dt_rec);
   return err;
 }
 
