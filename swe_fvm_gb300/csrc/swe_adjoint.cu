@@ -1239,8 +1239,9 @@ std::string Engine::adjoint_backward(const double* trace_grads_host, double* gra
       wq.drain = (double*)take(C * sizeof(double));
       wq.pwrec = (double*)take(C * sizeof(double));
       wq.maxwp = (unsigned long long*)take(N * sizeof(unsigned long long));
-      wq.pwlist = (int*)take(C * sizeof(int));
       kept_n[q] = (double*)take(3 * C * sizeof(double));
+      // (after the 8-byte arrays: an odd number of cells would misalign them)
+      wq.pwlist = (int*)take(C * sizeof(int));
       wq.pwcount = (int*)take(sizeof(int));
       wq.cls = (unsigned char*)take((size_t)C);
       kept[q] = wq;
