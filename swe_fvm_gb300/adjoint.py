@@ -170,6 +170,11 @@ def _torch_functions():
             prim[:, 1:] = _as_dev(uv0, device).reshape(-1, 2)
         return prim.contiguous()
 
+    def _stream(device):
+        # torch's default stream is the legacy one, whose handle is 0: that would select the context's own
+        # stream, unordered with torch's work, so its named handle (cudaStreamLegacy, 1) is passed
+        return torch.cuda.current_stream(device).cuda_stream or 1
+
     def _device(t):
         return t.device if t.is_cuda else torch.device("cuda", torch.cuda.current_device())
 
@@ -207,7 +212,7 @@ def _torch_functions():
         def _tape(ent, w0, z_np, uv0, device, args):
             scheme, n_steps, ckpt, g, obs = args
             sd = ent.holder.sd
-            sd.set_stream(torch.cuda.current_stream(device).cuda_stream)
+            sd.set_stream(_stream(device))
             if not np.array_equal(ent.z[0], z_np):
                 sd.set_bathymetry(z_np)
                 ent.z[0] = z_np.copy()
@@ -229,6 +234,7 @@ def _torch_functions():
                 GaugeRollout._tape(ent, w0, z_np, uv0, ctx.device, ctx.args)
                 ctx.tape = ent.tape
             sd = ent.holder.sd
+            sd.set_stream(_stream(ctx.device))
             tg = grad_traces.detach().to(device=ctx.device, dtype=torch.float64).contiguous()
             gp = torch.empty((sd.num_cells, 3), dtype=torch.float64, device=ctx.device)
             gz = torch.empty((sd.num_nodes,), dtype=torch.float64, device=ctx.device)
@@ -277,7 +283,7 @@ def _torch_functions():
             scheme, n_steps, ckpt, g, obs = args
             br = ent.holder
             b = br.batch
-            b.set_stream(torch.cuda.current_stream(device).cuda_stream)
+            b.set_stream(_stream(device))
             changed = [None if np.array_equal(ent.z[q], zs[q]) else zs[q] for q in range(len(zs))]
             if any(c is not None for c in changed):
                 b.set_bathymetry(changed)
@@ -305,6 +311,7 @@ def _torch_functions():
                 BatchGaugeRollout._tape(ent, w0, zs, uv0s, ctx.device, ctx.args)
                 ctx.tape = ent.tape
             br = ent.holder
+            br.batch.set_stream(_stream(ctx.device))
             tg = grad_traces.detach().to(device=ctx.device, dtype=torch.float64).contiguous()
             gp = torch.empty((int(br.cell_off[-1]), 3), dtype=torch.float64, device=ctx.device)
             gz = torch.empty((int(br.node_off[-1]),), dtype=torch.float64, device=ctx.device)
