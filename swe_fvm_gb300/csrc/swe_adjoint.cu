@@ -865,8 +865,60 @@ __global__ void __launch_bounds__(32) k_pw_jacobian(DevMesh m, DevWork wk, AdjWo
 }  // namespace
 
 // ----------------------------------------------------------------- driver
+// What one backward pass needs besides the adjoint's work arrays: the segments'
+// stores and kept intermediates, and the captured graphs of a full segment's
+// recompute and reverse.  It is kept for the next backward pass of the same shape
+// (an inversion repeats one) up to kPlanBytes, else given back at once: allocating
+// and capturing it again took 2 ms of the 8 ms of a 20k-cell pass.
+constexpr size_t kPlanBytes = size_t(1) << 30;
+struct BackwardPlan {
+  // the shape it was made for, and the tape's arrays its graphs read
+  Scheme sc{};
+  int64_t K = 0, nseg = 0, obs = 0;
+  int n_gauges = 0, n_tg = 0;
+  const void *d_dt = nullptr, *d_gauges = nullptr;
+  double reg_depth = 0.;
+  // what it holds
+  bool made = false, keep = false;
+  int sets = 1;
+  size_t bytes = 0;
+  std::vector<void*> mem;
+  std::vector<double*> store;
+  std::vector<DevWork> kept;
+  std::vector<double*> kept_n;  // state before ConsAssigner of each stage
+  double *d_tg = nullptr, *lam_step = nullptr, *d_dt_rec = nullptr;
+  long long* d_s0s = nullptr;  // first step of the segment in each set
+  cudaGraphExec_t g_rec[2] = {}, g_rev[2] = {};
+  bool tried[2] = {};
+
+  bool fits(const BackwardPlan& o) const {
+    bool same = made && K == o.K && nseg == o.nseg && obs == o.obs && n_gauges == o.n_gauges && n_tg == o.n_tg &&
+                d_dt == o.d_dt && d_gauges == o.d_gauges && reg_depth == o.reg_depth && sc.n == o.sc.n;
+    for (int q = 0; same && q < sc.n; ++q)
+      same = sc.s[q].first == o.sc.s[q].first && sc.s[q].a == o.sc.s[q].a && sc.s[q].b == o.sc.s[q].b &&
+             sc.s[q].c == o.sc.s[q].c;
+    return same;
+  }
+  void* take(size_t n) {
+    void* p = nullptr;
+    if (cudaMalloc(&p, n ? n : 1) != cudaSuccess) return nullptr;
+    mem.push_back(p);
+    bytes += n;
+    return p;
+  }
+  void release() {
+    for (int q = 0; q < 2; ++q) {
+      if (g_rec[q]) cudaGraphExecDestroy(g_rec[q]);
+      if (g_rev[q]) cudaGraphExecDestroy(g_rev[q]);
+    }
+    for (void* p : mem) cudaFree(p);
+    *this = BackwardPlan();
+  }
+};
+
 struct AdjointState {
   AdjWork aw{};
+  BackwardPlan plan;
   std::vector<void*> allocs;
   // tape of the last taped forward run
   int scheme = 1;
@@ -891,6 +943,34 @@ struct AdjointState {
     allocs.push_back(p);
     return (T*)p;
   }
+  int64_t dt_cap = 0, traces_cap = 0, gauges_cap = 0;
+  // Room for a run's tape: arrays that are large enough stay (their addresses
+  // are in the backward plan's graphs), spare checkpoints go back.
+  bool reserve_tape(int64_t n_dt, int64_t n_traces, int64_t n_g, int64_t n_ckpt, int64_t C) {
+    taped = false;
+    auto room = [](auto*& p, int64_t& cap, int64_t n) {
+      if (p && cap >= n) return true;
+      if (p) cudaFree(p);
+      p = nullptr;
+      cap = 0;
+      if (cudaMalloc(&p, (n ? n : 1) * sizeof(*p)) != cudaSuccess) {
+        p = nullptr;
+        return false;
+      }
+      cap = n;
+      return true;
+    };
+    while ((int64_t)checkpoints.size() > n_ckpt) {
+      cudaFree(checkpoints.back());
+      checkpoints.pop_back();
+    }
+    while ((int64_t)checkpoints.size() < n_ckpt) {
+      double* cp = nullptr;
+      if (cudaMalloc(&cp, 3 * C * sizeof(double)) != cudaSuccess) return false;
+      checkpoints.push_back(cp);
+    }
+    return room(d_dt, dt_cap, n_dt) && room(d_traces, traces_cap, n_traces) && room(d_gauges, gauges_cap, n_g);
+  }
   void free_tape() {
     for (double* p : checkpoints) cudaFree(p);
     checkpoints.clear();
@@ -899,9 +979,11 @@ struct AdjointState {
     if (d_gauges) cudaFree(d_gauges);
     d_dt = d_traces = nullptr;
     d_gauges = nullptr;
+    dt_cap = traces_cap = gauges_cap = 0;
     taped = false;
   }
   ~AdjointState() {
+    plan.release();
     free_tape();
     for (void* p : allocs) cudaFree(p);
     if (side) cudaStreamDestroy(side);
@@ -916,7 +998,7 @@ void adjoint_state_delete(AdjointState* a) { delete a; }
 // The work arrays, the topology lists and the side stream stay; a run's tape is
 // of the old bed, and so are the plane adjoints.
 cudaError_t adjoint_state_new_bed(AdjointState* a, const DevMesh& m, cudaStream_t s) {
-  a->free_tape();
+  a->taped = false;
   k_plane_adj_init<<<(m.C + 255) / 256, 256, 0, s>>>(m, a->aw.padj);
   return cudaGetLastError();
 }
@@ -1030,7 +1112,6 @@ std::string Engine::adjoint_forward(int scheme, int64_t n_steps, int64_t ckpt, c
   std::string err = adjoint_init();
   if (!err.empty()) return err;
   AdjointState& a = *adj_;
-  a.free_tape();
   const int64_t C = mesh_.C;
   a.scheme = scheme;
   a.sc = scheme_of(scheme);
@@ -1040,18 +1121,10 @@ std::string Engine::adjoint_forward(int scheme, int64_t n_steps, int64_t ckpt, c
   a.n_gauges = n_gauges;
   const int64_t n_obs = obs > 0 ? n_steps / obs : 0;
   const int64_t NI = I();
-  if (cudaMalloc(&a.d_dt, (n_steps ? n_steps : 1) * NI * sizeof(double)) != cudaSuccess) return "tape allocation failed";
-  if (cudaMalloc(&a.d_traces, (n_obs * n_gauges ? n_obs * n_gauges : 1) * sizeof(double)) != cudaSuccess)
-    return "tape allocation failed";
-  if (cudaMalloc(&a.d_gauges, (n_gauges ? n_gauges : 1) * sizeof(int)) != cudaSuccess) return "tape allocation failed";
-  cudaMemcpy(a.d_gauges, gauges, n_gauges * sizeof(int), cudaMemcpyHostToDevice);
   // every checkpoint allocated up front (no allocation inside the run)
   const int64_t n_ckpt = n_steps > 0 ? (n_steps + ckpt - 1) / ckpt : 0;
-  for (int64_t q = 0; q < n_ckpt; ++q) {
-    double* cp = nullptr;
-    if (cudaMalloc(&cp, 3 * C * sizeof(double)) != cudaSuccess) return "checkpoint allocation failed";
-    a.checkpoints.push_back(cp);
-  }
+  if (!a.reserve_tape(n_steps * NI, n_obs * n_gauges, n_gauges, n_ckpt, C)) return "tape allocation failed";
+  cudaMemcpyAsync(a.d_gauges, gauges, n_gauges * sizeof(int), cudaMemcpyHostToDevice, stream_);
   for (int64_t n = 0; n < n_steps; ++n) {
     if (n % ckpt == 0) {
       double* cp = a.checkpoints[n / ckpt];
@@ -1161,66 +1234,38 @@ __global__ void k_rows_to_caller(const double* in, const int* map, int n, int w,
     for (int c = 0; c < w; ++c) out[(size_t)w * map[i] + c] = in[(size_t)w * i + c];
 }
 
-std::string Engine::adjoint_backward(const double* trace_grads_host, double* grad_prim_host, double* grad_z_host,
-                                     bool device) {
-  if (!adj_ || !adj_->taped) return "no taped forward run to differentiate";
-  if (device) {
-    std::string e = caller_maps();
-    if (!e.empty()) return e;
-  }
-  AdjointState& a = *adj_;
-  AdjWork& w = a.aw;
-  w.reg_depth = adj_reg_depth_;
-  state_changed();  // the recompute may go through the step's own list
-  const int64_t C = mesh_.C, N = mesh_.N;
-  const Scheme sc = a.sc;
-  const int ns = sc.n;
-  const int64_t n_obs = a.obs > 0 ? a.n_steps / a.obs : 0;
-  double* d_tg = nullptr;
-  if (cudaMalloc(&d_tg, (n_obs * a.n_gauges ? n_obs * a.n_gauges : 1) * sizeof(double)) != cudaSuccess)
-    return "allocation failed";
-  if (n_obs * a.n_gauges)
-    cudaMemcpy(d_tg, trace_grads_host, n_obs * a.n_gauges * sizeof(double),
-               device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice);
-  const int64_t K = a.ckpt;
-  const int64_t nseg = (a.n_steps + K - 1) / K;
+std::string Engine::make_backward_plan() {
+  BackwardPlan& plan = adj_->plan;
+  const int64_t C = mesh_.C, E = mesh_.E, N = mesh_.N, K = plan.K;
+  const int ns = plan.sc.n;
   // per-stage forward intermediates of one segment (interface slots, fluxes,
   // draining dt, node maxima, part-wet list) when device memory allows, and two
   // sets of them where there is room: the recompute of the segment before then
   // runs on a stream of its own beside a segment's reverse (both are chains of
   // small kernels on all but the largest meshes)
-  const int64_t E = mesh_.E;
   const size_t per_stage = ((15 * C + 10 * E + 5 * C) * sizeof(double) + N * sizeof(unsigned long long) +
                             (C + 1) * sizeof(int) + C + 255) / 256 * 256;
   size_t free_b = 0, total_b = 0;
   cudaMemGetInfo(&free_b, &total_b);
   const double one_set = ((double)per_stage + 24. * (double)C) * (double)(K * ns);
-  const bool keep = (double)per_stage * (double)(K * ns) < 0.6 * (double)free_b;
-  const int sets = keep && nseg > 1 && 2. * one_set < 0.6 * (double)free_b ? 2 : 1;
-  // stage-input store of a segment: [K][ns] states of 3C, plus the segment end
-  const size_t per_set = (size_t)K * ns + 1;
-  std::vector<double*> store(per_set * sets, nullptr);
-  for (auto& p : store)
-    if (cudaMalloc(&p, 3 * C * sizeof(double)) != cudaSuccess) {
-      cudaFree(d_tg);
-      for (auto& q : store)
-        if (q) cudaFree(q);
-      return "segment store allocation failed";
-    }
-  const int b = 256, gc = (int)((C + b - 1) / b);
-  std::vector<DevWork> kept;
-  std::vector<double*> kept_n;  // state before ConsAssigner of each stage
-  char* kept_pool = nullptr;
-  if (keep) {
-    if (cudaMalloc(&kept_pool, per_stage * (size_t)(sets * K * ns)) != cudaSuccess) {
-      cudaFree(d_tg);
-      for (auto& q : store) cudaFree(q);
-      return "intermediate store allocation failed";
-    }
-    kept.resize((size_t)(sets * K * ns));
-    kept_n.resize((size_t)(sets * K * ns));
-    for (int64_t q = 0; q < sets * K * ns; ++q) {
-      char* p = kept_pool + per_stage * (size_t)q;
+  plan.keep = (double)per_stage * (double)(K * ns) < 0.6 * (double)free_b;
+  plan.sets = plan.keep && plan.nseg > 1 && 2. * one_set < 0.6 * (double)free_b ? 2 : 1;
+  plan.d_tg = (double*)plan.take(plan.n_tg * sizeof(double));
+  plan.lam_step = (double*)plan.take(3 * C * sizeof(double));  // adjoint of the current step's end state
+  plan.d_dt_rec = (double*)plan.take(I() * sizeof(double));    // the recompute's step dt
+  plan.d_s0s = (long long*)plan.take(2 * sizeof(long long));
+  if (!plan.d_tg || !plan.lam_step || !plan.d_dt_rec || !plan.d_s0s) return "allocation failed";
+  plan.store.assign(((size_t)K * ns + 1) * plan.sets, nullptr);
+  for (auto& p : plan.store)
+    if (!(p = (double*)plan.take(3 * C * sizeof(double)))) return "segment store allocation failed";
+  if (plan.keep) {
+    const int64_t n = plan.sets * K * ns;
+    char* pool = (char*)plan.take(per_stage * (size_t)n);
+    if (!pool) return "intermediate store allocation failed";
+    plan.kept.resize((size_t)n);
+    plan.kept_n.resize((size_t)n);
+    for (int64_t q = 0; q < n; ++q) {
+      char* p = pool + per_stage * (size_t)q;
       DevWork wq = work_;
       auto take = [&](size_t bytes) {
         char* r = p;
@@ -1239,14 +1284,72 @@ std::string Engine::adjoint_backward(const double* trace_grads_host, double* gra
       wq.drain = (double*)take(C * sizeof(double));
       wq.pwrec = (double*)take(C * sizeof(double));
       wq.maxwp = (unsigned long long*)take(N * sizeof(unsigned long long));
-      kept_n[q] = (double*)take(3 * C * sizeof(double));
+      plan.kept_n[q] = (double*)take(3 * C * sizeof(double));
       // (after the 8-byte arrays: an odd number of cells would misalign them)
       wq.pwlist = (int*)take(C * sizeof(int));
       wq.pwcount = (int*)take(sizeof(int));
       wq.cls = (unsigned char*)take((size_t)C);
-      kept[q] = wq;
+      plan.kept[q] = wq;
     }
   }
+  plan.made = true;
+  return "";
+}
+
+std::string Engine::adjoint_backward(const double* trace_grads_host, double* grad_prim_host, double* grad_z_host,
+                                     bool device) {
+  if (!adj_ || !adj_->taped) return "no taped forward run to differentiate";
+  if (device) {
+    std::string e = caller_maps();
+    if (!e.empty()) return e;
+  }
+  AdjointState& a = *adj_;
+  AdjWork& w = a.aw;
+  w.reg_depth = adj_reg_depth_;
+  state_changed();  // the recompute may go through the step's own list
+  const int64_t C = mesh_.C, N = mesh_.N;
+  const Scheme sc = a.sc;
+  const int ns = sc.n;
+  const int64_t n_obs = a.obs > 0 ? a.n_steps / a.obs : 0;
+  const int64_t K = a.ckpt;
+  const int64_t nseg = (a.n_steps + K - 1) / K;
+  const int64_t E = mesh_.E;
+  const int b = 256, gc = (int)((C + b - 1) / b);
+  const size_t per_set = (size_t)K * ns + 1;  // stage inputs of a segment, [K][ns] states of 3C, plus its end
+  BackwardPlan& plan = a.plan;
+  {
+    BackwardPlan want;
+    want.sc = sc;
+    want.K = K;
+    want.nseg = nseg;
+    want.obs = a.obs;
+    want.n_gauges = a.n_gauges;
+    want.n_tg = (int)(n_obs * a.n_gauges);
+    want.d_dt = a.d_dt;
+    want.d_gauges = a.d_gauges;
+    want.reg_depth = adj_reg_depth_;
+    if (!plan.fits(want)) {
+      cudaStreamSynchronize(stream_);
+      plan.release();
+      plan = want;
+      std::string e = make_backward_plan();
+      if (!e.empty()) {
+        plan.release();
+        return e;
+      }
+    }
+  }
+  const bool keep = plan.keep;
+  const int sets = plan.sets;
+  std::vector<double*>& store = plan.store;
+  std::vector<DevWork>& kept = plan.kept;
+  std::vector<double*>& kept_n = plan.kept_n;
+  double *const d_tg = plan.d_tg, *const lam_step = plan.lam_step, *const d_dt_rec = plan.d_dt_rec;
+  long long* const d_s0s = plan.d_s0s;
+  if (n_obs * a.n_gauges)
+    // on the engine's stream: device gradients are ordered with the work that made them there
+    cudaMemcpyAsync(d_tg, trace_grads_host, n_obs * a.n_gauges * sizeof(double),
+                    device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, stream_);
   cudaMemsetAsync(w.lam, 0, 3 * C * sizeof(double), stream_);
   cudaMemsetAsync(w.lz, 0, N * sizeof(double), stream_);
   cudaMemsetAsync(w.lscatter, 0, C * sizeof(double), stream_);
@@ -1254,18 +1357,11 @@ std::string Engine::adjoint_backward(const double* trace_grads_host, double* gra
   std::vector<double> tsum_saved((size_t)I(), 0.);  // the recompute must not advance the clocks
   cudaMemcpyAsync(tsum_saved.data(), work_.tsum, I() * sizeof(double), cudaMemcpyDeviceToHost, stream_);
   cudaStreamSynchronize(stream_);
-  double* lam_step = nullptr;  // adjoint of the current step's end state
-  cudaMalloc(&lam_step, 3 * C * sizeof(double));
   cudaMemsetAsync(lam_step, 0, 3 * C * sizeof(double), stream_);
   std::string err;
   // The first step index of the current segment lives on the device, so that
   // one captured graph of a full segment's recompute and one of its reverse
   // replay for every full segment.
-  long long* d_s0s = nullptr;  // one per set
-  if (cudaMalloc(&d_s0s, 2 * sizeof(long long)) != cudaSuccess) err = "allocation failed";
-  // the recompute's step dt (the reverse fetches its own into work_.dt)
-  double* d_dt_rec = nullptr;
-  if (cudaMalloc(&d_dt_rec, I() * sizeof(double)) != cudaSuccess) err = "allocation failed";
   const bool seeds = a.obs > 0 && a.n_gauges > 0;
   // recompute of steps s0 .. s0+len-1 with the recorded dt, keeping every
   // stage's forward intermediates when they fit
@@ -1361,8 +1457,8 @@ std::string Engine::adjoint_backward(const double* trace_grads_host, double* gra
     cudaGetLastError();
     return ge;
   };
-  cudaGraphExec_t g_rec[2] = {nullptr, nullptr}, g_rev[2] = {nullptr, nullptr};
-  bool tried[2] = {false, false};
+  cudaGraphExec_t *const g_rec = plan.g_rec, *const g_rev = plan.g_rev;
+  bool* const tried = plan.tried;
   const cudaStream_t main = stream_, rec = sets > 1 ? a.rec : main;
   // the recompute of segment seg into its set, after the reverse that last read
   // that set
@@ -1397,10 +1493,6 @@ std::string Engine::adjoint_backward(const double* trace_grads_host, double* gra
     if (sets > 1) cudaEventRecord(a.ev_rev[set], main);
   }
   if (sets > 1) cudaStreamSynchronize(rec);  // (all of it was waited for, but on an error)
-  for (int q = 0; q < 2; ++q) {
-    if (g_rec[q]) cudaGraphExecDestroy(g_rec[q]);
-    if (g_rev[q]) cudaGraphExecDestroy(g_rev[q]);
-  }
   if (err.empty()) {
     double* d_out = store[0];
     k_interleave<<<gc, b, 0, stream_>>>(lam_step, (int)C, d_out);
@@ -1416,12 +1508,10 @@ std::string Engine::adjoint_backward(const double* trace_grads_host, double* gra
     if (e != cudaSuccess) err = std::string("adjoint: ") + cudaGetErrorString(e);
   }
   cudaMemcpy(work_.tsum, tsum_saved.data(), I() * sizeof(double), cudaMemcpyHostToDevice);
-  if (kept_pool) cudaFree(kept_pool);
-  for (auto& p : store) cudaFree(p);
-  cudaFree(d_tg);
-  cudaFree(lam_step);
-  cudaFree(d_s0s);
-  cudaFree(d_dt_rec);
+  if (plan.bytes > kPlanBytes || !err.empty()) {
+    cudaStreamSynchronize(stream_);
+    plan.release();
+  }
   return err;
 }
 

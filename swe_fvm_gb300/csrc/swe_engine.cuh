@@ -341,6 +341,7 @@ class Engine {
   std::string adjoint_backward(const double* trace_grads_host, double* grad_prim_host, double* grad_z_host,
                                bool device = false);
   std::string adjoint_dts(double* out_host);
+  std::string make_backward_plan();  // allocates adj_->plan for the shape set in it
   // Depth below which the reverse regularises the w-slope of a PartWet1 level
   // that feeds a node maximum (kEta1 by default; 0 = exact derivative).
   void set_adjoint_regularisation(double depth) { adj_reg_depth_ = depth; }
