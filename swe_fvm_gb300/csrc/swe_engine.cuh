@@ -156,6 +156,7 @@ struct DevWork {
   double* pwrec;               // [C] PartWet1 level of listed cells
   // [C] pass-1 class of each cell: type (0 dry, 1 partially wet, 2 fully wet)
   // | neighbour combination mask << 2 | combination plane kept << 5
+  // | partially wet and finished by pass 1 << 6 (kFinished)
   unsigned char* cls;
   double* ftape;               // [7][E] flux intermediates kept for the adjoint, or null
   unsigned long long* r;       // [I] ordered key of min length-to-wavespeed

@@ -261,30 +261,46 @@ __device__ __forceinline__ void append_listed(const DevWork& wk, int C, bool par
   }
 }
 
+// A partially-wet cell whose level stands above its highest vertex (in practice
+// every wet cell along a wall) keeps that level, flat, in both passes
+// (src/MUSCLObject.cpp:96-97, 124): pass 1 finishes it, marks its class byte, and
+// only the others are listed.  Walls have most of the partially-wet cells of most
+// meshes (the 25,000-cell coast lists 601 of 1033, an all-wet basin none of its
+// rim: 20k-cell inversion iteration 12.1 -> 11.6 ms).  From kSoftCells cells on
+// they are listed all the same: there their edges, walls among them, cost k_flux
+// more than k_flux_pw, which runs beside it (32 basins of 218,000 cells 250 -> 257
+// us a step, 1M-cell dam break 608 -> 615).
+constexpr unsigned kFinished = 64u;
+__device__ __forceinline__ bool listed_class(unsigned cls) { return (cls & (3u | kFinished)) == 1u; }
+__device__ __forceinline__ bool above_all(const DevMesh& m, int i, double w) {
+  return dlt(m.pw1[(size_t)i * kPw1Stride], w);
+}
+
 // Whether cell i with level w is partially wet (neither dry nor fully wet,
-// src/MUSCLObject.cpp:13-29).
-__device__ __forceinline__ bool partly_wet(const DevMesh& m, int i, double w) {
+// src/MUSCLObject.cpp:13-29) and to be listed; finish: but for those cells.
+__device__ __forceinline__ bool to_list(const DevMesh& m, int i, double w, bool finish) {
   const double2 t = __ldg(m.thr + i);
-  return !dlt(w, t.x) && !dlt(t.y, w);
+  return !dlt(w, t.x) && !dlt(t.y, w) && !(finish && above_all(m, i, w));
 }
 
 // The partially-wet cells of a state that no update left (a new state or bed).
-__global__ void __launch_bounds__(256) k_list_partwet(DevMesh m, DevWork wk, const double* __restrict__ W) {
+__global__ void __launch_bounds__(256) k_list_partwet(DevMesh m, DevWork wk, const double* __restrict__ W,
+                                                      bool finish) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  append_listed(wk, m.C, i < m.C && partly_wet(m, i, W[i]), i);
+  append_listed(wk, m.C, i < m.C && to_list(m, i, W[i], finish), i);
 }
 
 // ---------------------------------------------------------------- kernels
 // Pass 1 but for the partly wet cells' levels (k_partwet1, beside it).  Bound by
-// its gathers.  append: list those cells (a step's are listed by the update
-// before it).
+// its gathers.  append: list the partially-wet cells, all of them (a step's are
+// listed by the update before it).  finish: see kFinished.
 // The wet test and the plane's positivity are comparisons with levels kept in
 // the mesh (DevMesh::thr, record entry 2) where the rounded sums would cost
 // seven FP64 operations; 6 are left in a fully-wet cell of 18.
 template <bool BATCH, int FORM>
 __global__ void __launch_bounds__(256, 5) k_recon1(DevMesh m, DevWork wk, const double* __restrict__ W,
                                                 const double* __restrict__ U, const double* __restrict__ V,
-                                                int latch_mode, bool append) {
+                                                int latch_mode, bool append, bool finish) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   bool part = false;
   unsigned char cls = 0;  // dry unless set below
@@ -326,17 +342,19 @@ __global__ void __launch_bounds__(256, 5) k_recon1(DevMesh m, DevWork wk, const 
         const double h = wet_slots ? dr[3 + k] - be : 0.;
         write_slot<FORM>(wk, slot, h, be, FORM == kLean ? 0. : dr[3 + k], 0., 0., gx, gy, cor);
       }
-    } else if (!dlt(level.y, w)) {
+    } else if (!dlt(level.y, w) && !(finish && above_all(m, i, w))) {
       // partially wet: listed for k_partwet1 and k_recon2
       part = true;
       cls = 1;
     } else {
-      // ReconstructFullWetCell (src/MUSCLObject.cpp:38-84)
+      // ReconstructFullWetCell (src/MUSCLObject.cpp:38-84); or flat, a
+      // partially-wet cell that is finished here
+      const bool flat = !dlt(level.y, w);
       int mask = 0;
-      bool first_order = false;
-      double wn[3];
+      bool first_order = flat;
+      double wn[3] = {w, w, w};
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
+      for (int k = 0; k < 3 && !flat; ++k) {
         const int nb = gidx(wk, m.cnbr[k * C + i], C);  // never a wall: fully-wet cells are interior
         const double wj = W[nb];
         wn[k] = wj;
@@ -349,7 +367,8 @@ __global__ void __launch_bounds__(256, 5) k_recon1(DevMesh m, DevWork wk, const 
           mask |= 1 << k;  // partially-wet neighbour: plane point at the edge centre
         }
       }
-      cls = (unsigned char)(2 | (mask << 2));
+      cls = (unsigned char)(flat ? 1u | kFinished : 2u | ((unsigned)mask << 2));
+      if (flat) wk.pwrec[i] = w;
       double at[3] = {w, w, w};  // the plane's level at the edge centres
       if (!first_order) {
         const double2* rec = (const double2*)(m.combo + combo_off(C, i, mask));
@@ -584,8 +603,7 @@ __device__ __forceinline__ bool flux_edge(const DevMesh& m, const DevWork& wk, c
 }
 
 // MODE 0: every edge, from the full interface values.  MODE 1: the edges none
-// of whose cells is partially wet (the others wait for PartWet2 and go through
-// k_flux_pw).
+// of whose cells is listed (the others wait for PartWet2 and go through k_flux_pw).
 // TAPE: also store the intermediates the adjoint's reverse reads (wk.ftape).
 // Register caps (the second __launch_bounds__ argument: blocks of 256 threads
 // per SM) measured on the 1M-cell dam break, CUDA events, same bits: k_flux at
@@ -605,7 +623,7 @@ __global__ void __launch_bounds__(256, 4) k_flux(DevMesh m, DevWork wk, const do
     bool mine = true;
     if (MODE == 1) {
       const int nb = m.enb[e];
-      mine = !(((wk.cls[gidx(wk, m.eown[e], m.C)] & 3) == 1) || (nb >= 0 && (wk.cls[gidx(wk, nb, m.C)] & 3) == 1));
+      mine = !(listed_class(wk.cls[gidx(wk, m.eown[e], m.C)]) || (nb >= 0 && listed_class(wk.cls[gidx(wk, nb, m.C)])));
     }
     if (mine && !flux_edge<FLUX, TAPE, SOFT, MODE == 0>(m, wk, W, U, V, e, inst, &lw)) {
       lw = kInf;
@@ -667,9 +685,10 @@ __global__ void __launch_bounds__(128) k_flux_pw(DevMesh m, DevWork wk, const do
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     const int q = t / 3, k = t - 3 * q;
     const int i = gidx(wk, wk.pwlist[q], C);
+    if (!listed_class(wk.cls[i])) continue;  // (a list that pass 1 itself made has all)
     const int e = gidx(wk, m.cedge[k * C + i], m.E);
     const int o = gidx(wk, m.eown[e], C);
-    if ((((wk.cls[o] & 3) == 1) ? o : m.enb[e]) != i) continue;
+    if ((listed_class(wk.cls[o]) ? o : m.enb[e]) != i) continue;
     const int inst = BATCH ? m.einst[e] : 0;
     double lw = kInf;
     flux_edge<FLUX, TAPE, false, false>(m, wk, W, U, V, e, inst, &lw);
@@ -850,7 +869,7 @@ __global__ void __launch_bounds__(256, 5) k_update(DevMesh m, DevWork wk, const 
   // list the next stage's partially-wet cells, so that their PartWet1 runs beside
   // its k_recon1 instead of after it (a plain append: one over the warp's lanes
   // kept registers across the whole kernel, 99 -> 110 us on a million cells)
-  if (!STORE_N && partly_wet(m, i, ow)) {
+  if (!STORE_N && to_list(m, i, ow, !SOFT)) {
     const int slot = atomicAdd(wk.pwcount, 1);
     if (slot < m.C) wk.pwlist[slot] = i;
   }
@@ -1104,14 +1123,15 @@ cudaError_t Engine::reset_pass(bool list) {
 void Engine::launch_recon1(const double* W, const double* U, const double* V, int latch_mode, bool slots,
                            bool append) {
   const int b = blk_[0], g = nblocks(mesh_.C, b);
+  const bool finish = !append && !soft_;
   const int form = !slots ? kLean : cor0_ ? kSlotsCor0 : kSlotsCor;
   switch (form + (batched_ ? 3 : 0)) {
-    case 0: k_recon1<false, kLean><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode, append); break;
-    case 1: k_recon1<false, kSlotsCor0><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode, append); break;
-    case 2: k_recon1<false, kSlotsCor><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode, append); break;
-    case 3: k_recon1<true, kLean><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode, append); break;
-    case 4: k_recon1<true, kSlotsCor0><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode, append); break;
-    default: k_recon1<true, kSlotsCor><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode, append); break;
+    case 0: k_recon1<false, kLean><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode, append, finish); break;
+    case 1: k_recon1<false, kSlotsCor0><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode, append, finish); break;
+    case 2: k_recon1<false, kSlotsCor><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode, append, finish); break;
+    case 3: k_recon1<true, kLean><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode, append, finish); break;
+    case 4: k_recon1<true, kSlotsCor0><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode, append, finish); break;
+    default: k_recon1<true, kSlotsCor><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode, append, finish); break;
   }
   ++launches_;
 }
@@ -1130,7 +1150,7 @@ void Engine::launch_partwet1(const double* W, cudaStream_t s) {
 
 cudaError_t Engine::list_partwet(const double* W) {
   cudaError_t e = cudaMemsetAsync(work_.pwcount, 0, sizeof(int), stream_);
-  k_list_partwet<<<nblocks(mesh_.C, 256), 256, 0, stream_>>>(mesh_, work_, W);
+  k_list_partwet<<<nblocks(mesh_.C, 256), 256, 0, stream_>>>(mesh_, work_, W, !soft_);
   ++launches_;
   return e == cudaSuccess ? cudaGetLastError() : e;
 }
