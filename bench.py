@@ -39,13 +39,13 @@ import numpy as np  # noqa: E402
 # 24 x N/C ~ 12 = 84 B; stage 2 re-reads the step's initial state, 24 B.
 BYTES_PER_CELL_STEP = 2 * 84 + 24
 # FP64 instructions issued per SSPRK2 cell-step by the step kernels: ncu
-# smsp__sass_thread_inst_executed_op_fp64_pred_on summed over the 12 launches
-# of one step of the dam break at lattice 500 (498,002 cells): 1.942e8, i.e.
-# per stage k_flux 62 per edge x 1.5 edges per cell + k_update 73-79 +
-# k_recon1 18 + k_drain 7 per cell, plus the few part-wet cells.  The bound of
-# the step on GB300, whose FP64 pipe issues one instruction per lane and cycle
-# (DFMA = 2 flops).
-FP64_INST_PER_CELL_STEP = 390
+# smsp__sass_thread_inst_executed_op_fp64_pred_on summed over the 14 launches
+# of one step of the dam break at lattice 500 (498,002 cells): 8.289e7, i.e.
+# per stage k_flux 30 per edge x 1.5 edges per cell + k_update 26-30 +
+# k_recon1 6 + k_drain 3 per cell, plus the few part-wet cells (the products of
+# the flux and update are on the integer pipe).  GB300's FP64 pipe issues one
+# instruction per lane and cycle on 2 lanes an SM (DFMA = 2 flops).
+FP64_INST_PER_CELL_STEP = 166
 LATTICE = int(os.environ.get("SWE_BENCH_LATTICE", "708"))
 CFL = 0.15
 
@@ -632,11 +632,11 @@ def run_batch_adjoint(torch, stream):
 
 
 # DRAM bytes per SSPRK2 step: dram__bytes_read.sum + dram__bytes_write.sum over
-# the step's 12 kernels in one ncu capture of the same command line at lattice
-# 500 (498,002 cells, tuned order and blocks): 802.8 MB, 1612 B per cell,
+# the step's 14 kernels in one ncu capture of the same command line at lattice
+# 500 (498,002 cells, tuned order and blocks): 592.3 MB, 1189 B per cell,
 # scaled by the cell count to the 999,698-cell mesh (every kernel's bytes grow
 # with its cells or edges).
-TRAFFIC_PER_STEP = {500: 8.028e8, 708: 1.6115e9}
+TRAFFIC_PER_STEP = {500: 5.923e8, 708: 1.1890e9}
 
 
 def run_reference(args):
