@@ -288,7 +288,10 @@ class Engine {
   cudaError_t reset_pass(bool list = true);
   // The state in buffer 0 was written from outside: its part-wet list is to be
   // made before the next step (a step leaves the next one's).
-  void state_changed() { list_valid_ = false; }
+  void state_changed() {
+    list_valid_ = false;
+    note_capture();
+  }
   // Launches one reconstruction (pass 1 + pass 2) with the full interface
   // values, and one flux pass from them.
   cudaError_t interface_values(const double* W, const double* U, const double* V);
@@ -378,7 +381,7 @@ class Engine {
 
  private:
   cudaError_t launch_stage(const Stage& st, const double* const* in, const double* const* u0, double* const* out,
-                           bool first_stage_of_step, int latch_mode, cudaEvent_t* ev = nullptr);
+                           bool first_stage_of_step, int latch_mode, bool full = false, cudaEvent_t* ev = nullptr);
   template <class T>
   T* dalloc(size_t n);
 
@@ -405,6 +408,14 @@ class Engine {
   cudaError_t list_partwet(const double* W);  // empties the list and fills it from W
   cudaError_t ensure_list();
   bool list_valid_ = false;  // the part-wet list is that of the state in buffer 0
+  // A state upload, a reconstruction or a flux pass was recorded into the
+  // caller's own CUDA graph, whose replays this object does not see: from then
+  // on every run lists its cells itself, every stage leaves the full interface
+  // values, and buffer 1 keeps the state that these were made of.
+  bool captured_ = false;
+  bool graphs_slots_ = false;  // graphs_ were made after that
+  bool note_capture();         // whether the stream is being captured now
+  cudaError_t keep_input();    // buffer 0 into buffer 1
   void launch_recon2(const double* W, const double* U, const double* V, cudaStream_t s, bool slots);
   // the fluxes of a stage's input: the edges with no partially-wet cell, and
   // the others (those of the listed cells) on stream s

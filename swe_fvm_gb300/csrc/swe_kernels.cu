@@ -1156,7 +1156,7 @@ cudaError_t Engine::list_partwet(const double* W) {
 }
 
 cudaError_t Engine::ensure_list() {
-  if (list_valid_) return cudaSuccess;
+  if (list_valid_ && !captured_) return cudaSuccess;
   list_valid_ = true;
   return list_partwet(state(0, 0));
 }
@@ -1175,18 +1175,39 @@ void Engine::launch_recon2(const double* W, const double* U, const double* V, cu
   ++launches_;
 }
 
+bool Engine::note_capture() {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream_, &st) != cudaSuccess) cudaGetLastError();
+  const bool now = st == cudaStreamCaptureStatusActive;
+  captured_ = captured_ || now;
+  return now;
+}
+
+cudaError_t Engine::keep_input() {
+  cudaError_t e = cudaSuccess;
+  for (int c = 0; c < 3 && e == cudaSuccess; ++c)
+    e = cudaMemcpyAsync(state(1, c), state(0, c), mesh_.C * sizeof(double), cudaMemcpyDeviceToDevice, stream_);
+  return e;
+}
+
 cudaError_t Engine::interface_values(const double* W, const double* U, const double* V) {
+  const bool now = W == state(0, 0) && note_capture();
+  if (W == state(0, 0) && captured_) {
+    cudaError_t e = keep_input();
+    if (e != cudaSuccess) return e;
+  }
   launch_recon1(W, U, V, 0, true, true);
   launch_partwet1(W, stream_);
   launch_recon2(W, U, V, stream_, true);
   k_node_max_all<<<nblocks(std::max(mesh_.N, 1), 256), 256, 0, stream_>>>(mesh_, work_, W);
   ++launches_;
-  slots_stale_ = false;
+  slots_stale_ = slots_stale_ && now;  // recorded only: nothing has run
   list_valid_ = W == state(0, 0);
   return cudaGetLastError();
 }
 
 cudaError_t Engine::refresh_slots() {
+  const bool now = note_capture();
   if (!slots_stale_) return cudaSuccess;
   // the last stage read buffer 1; the CFL ratio of its flux pass stays
   cudaError_t e = cudaMemsetAsync(work_.pwcount, 0, sizeof(int), stream_);
@@ -1194,7 +1215,7 @@ cudaError_t Engine::refresh_slots() {
   launch_recon1(state(1, 0), state(1, 1), state(1, 2), 3, true, true);
   launch_partwet1(state(1, 0), stream_);
   launch_recon2(state(1, 0), state(1, 1), state(1, 2), stream_, true);
-  slots_stale_ = false;
+  slots_stale_ = now;
   list_valid_ = false;  // it is that buffer's now
   return cudaGetLastError();
 }
@@ -1260,12 +1281,12 @@ void Engine::stage_fluxes_pw(const double* const* in, cudaStream_t s) {
 }
 
 cudaError_t Engine::launch_stage(const Stage& st, const double* const* in, const double* const* u0,
-                                 double* const* out, bool first_stage_of_step, int latch_mode, cudaEvent_t* ev) {
+                                 double* const* out, bool first_stage_of_step, int latch_mode, bool full, cudaEvent_t* ev) {
   const int b = blk_[2];
   const int lm = first_stage_of_step ? latch_mode : 0;
   // a stage that overwrites its own input leaves the full interface values now
   // (refresh_slots could not make them later)
-  const bool slots = in[0] == out[0];
+  const bool slots = full || in[0] == out[0];
   // (the input's partially-wet cells are listed: by the update before, or ensure_list)
   if (ev) {
     // per-kernel timing: the kernels one after another
@@ -1345,13 +1366,14 @@ cudaError_t Engine::step_timed(int scheme, int latch_mode, double* acc) {
   for (auto& row : ev)
     for (auto& x : row) cudaEventCreate(&x);
   cudaError_t e = ensure_list();
+  if (e == cudaSuccess && captured_ && sc.n == 1) e = keep_input();
   for (int s = 0; s < sc.n && e == cudaSuccess; ++s) {
     const bool last = (s == sc.n - 1);
     const double* const* in = (s == 0) ? S0 : S1;
     double* const* out = last ? S0 : S1;
-    e = launch_stage(sc.s[s], in, S0, out, s == 0, latch_mode, ev[s]);
+    e = launch_stage(sc.s[s], in, S0, out, s == 0, latch_mode, captured_, ev[s]);
   }
-  slots_stale_ = sc.n > 1;
+  slots_stale_ = sc.n > 1 && !captured_;
   if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
   if (e == cudaSuccess) {
     for (int s = 0; s < sc.n; ++s)
@@ -1559,11 +1581,15 @@ cudaError_t Engine::step(int scheme, int latch_mode) {
   const Scheme sc = scheme_of(scheme);
   double* S0[3] = {state(0, 0), state(0, 1), state(0, 2)};
   double* S1[3] = {state(1, 0), state(1, 1), state(1, 2)};
+  if (captured_ && sc.n == 1) {
+    cudaError_t e = keep_input();
+    if (e != cudaSuccess) return e;
+  }
   for (int s = 0; s < sc.n; ++s) {
     const bool last = (s == sc.n - 1);
     const double* const* in = (s == 0) ? S0 : S1;
     double* const* out = last ? S0 : S1;
-    cudaError_t e = launch_stage(sc.s[s], in, S0, out, s == 0, latch_mode);
+    cudaError_t e = launch_stage(sc.s[s], in, S0, out, s == 0, latch_mode, captured_);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -1573,6 +1599,17 @@ cudaError_t Engine::run_graph(int scheme, int latch_mode, int64_t n) {
   if (n <= 0) return cudaSuccess;
   const cudaError_t el = ensure_list();
   if (el != cudaSuccess) return el;
+  if (captured_ && !graphs_slots_) {
+    // the graphs of before leave no interface values; dropped here, as a call
+    // that frees something would break off the caller's capture
+    for (auto& row : graphs_)
+      for (auto& g : row)
+        if (g) {
+          cudaGraphExecDestroy(g);
+          g = nullptr;
+        }
+    graphs_slots_ = true;
+  }
   cudaGraphExec_t& ge = graphs_[scheme][latch_mode];
   const int64_t per_step = launches_;
   if (!ge) {
@@ -1604,10 +1641,13 @@ cudaError_t Engine::run_graph(int scheme, int latch_mode, int64_t n) {
     launches_ = per_step;  // capture launched nothing
   }
   const int64_t kernels_per_step = 7 * scheme_of(scheme).n;
-  slots_stale_ = scheme_of(scheme).n > 1;
+  slots_stale_ = scheme_of(scheme).n > 1 && !captured_;
   for (int64_t s = 0; s < n; ++s) {
     cudaError_t e = cudaGraphLaunch(ge, stream_);
-    if (e != cudaSuccess) return e;
+    if (e != cudaSuccess) {
+      list_valid_ = false;  // refused (a stream that is being captured): no listing ran
+      return e;
+    }
   }
   launches_ += kernels_per_step * n;
   return cudaSuccess;
