@@ -1547,6 +1547,14 @@ std::string Engine::set_bathymetry(const std::vector<const double*>& z) {
     for (int64_t p = 0; p < h.N; ++p)
       if (!std::isfinite(z[q][(L && !L->identity()) ? L->node_from[p] : p])) return "bathymetry has a non-finite value";
   }
+  // the interface values stay those of the last reconstruction: left to a getter,
+  // they would be made of its input and the new bed.  (A batch has no call that
+  // reads them.)  Three kernels, within the runs' spread (1 %) of an iteration of
+  // a 20k-cell gauge inversion, 11.7 ms.
+  if (!batched_) {
+    const cudaError_t es = refresh_slots();
+    if (es != cudaSuccess) return std::string("interface values of the old bed: ") + cudaGetErrorString(es);
+  }
   for (size_t q = 0; q < host.size(); ++q) {
     if (!z[q]) continue;
     HostInstance& h = host[q];
