@@ -407,6 +407,7 @@ class Engine {
   int listed_blocks() const;
   cudaError_t list_partwet(const double* W);  // empties the list and fills it from W
   cudaError_t ensure_list();
+  void note_steps(int n);
   bool list_valid_ = false;  // the part-wet list is that of the state in buffer 0
   // A state upload, a reconstruction or a flux pass was recorded into the
   // caller's own CUDA graph, whose replays this object does not see: from then

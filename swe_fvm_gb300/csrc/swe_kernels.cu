@@ -1157,8 +1157,15 @@ cudaError_t Engine::list_partwet(const double* W) {
 
 cudaError_t Engine::ensure_list() {
   if (list_valid_ && !captured_) return cudaSuccess;
-  list_valid_ = true;
   return list_partwet(state(0, 0));
+}
+
+// The flags of steps of n stages that were accepted: the last update listed the
+// new state's cells, and steps of several stages leave the full interface values
+// to refresh_slots.  (A refused one leaves both as they are, or unlisted.)
+void Engine::note_steps(int n) {
+  list_valid_ = true;
+  slots_stale_ = n > 1 && !captured_;
 }
 
 void Engine::launch_recon2(const double* W, const double* U, const double* V, cudaStream_t s, bool slots) {
@@ -1373,9 +1380,10 @@ cudaError_t Engine::step_timed(int scheme, int latch_mode, double* acc) {
     double* const* out = last ? S0 : S1;
     e = launch_stage(sc.s[s], in, S0, out, s == 0, latch_mode, captured_, ev[s]);
   }
-  slots_stale_ = sc.n > 1 && !captured_;
   if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);
+  if (e != cudaSuccess) list_valid_ = false;
   if (e == cudaSuccess) {
+    note_steps(sc.n);
     for (int s = 0; s < sc.n; ++s)
       for (int k = 0; k < 5; ++k) {
         float ms = 0.f;
@@ -1649,13 +1657,13 @@ cudaError_t Engine::run_graph(int scheme, int latch_mode, int64_t n) {
     launches_ = per_step;  // capture launched nothing
   }
   const int64_t kernels_per_step = 7 * scheme_of(scheme).n;
-  slots_stale_ = scheme_of(scheme).n > 1 && !captured_;
   for (int64_t s = 0; s < n; ++s) {
     cudaError_t e = cudaGraphLaunch(ge, stream_);
     if (e != cudaSuccess) {
       list_valid_ = false;  // refused (a stream that is being captured): no listing ran
       return e;
     }
+    if (s == 0) note_steps(scheme_of(scheme).n);
   }
   launches_ += kernels_per_step * n;
   return cudaSuccess;
