@@ -58,6 +58,7 @@ swe_status fail(std::string* slot, swe_status st, const std::string& msg) {
 }
 
 swe_status cuda_fail(std::string* slot, cudaError_t e, const char* where) {
+  swe::consume(e);
   return fail(slot, SWE_ERR_CUDA, std::string(where) + ": " + cudaGetErrorString(e));
 }
 
@@ -122,6 +123,11 @@ __global__ void k_node_rows(const unsigned long long* key, int n, const int* __r
 // a scalar from the launch's own arguments (an 8-byte copy from pageable memory
 // goes through the copy engine)
 __global__ void k_set_value(double* p, double v) { *p = v; }
+cudaError_t set_dt(Engine& eng, double dt) {
+  const cudaError_t pending = cudaPeekAtLastError();
+  k_set_value<<<1, 1, 0, eng.stream()>>>(eng.d_fixed_dt, dt);
+  return swe::launch_error(pending);
+}
 
 swe_status read_instance(const swe_mesh* m, const swe_params* p, HostInstance* h, std::string* why) {
   if (!m || !m->geometry || !m->edge_nodes || !m->edge_cells || !m->cell_nodes || !m->cell_edges ||
@@ -527,8 +533,7 @@ swe_status swe_step(swe_ctx* ctx, int32_t scheme, double dt) {
   SWE_GUARD_BEGIN
   if (!ctx->eng.has_scheme(scheme)) return fail(&ctx->err, SWE_ERR_INVALID_ARGUMENT, kSchemeMsg);
   if (!(dt > 0.) || !std::isfinite(dt)) return fail(&ctx->err, SWE_ERR_INVALID_ARGUMENT, "dt must be positive and finite");
-  k_set_value<<<1, 1, 0, ctx->eng.stream()>>>(ctx->eng.d_fixed_dt, dt);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = set_dt(ctx->eng, dt);
   // one replay of the step's CUDA graph (captured on first use)
   if (e == cudaSuccess) e = ctx->eng.run_graph(scheme, 2, 1);
   if (e != cudaSuccess) return cuda_fail(&ctx->err, e, "swe_step");
@@ -543,8 +548,7 @@ swe_status swe_run(swe_ctx* ctx, int32_t scheme, double dt, int64_t n_steps) {
   if (!ctx->eng.has_scheme(scheme)) return fail(&ctx->err, SWE_ERR_INVALID_ARGUMENT, kSchemeMsg);
   if (!(dt > 0.) || !std::isfinite(dt)) return fail(&ctx->err, SWE_ERR_INVALID_ARGUMENT, "dt must be positive and finite");
   if (n_steps < 0) return fail(&ctx->err, SWE_ERR_INVALID_ARGUMENT, "n_steps must be >= 0");
-  k_set_value<<<1, 1, 0, ctx->eng.stream()>>>(ctx->eng.d_fixed_dt, dt);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = set_dt(ctx->eng, dt);
   if (e == cudaSuccess) e = ctx->eng.run_graph(scheme, 2, n_steps);
   if (e != cudaSuccess) return cuda_fail(&ctx->err, e, "swe_run");
   return SWE_OK;
@@ -668,9 +672,10 @@ swe_status swe_get_edge_values(swe_ctx* ctx, double* edg_out, double* src_out) {
     const size_t bytes = 6 * (size_t)g.E() * sizeof(double);
     if (e == cudaSuccess) e = cudaMemsetAsync(g.d_rows, 0, bytes, g.stream());
     if (e != cudaSuccess) return;
+    const cudaError_t pending = cudaPeekAtLastError();
     k_edge_rows<<<(n + 255) / 256, 256, 0, g.stream()>>>(g.mesh(), a, b, c, g.d_edge_caller, g.d_cell_caller,
                                                          g.d_rows);
-    e = cudaGetLastError();
+    e = swe::launch_error(pending);
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, g.d_rows, bytes, cudaMemcpyDeviceToHost, g.stream());
   };
   if (edg_out) rows(w.ew, w.eu, w.ev, edg_out);
@@ -688,9 +693,10 @@ swe_status swe_get_fluxes(swe_ctx* ctx, double* f_out) {
   const std::string why = g.field_rows();
   if (!why.empty()) return fail(&ctx->err, SWE_ERR_CUDA, why);
   const int n = g.E();
+  const cudaError_t pending = cudaPeekAtLastError();
   k_flux_rows<<<(n + 255) / 256, 256, 0, g.stream()>>>(g.work().f0, g.work().f1, g.work().f2, n, g.d_edge_caller,
                                                        g.d_rows);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = swe::launch_error(pending);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(f_out, g.d_rows, 3 * (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, g.stream());
   if (e == cudaSuccess) e = cudaStreamSynchronize(g.stream());
@@ -706,8 +712,9 @@ swe_status swe_get_node_max(swe_ctx* ctx, double* max_out) {
   const std::string why = g.field_rows();
   if (!why.empty()) return fail(&ctx->err, SWE_ERR_CUDA, why);
   const int n = g.N();
+  const cudaError_t pending = cudaPeekAtLastError();
   k_node_rows<<<(n + 255) / 256, 256, 0, g.stream()>>>(g.work().maxwp, n, g.d_node_caller, g.d_rows);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = swe::launch_error(pending);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(max_out, g.d_rows, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, g.stream());
   if (e == cudaSuccess) e = cudaStreamSynchronize(g.stream());

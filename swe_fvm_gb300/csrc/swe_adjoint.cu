@@ -900,8 +900,8 @@ struct BackwardPlan {
     return same;
   }
   void* take(size_t n) {
-    void* p = nullptr;
-    if (cudaMalloc(&p, n ? n : 1) != cudaSuccess) return nullptr;
+    char* p = nullptr;
+    if (device_alloc(&p, n) != cudaSuccess) return nullptr;
     mem.push_back(p);
     bytes += n;
     return p;
@@ -938,10 +938,10 @@ struct AdjointState {
   cudaEvent_t ev_rec[2] = {}, ev_rev[2] = {};
   template <class T>
   T* alloc(size_t n) {
-    void* p = nullptr;
-    if (cudaMalloc(&p, (n ? n : 1) * sizeof(T)) != cudaSuccess) return nullptr;
+    T* p = nullptr;
+    if (device_alloc(&p, n) != cudaSuccess) return nullptr;
     allocs.push_back(p);
-    return (T*)p;
+    return p;
   }
   int64_t dt_cap = 0, traces_cap = 0, gauges_cap = 0;
   // Room for a run's tape: arrays that are large enough stay (their addresses
@@ -953,10 +953,7 @@ struct AdjointState {
       if (p) cudaFree(p);
       p = nullptr;
       cap = 0;
-      if (cudaMalloc(&p, (n ? n : 1) * sizeof(*p)) != cudaSuccess) {
-        p = nullptr;
-        return false;
-      }
+      if (device_alloc(&p, n) != cudaSuccess) return false;
       cap = n;
       return true;
     };
@@ -966,7 +963,7 @@ struct AdjointState {
     }
     while ((int64_t)checkpoints.size() < n_ckpt) {
       double* cp = nullptr;
-      if (cudaMalloc(&cp, 3 * C * sizeof(double)) != cudaSuccess) return false;
+      if (device_alloc(&cp, 3 * C) != cudaSuccess) return false;
       checkpoints.push_back(cp);
     }
     return room(d_dt, dt_cap, n_dt) && room(d_traces, traces_cap, n_traces) && room(d_gauges, gauges_cap, n_g);
@@ -999,8 +996,9 @@ void adjoint_state_delete(AdjointState* a) { delete a; }
 // of the old bed, and so are the plane adjoints.
 cudaError_t adjoint_state_new_bed(AdjointState* a, const DevMesh& m, cudaStream_t s) {
   a->taped = false;
+  const cudaError_t pending = cudaPeekAtLastError();
   k_plane_adj_init<<<(m.C + 255) / 256, 256, 0, s>>>(m, a->aw.padj);
-  return cudaGetLastError();
+  return launch_error(pending);
 }
 
 std::string Engine::adjoint_init() {
@@ -1163,9 +1161,8 @@ std::string Engine::run_traces(int scheme, int64_t n_steps, const double* dts_ho
     if (d_tr) cudaFree(d_tr);
     if (d_g) cudaFree(d_g);
   };
-  if (cudaMalloc(&d_dts, (n_steps ? n_steps : 1) * NI * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&d_tr, (n_obs * n_gauges ? n_obs * n_gauges : 1) * sizeof(double)) != cudaSuccess ||
-      cudaMalloc(&d_g, (n_gauges ? n_gauges : 1) * sizeof(int)) != cudaSuccess) {
+  if (device_alloc(&d_dts, n_steps * NI) != cudaSuccess || device_alloc(&d_tr, n_obs * n_gauges) != cudaSuccess ||
+      device_alloc(&d_g, n_gauges) != cudaSuccess) {
     release();
     return "allocation failed";
   }

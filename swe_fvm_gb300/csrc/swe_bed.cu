@@ -277,12 +277,13 @@ __global__ void __launch_bounds__(256) k_bed_edges(DevMesh m, BedArrays o) {
 }  // namespace
 
 cudaError_t Engine::compute_bed(const double* nz_host) {
+  const cudaError_t pending = cudaPeekAtLastError();
   cudaError_t e = cudaMemcpyAsync(bed_.nz, nz_host, mesh_.N * sizeof(double), cudaMemcpyHostToDevice, stream_);
   if (e != cudaSuccess) return e;
   k_bed_cells<<<dim3((mesh_.C + 127) / 128, 9), 128, 0, stream_>>>(mesh_, bed_);
   k_bed_edges<<<(mesh_.E + 255) / 256, 256, 0, stream_>>>(mesh_, bed_);
   launches_ += 2;
-  return cudaGetLastError();
+  return launch_error(pending);
 }
 
 }  // namespace swe

@@ -27,6 +27,25 @@ constexpr int kDryStride = 8;     // doubles per dry-cell record
 
 enum : unsigned { kErrNonFinite = 1u, kErrBadState = 2u, kErrBadIndex = 4u };
 
+// Errors of the runtime.  One that a call of this library reports does not stay
+// pending in the runtime (the next call that asks for it after a launch would take
+// it for its own), and one that was pending before is neither reported nor
+// consumed where launches alone are checked: it belongs to whoever made it.
+inline cudaError_t consume(cudaError_t e) {
+  if (e != cudaSuccess && cudaPeekAtLastError() == e) cudaGetLastError();
+  return e;
+}
+// of the launches since `pending` was peeked
+inline cudaError_t launch_error(cudaError_t pending) {
+  return pending == cudaSuccess ? cudaGetLastError() : cudaSuccess;
+}
+template <class T>
+cudaError_t device_alloc(T** p, size_t n) {  // n elements; null where it fails
+  const cudaError_t e = consume(cudaMalloc((void**)p, (n ? n : 1) * sizeof(T)));
+  if (e != cudaSuccess) *p = nullptr;
+  return e;
+}
+
 // The full-wet combination records are stored combination-major, [8][C][6]:
 // the record of cell i for neighbour combination `mask` starts here.  Nearly
 // every fully-wet cell has only fully-wet neighbours (mask 0), so the records
@@ -428,6 +447,7 @@ class Engine {
                      double* nst);
   int64_t launches_ = 0;
   size_t bytes_ = 0;
+  cudaError_t alloc_error_ = cudaSuccess;  // of the last allocation that failed
   // copy of the state (3 x C) to or from buf; after a restore also zeroes the
   // accumulated time, the step dt and the error word
   cudaError_t snapshot(double* buf, bool restore);

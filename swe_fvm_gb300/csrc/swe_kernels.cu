@@ -888,12 +888,16 @@ inline int nblocks(int64_t n, int b) { return (int)((n + b - 1) / b); }
 // ------------------------------------------------------------------ engine
 template <class T>
 T* Engine::dalloc(size_t n) {
-  void* p = nullptr;
+  T* p = nullptr;
   if (n == 0) n = 1;
-  if (cudaMalloc(&p, n * sizeof(T)) != cudaSuccess) return nullptr;
+  const cudaError_t e = device_alloc(&p, n);
+  if (e != cudaSuccess) {
+    alloc_error_ = e;
+    return nullptr;
+  }
   allocs_.push_back(p);
   bytes_ += n * sizeof(T);
-  return (T*)p;
+  return p;
 }
 template int* Engine::dalloc<int>(size_t);
 template double* Engine::dalloc<double>(size_t);
@@ -1010,7 +1014,8 @@ std::string Engine::init(std::vector<HostInstance>&& inst, int flux, int ws, int
        bed_.ezm && bed_.nz;
   if (!ok) {
     *st = 6;
-    return std::string("device allocation or upload failed: ") + cudaGetErrorString(cudaGetLastError());
+    return std::string("device allocation or upload failed: ") +
+           cudaGetErrorString(alloc_error_ != cudaSuccess ? alloc_error_ : cudaGetLastError());
   }
   M.cnode = p_cnode; M.cnbr = p_cnbr; M.cedge = p_cedge; M.cinst = p_cinst; M.cown = bed_.cown;
   M.bc = bed_.bc; M.thr = bed_.thr; M.combov = bed_.combov; M.area = p_area; M.zn = bed_.zn; M.ze = bed_.ze; M.cek = p_cek;
@@ -1149,10 +1154,12 @@ void Engine::launch_partwet1(const double* W, cudaStream_t s) {
 }
 
 cudaError_t Engine::list_partwet(const double* W) {
+  const cudaError_t pending = cudaPeekAtLastError();
   cudaError_t e = cudaMemsetAsync(work_.pwcount, 0, sizeof(int), stream_);
+  if (e != cudaSuccess) return e;
   k_list_partwet<<<nblocks(mesh_.C, 256), 256, 0, stream_>>>(mesh_, work_, W, !soft_);
   ++launches_;
-  return e == cudaSuccess ? cudaGetLastError() : e;
+  return launch_error(pending);
 }
 
 cudaError_t Engine::ensure_list() {
@@ -1216,6 +1223,7 @@ cudaError_t Engine::interface_values(const double* W, const double* U, const dou
 cudaError_t Engine::refresh_slots() {
   const bool now = note_capture();
   if (!slots_stale_) return cudaSuccess;
+  const cudaError_t pending = cudaPeekAtLastError();
   // the last stage read buffer 1; the CFL ratio of its flux pass stays
   cudaError_t e = cudaMemsetAsync(work_.pwcount, 0, sizeof(int), stream_);
   if (e != cudaSuccess) return e;
@@ -1224,7 +1232,7 @@ cudaError_t Engine::refresh_slots() {
   launch_recon2(state(1, 0), state(1, 1), state(1, 2), stream_, true);
   slots_stale_ = now;
   list_valid_ = false;  // it is that buffer's now
-  return cudaGetLastError();
+  return launch_error(pending);
 }
 
 // The plugin of (flux, wave speed), given to f as a type.
@@ -1457,7 +1465,7 @@ cudaError_t Engine::autotune_blocks(int scheme) {
     }
   }
   double* save = nullptr;
-  e = cudaMalloc(&save, 3 * (size_t)mesh_.C * sizeof(double));
+  e = device_alloc(&save, 3 * (size_t)mesh_.C);
   if (e != cudaSuccess) return e;
   static const int kCand[3] = {64, 128, 256};
   const double inf = std::numeric_limits<double>::infinity();
@@ -1499,7 +1507,7 @@ cudaError_t Engine::autotune_blocks(int scheme) {
 
 cudaError_t Engine::time_steps(int scheme, int n, float* ms) {
   double* save = nullptr;
-  cudaError_t e = cudaMalloc(&save, 3 * (size_t)mesh_.C * sizeof(double));
+  cudaError_t e = device_alloc(&save, 3 * (size_t)mesh_.C);
   if (e != cudaSuccess) return e;
   cudaEvent_t a = nullptr, b = nullptr;
   e = snapshot(save, false);
@@ -1661,7 +1669,7 @@ cudaError_t Engine::run_graph(int scheme, int latch_mode, int64_t n) {
     cudaError_t e = cudaGraphLaunch(ge, stream_);
     if (e != cudaSuccess) {
       list_valid_ = false;  // refused (a stream that is being captured): no listing ran
-      return e;
+      return consume(e);
     }
     if (s == 0) note_steps(scheme_of(scheme).n);
   }
