@@ -1384,7 +1384,7 @@ std::string Engine::adjoint_backward(const double* trace_grads_host, double* gra
             // the plain stage's kernels with PartWet2 and the fluxes next to
             // partially-wet cells on the side stream, keeping every
             // intermediate (k_drain_keep leaves the node maxima and the list)
-            launch_recon1(in[0], in[1], in[2], s == 0 ? 2 : 0, true, true);
+            launch_recon1(in[0], in[1], in[2], s == 0 ? 2 : 0, true, kEveryPartWet);
             cudaEventRecord(ev_fork_, stream_);
             cudaStreamWaitEvent(side_, ev_fork_, 0);
             launch_partwet1(in[0], side_);
@@ -1524,7 +1524,7 @@ cudaError_t Engine::adjoint_stage_reverse(const Stage& st, const double* const* 
                                           AdjWork& aw) {
   // recompute the stage's forward intermediates from its input into work_
   cudaError_t e = reset_pass();
-  if (e == cudaSuccess) e = interface_values(in[0], in[1], in[2]);
+  if (e == cudaSuccess) e = interface_values(in[0], in[1], in[2], kEveryPartWet);
   if (e == cudaSuccess) e = fluxes(in[0]);
   if (e != cudaSuccess) return e;
   const int b = kReverseBlock;

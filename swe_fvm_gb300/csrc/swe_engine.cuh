@@ -311,9 +311,13 @@ class Engine {
     list_valid_ = false;
     note_capture();
   }
+  // Which partially-wet cells pass 1 appends to the list: none (the list is
+  // there), the step's (k_partwet1 and k_recon2 then share no cell with pass 1,
+  // which finishes the others), or every one (the adjoint's reverse).
+  enum List { kNoList, kStepList, kEveryPartWet };
   // Launches one reconstruction (pass 1 + pass 2) with the full interface
   // values, and one flux pass from them.
-  cudaError_t interface_values(const double* W, const double* U, const double* V);
+  cudaError_t interface_values(const double* W, const double* U, const double* V, List list = kStepList);
   cudaError_t fluxes(const double* W);
   // The full interface values as of the last reconstruction: a step of several
   // stages leaves only what its own kernels read, and the rest is written here
@@ -421,7 +425,7 @@ class Engine {
   double* d_integrals_ = nullptr;  // partial sums of the integrals
   // slots: also the full interface values (DevWork::ew ...).  latch_mode: 0
   // none, 1 the CFL dt, 2 the fixed dt, 3 none and the CFL ratio kept
-  void launch_recon1(const double* W, const double* U, const double* V, int latch_mode, bool slots, bool append);
+  void launch_recon1(const double* W, const double* U, const double* V, int latch_mode, bool slots, List list);
   void launch_partwet1(const double* W, cudaStream_t s);
   int listed_blocks() const;
   cudaError_t list_partwet(const double* W);  // empties the list and fills it from W

@@ -292,8 +292,8 @@ __global__ void __launch_bounds__(256) k_list_partwet(DevMesh m, DevWork wk, con
 
 // ---------------------------------------------------------------- kernels
 // Pass 1 but for the partly wet cells' levels (k_partwet1, beside it).  Bound by
-// its gathers.  append: list the partially-wet cells, all of them (a step's are
-// listed by the update before it).  finish: see kFinished.
+// its gathers.  append: list the partially-wet cells that are left to it (a step's
+// are listed by the update before it).  finish: see kFinished.
 // The wet test and the plane's positivity are comparisons with levels kept in
 // the mesh (DevMesh::thr, record entry 2) where the rounded sums would cost
 // seven FP64 operations; 6 are left in a fully-wet cell of 18.
@@ -685,7 +685,6 @@ __global__ void __launch_bounds__(128) k_flux_pw(DevMesh m, DevWork wk, const do
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     const int q = t / 3, k = t - 3 * q;
     const int i = gidx(wk, wk.pwlist[q], C);
-    if (!listed_class(wk.cls[i])) continue;  // (a list that pass 1 itself made has all)
     const int e = gidx(wk, m.cedge[k * C + i], m.E);
     const int o = gidx(wk, m.eown[e], C);
     if ((listed_class(wk.cls[o]) ? o : m.enb[e]) != i) continue;
@@ -1126,9 +1125,9 @@ cudaError_t Engine::reset_pass(bool list) {
 }
 
 void Engine::launch_recon1(const double* W, const double* U, const double* V, int latch_mode, bool slots,
-                           bool append) {
+                           List list) {
   const int b = blk_[0], g = nblocks(mesh_.C, b);
-  const bool finish = !append && !soft_;
+  const bool append = list != kNoList, finish = list != kEveryPartWet && !soft_;
   const int form = !slots ? kLean : cor0_ ? kSlotsCor0 : kSlotsCor;
   switch (form + (batched_ ? 3 : 0)) {
     case 0: k_recon1<false, kLean><<<g, b, 0, stream_>>>(mesh_, work_, W, U, V, latch_mode, append, finish); break;
@@ -1204,19 +1203,19 @@ cudaError_t Engine::keep_input() {
   return e;
 }
 
-cudaError_t Engine::interface_values(const double* W, const double* U, const double* V) {
+cudaError_t Engine::interface_values(const double* W, const double* U, const double* V, List list) {
   const bool now = W == state(0, 0) && note_capture();
   if (W == state(0, 0) && captured_) {
     cudaError_t e = keep_input();
     if (e != cudaSuccess) return e;
   }
-  launch_recon1(W, U, V, 0, true, true);
+  launch_recon1(W, U, V, 0, true, list);
   launch_partwet1(W, stream_);
   launch_recon2(W, U, V, stream_, true);
   k_node_max_all<<<nblocks(std::max(mesh_.N, 1), 256), 256, 0, stream_>>>(mesh_, work_, W);
   ++launches_;
   slots_stale_ = slots_stale_ && now;  // recorded only: nothing has run
-  list_valid_ = W == state(0, 0);
+  list_valid_ = W == state(0, 0) && list == kStepList;
   return cudaGetLastError();
 }
 
@@ -1227,7 +1226,7 @@ cudaError_t Engine::refresh_slots() {
   // the last stage read buffer 1; the CFL ratio of its flux pass stays
   cudaError_t e = cudaMemsetAsync(work_.pwcount, 0, sizeof(int), stream_);
   if (e != cudaSuccess) return e;
-  launch_recon1(state(1, 0), state(1, 1), state(1, 2), 3, true, true);
+  launch_recon1(state(1, 0), state(1, 1), state(1, 2), 3, true, kStepList);
   launch_partwet1(state(1, 0), stream_);
   launch_recon2(state(1, 0), state(1, 1), state(1, 2), stream_, true);
   slots_stale_ = now;
@@ -1306,7 +1305,7 @@ cudaError_t Engine::launch_stage(const Stage& st, const double* const* in, const
   if (ev) {
     // per-kernel timing: the kernels one after another
     cudaEventRecord(ev[0], stream_);
-    launch_recon1(in[0], in[1], in[2], lm, slots, false);
+    launch_recon1(in[0], in[1], in[2], lm, slots, kNoList);
     cudaEventRecord(ev[1], stream_);
     launch_partwet1(in[0], stream_);
     launch_recon2(in[0], in[1], in[2], stream_, slots);
@@ -1321,7 +1320,7 @@ cudaError_t Engine::launch_stage(const Stage& st, const double* const* in, const
     cudaEventRecord(ev_fork_, stream_);
     cudaStreamWaitEvent(side_, ev_fork_, 0);
     launch_partwet1(in[0], side_);
-    launch_recon1(in[0], in[1], in[2], lm, slots, false);
+    launch_recon1(in[0], in[1], in[2], lm, slots, kNoList);
     cudaEventRecord(ev_pass1_, stream_);
     cudaStreamWaitEvent(side_, ev_pass1_, 0);
     launch_recon2(in[0], in[1], in[2], side_, slots);
