@@ -93,7 +93,9 @@ __global__ void k_unpack(const double* __restrict__ in, double* __restrict__ W, 
 // that each is one copy to the host (host loops over five arrays of 3 C values
 // took 0.5 ms of the 0.77 ms in which a program reads all fields of 18,000 cells).
 // Row 2 e + (c < n) of edge e holds the value of its cell c towards cell n
-// (EdgeIndexer::Id, include/ValueField.h:70-75); a null component is zero.
+// (EdgeIndexer::Id, include/ValueField.h:70-75); a null component is zero, and so
+// is a null map the identity.
+__device__ __forceinline__ int caller_of(const int* __restrict__ map, int i) { return map ? map[i] : i; }
 __global__ void k_edge_rows(swe::DevMesh m, const double* a, const double* b, const double* c,
                             const int* __restrict__ edge_caller, const int* __restrict__ cell_caller,
                             double* __restrict__ out) {
@@ -101,7 +103,8 @@ __global__ void k_edge_rows(swe::DevMesh m, const double* a, const double* b, co
   if (s >= 3 * m.C) return;
   const int i = s % m.C, nb = m.cnbr[s];
   const long long row =
-      2ll * edge_caller[m.cedge[s]] + (cell_caller[i] < (nb < 0 ? nb : cell_caller[nb]) ? 1 : 0);
+      2ll * caller_of(edge_caller, m.cedge[s]) +
+      (caller_of(cell_caller, i) < (nb < 0 ? nb : caller_of(cell_caller, nb)) ? 1 : 0);
   out[3 * row] = a ? a[s] : 0.;
   out[3 * row + 1] = b[s];
   out[3 * row + 2] = c[s];
@@ -110,7 +113,7 @@ __global__ void k_flux_rows(const double* a, const double* b, const double* c, i
                             const int* __restrict__ edge_caller, double* __restrict__ out) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n) return;
-  const long long r = 3ll * edge_caller[e];
+  const long long r = 3ll * caller_of(edge_caller, e);
   out[r] = a[e];
   out[r + 1] = b[e];
   out[r + 2] = c[e];
@@ -118,7 +121,7 @@ __global__ void k_flux_rows(const double* a, const double* b, const double* c, i
 __global__ void k_node_rows(const unsigned long long* key, int n, const int* __restrict__ node_caller,
                             double* __restrict__ out) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q < n) out[node_caller[q]] = swe::order_val(key[q]);
+  if (q < n) out[caller_of(node_caller, q)] = swe::order_val(key[q]);
 }
 // a scalar from the launch's own arguments (an 8-byte copy from pageable memory
 // goes through the copy engine)
@@ -666,8 +669,6 @@ swe_status swe_get_edge_values(swe_ctx* ctx, double* edg_out, double* src_out) {
   const swe::DevWork& w = g.work();
   const int n = 3 * g.C();
   cudaError_t e = g.refresh_slots();
-  std::string why = e == cudaSuccess ? g.field_rows() : std::string();
-  if (!why.empty()) return fail(&ctx->err, SWE_ERR_CUDA, why);
   auto rows = [&](const double* a, const double* b, const double* c, double* out) {
     const size_t bytes = 6 * (size_t)g.E() * sizeof(double);
     if (e == cudaSuccess) e = cudaMemsetAsync(g.d_rows, 0, bytes, g.stream());
@@ -690,8 +691,6 @@ swe_status swe_get_fluxes(swe_ctx* ctx, double* f_out) {
   if (!ctx || !f_out) return SWE_ERR_INVALID_ARGUMENT;
   SWE_GUARD_BEGIN
   Engine& g = ctx->eng;
-  const std::string why = g.field_rows();
-  if (!why.empty()) return fail(&ctx->err, SWE_ERR_CUDA, why);
   const int n = g.E();
   const cudaError_t pending = cudaPeekAtLastError();
   k_flux_rows<<<(n + 255) / 256, 256, 0, g.stream()>>>(g.work().f0, g.work().f1, g.work().f2, n, g.d_edge_caller,
@@ -709,8 +708,6 @@ swe_status swe_get_node_max(swe_ctx* ctx, double* max_out) {
   if (!ctx || !max_out) return SWE_ERR_INVALID_ARGUMENT;
   SWE_GUARD_BEGIN
   Engine& g = ctx->eng;
-  const std::string why = g.field_rows();
-  if (!why.empty()) return fail(&ctx->err, SWE_ERR_CUDA, why);
   const int n = g.N();
   const cudaError_t pending = cudaPeekAtLastError();
   k_node_rows<<<(n + 255) / 256, 256, 0, g.stream()>>>(g.work().maxwp, n, g.d_node_caller, g.d_rows);

@@ -1200,13 +1200,9 @@ std::string Engine::caller_maps() {
     for (int64_t j = 0; j < node_off[q + 1] - node_off[q]; ++j)
       nm[node_off[q] + j] = (int)(node_off[q] + (id ? j : L->node_from[j]));
   }
-  d_cell_caller = dalloc<int>(cm.size());
-  d_node_caller = dalloc<int>(nm.size());
-  if (!d_cell_caller || !d_node_caller) return "device allocation failed";
-  if (cudaMemcpy(d_cell_caller, cm.data(), cm.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(d_node_caller, nm.data(), nm.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
-    return std::string("uploading the caller order: ") + cudaGetErrorString(cudaGetLastError());
-  return "";
+  std::string e = d_cell_caller ? "" : upload_map(cm, &d_cell_caller);
+  if (e.empty() && !d_node_caller) e = upload_map(nm, &d_node_caller);
+  return e;
 }
 
 std::string Engine::adjoint_dts(double* out_host) {

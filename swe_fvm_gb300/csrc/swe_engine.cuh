@@ -387,26 +387,28 @@ class Engine {
   std::vector<int64_t> cell_off, edge_off, node_off;
   // Host copies of the per-instance topology needed by the layout getters.
   std::vector<HostInstance> host;
-  // global device cell / node position -> global caller index, built on first
-  // use by the device-memory adjoint outputs
+  // global device cell / node position -> global caller index: a context in
+  // another order has them for its field getters, with the edges' (null there: the
+  // caller's order); the device-memory adjoint outputs build theirs on first use
   int* d_cell_caller = nullptr;
   int* d_node_caller = nullptr;
+  int* d_edge_caller = nullptr;
   std::string caller_maps();
+  // max(6 E, N) doubles or more: the field getters' rows, and, at other times, the
+  // arrays that live inside one stage or one call (DevWork::eh, gx, gy, drain and
+  // pwrec, and d_io)
+  double* d_rows = nullptr;
   double* d_io = nullptr;        // [3C] staging buffer for the interleaved 3 x C field
   unsigned* d_ioflag = nullptr;  // non-finite flag of the last upload
   double* d_fixed_dt = nullptr;  // [I] device dt of fixed-step runs
   unsigned long long* h_word = nullptr;  // pinned host word for scalars read back
-  // device edge -> the caller's edge (one instance), and a staging buffer of
-  // max(6 E, N) doubles for the field getters; made by the first of them
-  int* d_edge_caller = nullptr;
-  double* d_rows = nullptr;
-  std::string field_rows();
 
  private:
   cudaError_t launch_stage(const Stage& st, const double* const* in, const double* const* u0, double* const* out,
                            bool first_stage_of_step, int latch_mode, bool full = false, cudaEvent_t* ev = nullptr);
   template <class T>
   T* dalloc(size_t n);
+  std::string upload_map(const std::vector<int>& h, int** d);
 
   DevMesh mesh_{};
   DevWork work_{};

@@ -1026,15 +1026,20 @@ std::string Engine::init(std::vector<HostInstance>&& inst, int flux, int ws, int
   M.nptr = p_nptr; M.ncell = p_ncell;
 
   DevWork& Wk = work_;
-  Wk.eh = dalloc<double>(3 * C); Wk.gx = dalloc<double>(C); Wk.gy = dalloc<double>(C);
+  // What lives inside one stage or one call shares an allocation, in which the
+  // field getters lay out their rows: they need no memory of their own.
+  const size_t part = ((size_t)C + 31) / 32 * 32;  // 256-byte steps
+  d_rows = dalloc<double>(std::max({10 * part, 6 * (size_t)E, (size_t)N}));
+  if (d_rows) {
+    Wk.eh = d_rows; Wk.gx = d_rows + 3 * part; Wk.gy = d_rows + 4 * part;
+    Wk.drain = d_rows + 5 * part; Wk.pwrec = d_rows + 6 * part; d_io = d_rows + 7 * part;
+  }
   Wk.ew = dalloc<double>(3 * C); Wk.eu = dalloc<double>(3 * C); Wk.ev = dalloc<double>(3 * C);
   Wk.sx = dalloc<double>(3 * C); Wk.sy = dalloc<double>(3 * C);
   Wk.f0 = dalloc<double>(E); Wk.f1 = dalloc<double>(E); Wk.f2 = dalloc<double>(E);
-  Wk.drain = dalloc<double>(C);
   Wk.maxwp = dalloc<unsigned long long>(N);
   Wk.pwlist = dalloc<int>(C);
   Wk.pwcount = dalloc<int>(1);
-  Wk.pwrec = dalloc<double>(C);
   Wk.cls = dalloc<unsigned char>(C);
   Wk.ftape = nullptr;
   Wk.r = dalloc<unsigned long long>(I);
@@ -1045,11 +1050,10 @@ std::string Engine::init(std::vector<HostInstance>&& inst, int flux, int ws, int
   Wk.err = dalloc<unsigned>(1);
   M.err = Wk.err;
   for (int q = 0; q < 6; ++q) state_[q] = dalloc<double>(C);
-  d_io = dalloc<double>(3 * C);
   d_ioflag = dalloc<unsigned>(1);
-  if (!Wk.eh || !Wk.gx || !Wk.gy || !Wk.ew || !Wk.eu || !Wk.ev || !Wk.sx || !Wk.sy || !Wk.f0 || !Wk.f1 || !Wk.f2 || !Wk.drain || !Wk.maxwp ||
-      !Wk.pwlist || !Wk.pwcount || !Wk.pwrec || !Wk.cls || !Wk.r || !Wk.dt || !Wk.tsum || !d_fixed_dt || !Wk.err ||
-      !state_[5] || !d_io || !d_ioflag) {
+  if (!d_rows || !Wk.ew || !Wk.eu || !Wk.ev || !Wk.sx || !Wk.sy || !Wk.f0 || !Wk.f1 || !Wk.f2 || !Wk.maxwp ||
+      !Wk.pwlist || !Wk.pwcount || !Wk.cls || !Wk.r || !Wk.dt || !Wk.tsum || !d_fixed_dt || !Wk.err ||
+      !state_[5] || !d_ioflag) {
     *st = 6;
     return "device allocation failed";
   }
@@ -1097,25 +1101,6 @@ std::string Engine::init(std::vector<HostInstance>&& inst, int flux, int ws, int
     return std::string("CUDA error during set-up: ") + cudaGetErrorString(ce);
   }
   return "";
-}
-
-std::string Engine::field_rows() {
-  if (d_rows) return "";
-  std::string e = caller_maps();
-  if (!e.empty()) return e;
-  std::vector<int> em((size_t)mesh_.E);
-  for (size_t q = 0; q < host.size(); ++q) {
-    const Layout* L = q < layouts.size() ? &layouts[q] : nullptr;
-    const bool id = !L || L->identity();
-    for (int64_t j = 0; j < edge_off[q + 1] - edge_off[q]; ++j)
-      em[edge_off[q] + j] = (int)(edge_off[q] + (id ? j : L->edge_from[j]));
-  }
-  if (!d_edge_caller) d_edge_caller = dalloc<int>(em.size());
-  if (!d_edge_caller) return "device allocation failed";
-  if (cudaMemcpy(d_edge_caller, em.data(), em.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
-    return std::string("uploading the caller order: ") + cudaGetErrorString(cudaGetLastError());
-  d_rows = dalloc<double>(std::max(6 * (size_t)mesh_.E, (size_t)mesh_.N));
-  return d_rows ? "" : "device allocation failed";
 }
 
 cudaError_t Engine::reset_pass(bool list) {
@@ -1550,6 +1535,21 @@ std::string Engine::set_layouts(std::vector<Layout>&& lay) {
   if (cudaMemcpy(d_cell_from, from.data(), from.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(d_cell_to, to.data(), to.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
     return std::string("uploading the cell layout: ") + cudaGetErrorString(cudaGetLastError());
+  if (batched_) return "";
+  // a context's field getters renumber edges and nodes too
+  auto ints = [](const std::vector<int64_t>& v) { return std::vector<int>(v.begin(), v.end()); };
+  std::string e = upload_map(ints(layouts[0].edge_from), &d_edge_caller);
+  if (e.empty()) e = upload_map(ints(layouts[0].node_from), &d_node_caller);
+  d_cell_caller = d_cell_from;
+  return e;
+}
+
+std::string Engine::upload_map(const std::vector<int>& h, int** d) {
+  int* p = dalloc<int>(h.size());
+  if (!p) return "device allocation failed";
+  const cudaError_t e = consume(cudaMemcpy(p, h.data(), h.size() * sizeof(int), cudaMemcpyHostToDevice));
+  if (e != cudaSuccess) return std::string("uploading the caller order: ") + cudaGetErrorString(e);
+  *d = p;
   return "";
 }
 
