@@ -869,7 +869,8 @@ __global__ void __launch_bounds__(32) k_pw_jacobian(DevMesh m, DevWork wk, AdjWo
 // stores and kept intermediates, and the captured graphs of a full segment's
 // recompute and reverse.  It is kept for the next backward pass of the same shape
 // (an inversion repeats one) up to kPlanBytes, else given back at once: allocating
-// and capturing it again took 2 ms of the 8 ms of a 20k-cell pass.
+// and capturing it again took 2 ms of the 8 ms of a 20k-cell pass.  A plan that the
+// device had too little memory for is given back too.
 constexpr size_t kPlanBytes = size_t(1) << 30;
 struct BackwardPlan {
   // the shape it was made for, and the tape's arrays its graphs read
@@ -1501,7 +1502,10 @@ std::string Engine::adjoint_backward(const double* trace_grads_host, double* gra
     if (e != cudaSuccess) err = std::string("adjoint: ") + cudaGetErrorString(e);
   }
   cudaMemcpy(work_.tsum, tsum_saved.data(), I() * sizeof(double), cudaMemcpyHostToDevice);
-  if (plan.bytes > kPlanBytes || !err.empty()) {
+  // kept for the next pass, unless it is large or what it could hold was decided by
+  // a lack of memory: the next pass looks again
+  const bool short_of_memory = !plan.keep || (plan.sets == 1 && nseg > 1);
+  if (plan.bytes > kPlanBytes || short_of_memory || !err.empty()) {
     cudaStreamSynchronize(stream_);
     plan.release();
   }

@@ -1,0 +1,49 @@
+"""The backward pass where the segment's intermediates do not fit (the stage by
+stage reverse), and that each pass decides by the memory there is then."""
+import numpy as np
+import pytest
+
+from swe_fvm_gb300 import scenarios
+from swe_fvm_gb300.adjoint import Rollout
+
+pytestmark = pytest.mark.gpu
+
+
+def backward(ro, prim, gauges, segment):
+    """Gradients of one pass, and the launches it took (nothing is replayed: no segment is full)."""
+    ro.sd.SetVolField(prim)
+    ro.sd.prime()
+    tr = ro.forward(1, 6, segment, gauges, 2)
+    n = ro.sd.launch_count()
+    g = ro.backward(np.cos(np.arange(tr.size)).reshape(tr.shape))
+    return g, ro.sd.launch_count() - n
+
+
+def alike(a, b):
+    # (node sums are atomic: their order varies by rounding)
+    return all(np.allclose(x, y, rtol=1e-9, atol=1e-11 * np.abs(y).max()) for x, y in zip(a, b))
+
+
+def test_each_pass_decides_by_the_memory_there_is(gpu):
+    import torch
+
+    m, prim = scenarios.sloped_bump_case(101, 3)
+    gauges = np.random.default_rng(0).integers(0, m.num_cells, 5)
+    C, ns = m.num_cells, 2
+    # a segment whose stage inputs (24 B a cell) are under the 1 GiB that is kept
+    # between passes and whose intermediates (about 290 B a cell) are not
+    segment = int(0.9 * 2 ** 30 / (24 * C * ns))
+    base, plain = Rollout(m, prim), Rollout(m, prim)
+    want, n_kept = backward(plain, prim, gauges, segment)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    leave = 16 << 30  # most of the device stands for other programs' data; untouched, and far from all of it
+    hold = torch.empty(max(free - leave, 1), dtype=torch.uint8, device="cuda")
+    got, n_staged = backward(base, prim, gauges, segment)
+    assert alike(got, want)
+    assert n_staged != n_kept
+    del hold
+    torch.cuda.empty_cache()
+    got, n = backward(base, prim, gauges, segment)
+    assert n == n_kept
+    assert alike(got, want)
