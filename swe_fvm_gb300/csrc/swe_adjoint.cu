@@ -875,8 +875,8 @@ constexpr size_t kPlanBytes = size_t(1) << 30;
 struct BackwardPlan {
   // the shape it was made for, and the tape's arrays its graphs read
   Scheme sc{};
-  int64_t K = 0, nseg = 0, obs = 0;
-  int n_gauges = 0, n_tg = 0;
+  int64_t K = 0, nseg = 0, obs = 0, n_tg = 0;
+  int n_gauges = 0;
   const void *d_dt = nullptr, *d_gauges = nullptr;
   double reg_depth = 0.;
   // what it holds
@@ -1318,7 +1318,7 @@ std::string Engine::adjoint_backward(const double* trace_grads_host, double* gra
     want.nseg = nseg;
     want.obs = a.obs;
     want.n_gauges = a.n_gauges;
-    want.n_tg = (int)(n_obs * a.n_gauges);
+    want.n_tg = n_obs * a.n_gauges;
     want.d_dt = a.d_dt;
     want.d_gauges = a.d_gauges;
     want.reg_depth = adj_reg_depth_;

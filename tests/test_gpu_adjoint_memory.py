@@ -1,9 +1,12 @@
 """The backward pass where the segment's intermediates do not fit (the stage by
-stage reverse), and that each pass decides by the memory there is then."""
+stage reverse), that each pass decides by the memory there is then, and traces of
+more than 2^31 values."""
+import ctypes
+
 import numpy as np
 import pytest
 
-from swe_fvm_gb300 import scenarios
+from swe_fvm_gb300 import _lib, scenarios
 from swe_fvm_gb300.adjoint import Rollout
 
 pytestmark = pytest.mark.gpu
@@ -47,3 +50,30 @@ def test_each_pass_decides_by_the_memory_there_is(gpu):
     got, n = backward(base, prim, gauges, segment)
     assert n == n_kept
     assert alike(got, want)
+
+
+def test_large_traces(gpu):
+    """More trace values than an int counts."""
+    import torch
+
+    m, prim = scenarios.sloped_bump_case(101, 3)
+    L = _lib.load()
+    n_gauges, n_obs, last = 1 << 27, 17, 7777
+    cells = np.arange(n_gauges, dtype=np.int64) % m.num_cells
+    cells[-1] = last
+    ro, small = Rollout(m, prim), Rollout(m, prim)
+    traces = torch.empty((n_obs, n_gauges), dtype=torch.float64, device="cuda")
+    ro.sd._check(L.swe_adjoint_forward_device(ro.sd.ctx, 1, n_obs, 4, n_gauges, cells.ctypes.data, 1,
+                                              ctypes.c_void_p(traces.data_ptr())))
+    want = small.forward(1, n_obs, 4, np.array([last]), 1)
+    assert np.array_equal(traces[:, -1].cpu().numpy(), want[:, 0])
+    weights = np.cos(np.arange(n_obs))
+    grads = traces.zero_()
+    grads[:, -1] = torch.as_tensor(weights, device="cuda")
+    torch.cuda.synchronize()
+    gp = torch.empty((m.num_cells, 3), dtype=torch.float64, device="cuda")
+    gz = torch.empty((m.num_nodes,), dtype=torch.float64, device="cuda")
+    ro.sd._check(L.swe_adjoint_backward_device(ro.sd.ctx, ctypes.c_void_p(grads.data_ptr()),
+                                               ctypes.c_void_p(gp.data_ptr()), ctypes.c_void_p(gz.data_ptr())))
+    ro.sd.synchronize()
+    assert alike((gp.cpu().numpy(), gz.cpu().numpy()), small.backward(weights[:, None]))
