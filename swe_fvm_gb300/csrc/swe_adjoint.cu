@@ -870,7 +870,8 @@ __global__ void __launch_bounds__(32) k_pw_jacobian(DevMesh m, DevWork wk, AdjWo
 // recompute and reverse.  It is kept for the next backward pass of the same shape
 // (an inversion repeats one) up to kPlanBytes, else given back at once: allocating
 // and capturing it again took 2 ms of the 8 ms of a 20k-cell pass.  A plan that the
-// device had too little memory for is given back too.
+// device had too little memory for is given back too, and a kept one when a tape
+// does not fit beside it.
 constexpr size_t kPlanBytes = size_t(1) << 30;
 struct BackwardPlan {
   // the shape it was made for, and the tape's arrays its graphs read
@@ -1122,7 +1123,13 @@ std::string Engine::adjoint_forward(int scheme, int64_t n_steps, int64_t ckpt, c
   const int64_t NI = I();
   // every checkpoint allocated up front (no allocation inside the run)
   const int64_t n_ckpt = n_steps > 0 ? (n_steps + ckpt - 1) / ckpt : 0;
-  if (!a.reserve_tape(n_steps * NI, n_obs * n_gauges, n_gauges, n_ckpt, C)) return "tape allocation failed";
+  auto reserve = [&] { return a.reserve_tape(n_steps * NI, n_obs * n_gauges, n_gauges, n_ckpt, C); };
+  if (!reserve()) {
+    // once more without what the last backward pass kept
+    cudaStreamSynchronize(stream_);
+    a.plan.release();
+    if (!reserve()) return "tape allocation failed";
+  }
   cudaMemcpyAsync(a.d_gauges, gauges, n_gauges * sizeof(int), cudaMemcpyHostToDevice, stream_);
   for (int64_t n = 0; n < n_steps; ++n) {
     if (n % ckpt == 0) {

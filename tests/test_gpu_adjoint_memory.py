@@ -1,6 +1,6 @@
 """The backward pass where the segment's intermediates do not fit (the stage by
-stage reverse), that each pass decides by the memory there is then, and traces of
-more than 2^31 values."""
+stage reverse), that each pass decides by the memory there is then, that a tape
+may take what a pass kept, and traces of more than 2^31 values."""
 import ctypes
 
 import numpy as np
@@ -53,7 +53,8 @@ def test_each_pass_decides_by_the_memory_there_is(gpu):
 
 
 def test_large_traces(gpu):
-    """More trace values than an int counts."""
+    """More trace values than an int counts, and a tape that fits beside the rest
+    only without the workspace that a backward pass kept."""
     import torch
 
     m, prim = scenarios.sloped_bump_case(101, 3)
@@ -62,9 +63,21 @@ def test_large_traces(gpu):
     cells = np.arange(n_gauges, dtype=np.int64) % m.num_cells
     cells[-1] = last
     ro, small = Rollout(m, prim), Rollout(m, prim)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    ro.backward(np.ones_like(ro.forward(1, 40, 20, cells[:4], 10)))
+    ro.sd.SetVolField(prim)
+    ro.sd.prime()
+    torch.cuda.synchronize()
+    kept = free - torch.cuda.mem_get_info()[0]
+    assert 2 ** 28 < kept < 2 ** 30
     traces = torch.empty((n_obs, n_gauges), dtype=torch.float64, device="cuda")
+    tape = traces.numel() * 8 + n_gauges * 4
+    hold = torch.empty(max(torch.cuda.mem_get_info()[0] - tape + kept // 2, 1), dtype=torch.uint8, device="cuda")
     ro.sd._check(L.swe_adjoint_forward_device(ro.sd.ctx, 1, n_obs, 4, n_gauges, cells.ctypes.data, 1,
                                               ctypes.c_void_p(traces.data_ptr())))
+    del hold
+    torch.cuda.empty_cache()
     want = small.forward(1, n_obs, 4, np.array([last]), 1)
     assert np.array_equal(traces[:, -1].cpu().numpy(), want[:, 0])
     weights = np.cos(np.arange(n_obs))
