@@ -95,7 +95,9 @@ __global__ void k_unpack(const double* __restrict__ in, double* __restrict__ W, 
 // Row 2 e + (c < n) of edge e holds the value of its cell c towards cell n
 // (EdgeIndexer::Id, include/ValueField.h:70-75); a null component is zero, and so
 // is a null map the identity.
-__device__ __forceinline__ int caller_of(const int* __restrict__ map, int i) { return map ? map[i] : i; }
+__device__ __forceinline__ int caller_of(const swe::DevMesh& m, const int* __restrict__ map, int i, int n) {
+  return map ? swe::gidx(m, map[swe::gidx(m, i, n)], n) : swe::gidx(m, i, n);
+}
 __global__ void k_edge_rows(swe::DevMesh m, const double* a, const double* b, const double* c,
                             const int* __restrict__ edge_caller, const int* __restrict__ cell_caller,
                             double* __restrict__ out) {
@@ -103,25 +105,25 @@ __global__ void k_edge_rows(swe::DevMesh m, const double* a, const double* b, co
   if (s >= 3 * m.C) return;
   const int i = s % m.C, nb = m.cnbr[s];
   const long long row =
-      2ll * caller_of(edge_caller, m.cedge[s]) +
-      (caller_of(cell_caller, i) < (nb < 0 ? nb : caller_of(cell_caller, nb)) ? 1 : 0);
+      2ll * caller_of(m, edge_caller, m.cedge[s], m.E) +
+      (caller_of(m, cell_caller, i, m.C) < (nb < 0 ? nb : caller_of(m, cell_caller, nb, m.C)) ? 1 : 0);
   out[3 * row] = a ? a[s] : 0.;
   out[3 * row + 1] = b[s];
   out[3 * row + 2] = c[s];
 }
-__global__ void k_flux_rows(const double* a, const double* b, const double* c, int n,
+__global__ void k_flux_rows(swe::DevMesh m, const double* a, const double* b, const double* c,
                             const int* __restrict__ edge_caller, double* __restrict__ out) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n) return;
-  const long long r = 3ll * caller_of(edge_caller, e);
+  if (e >= m.E) return;
+  const long long r = 3ll * caller_of(m, edge_caller, e, m.E);
   out[r] = a[e];
   out[r + 1] = b[e];
   out[r + 2] = c[e];
 }
-__global__ void k_node_rows(const unsigned long long* key, int n, const int* __restrict__ node_caller,
+__global__ void k_node_rows(swe::DevMesh m, const unsigned long long* key, const int* __restrict__ node_caller,
                             double* __restrict__ out) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q < n) out[caller_of(node_caller, q)] = swe::order_val(key[q]);
+  if (q < m.N) out[caller_of(m, node_caller, q, m.N)] = swe::order_val(key[q]);
 }
 // a scalar from the launch's own arguments (an 8-byte copy from pageable memory
 // goes through the copy engine)
@@ -693,8 +695,8 @@ swe_status swe_get_fluxes(swe_ctx* ctx, double* f_out) {
   Engine& g = ctx->eng;
   const int n = g.E();
   const cudaError_t pending = cudaPeekAtLastError();
-  k_flux_rows<<<(n + 255) / 256, 256, 0, g.stream()>>>(g.work().f0, g.work().f1, g.work().f2, n, g.d_edge_caller,
-                                                       g.d_rows);
+  k_flux_rows<<<(n + 255) / 256, 256, 0, g.stream()>>>(g.mesh(), g.work().f0, g.work().f1, g.work().f2,
+                                                       g.d_edge_caller, g.d_rows);
   cudaError_t e = swe::launch_error(pending);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(f_out, g.d_rows, 3 * (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, g.stream());
@@ -710,7 +712,7 @@ swe_status swe_get_node_max(swe_ctx* ctx, double* max_out) {
   Engine& g = ctx->eng;
   const int n = g.N();
   const cudaError_t pending = cudaPeekAtLastError();
-  k_node_rows<<<(n + 255) / 256, 256, 0, g.stream()>>>(g.work().maxwp, n, g.d_node_caller, g.d_rows);
+  k_node_rows<<<(n + 255) / 256, 256, 0, g.stream()>>>(g.mesh(), g.work().maxwp, g.d_node_caller, g.d_rows);
   cudaError_t e = swe::launch_error(pending);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(max_out, g.d_rows, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, g.stream());

@@ -26,7 +26,8 @@ struct P3 {
   __device__ double operator[](int r) const { return v[r]; }
 };
 
-__device__ __forceinline__ P3 node(const DevMesh& m, int n) {
+__device__ __forceinline__ P3 node(const DevMesh& m, int id) {
+  const int n = gidx(m, id, m.N);
   const double2 p = m.nxy[n];
   return P3{{p.x, p.y, m.nz[n]}};
 }
@@ -40,7 +41,7 @@ __device__ __forceinline__ P3 centroid(const P3& a, const P3& b, const P3& c) {
 }
 // edge centre = midpoint of the edge's nodes (Domain::E is a stub in the reference)
 __device__ __forceinline__ P3 midpoint_of(const DevMesh& m, int e) {
-  const int2 n = m.enode[e];
+  const int2 n = m.enode[gidx(m, e, m.E)];
   const P3 a = node(m, n.x), b = node(m, n.y);
   P3 t;
 #pragma unroll
@@ -108,7 +109,7 @@ __device__ void plane_record(const DevMesh& m, int i, int mask, double* rec, dou
   }
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const int j = m.cnbr[k * C + i];
+    const int j = gidx(m, m.cnbr[k * C + i], C);
     if (mask >> k & 1) Q[k] = E[k];
     else Q[k] = centroid(node(m, m.cnode[j]), node(m, m.cnode[C + j]), node(m, m.cnode[2 * C + j]));
   }
@@ -269,7 +270,7 @@ __global__ void __launch_bounds__(256) k_bed_edges(DevMesh m, BedArrays o) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= m.E) return;
   const int2 n = m.enode[e];
-  const double z = (m.nz[n.x] + m.nz[n.y]) * 0.5;
+  const double z = (m.nz[gidx(m, n.x, m.N)] + m.nz[gidx(m, n.y, m.N)]) * 0.5;
   o.ezm[e] = z;
   o.erec[e].b = z;
 }
