@@ -375,7 +375,7 @@ def run_gpu(args):
     _lib.check(L.swe_measure_fp64_peak(ctypes.byref(fp64)))
     hbm, src = peaks()
     achieved = BYTES_PER_CELL_STEP * C / (ms_step * 1e-3) / 1e9
-    roof = {"bound": "hbm", "kernel": "ssprk2_step (one CUDA graph: 2 stages x 6 kernels on two streams)",
+    roof = {"bound": "hbm", "kernel": "ssprk2_step (one CUDA graph: 2 stages x 7 kernels on two streams)",
             "achieved": achieved,
             "peak": hbm, "unit": "GB/s", "frac": achieved / hbm, "peak_source": src,
             "algorithmic_bytes_per_launch": BYTES_PER_CELL_STEP * C,

@@ -112,7 +112,8 @@ typedef struct swe_batch swe_batch;
 swe_status swe_params_default(swe_params* p);
 
 /* Builds a context: validates and copies the mesh, precomputes the static
- * geometry on the host, uploads it and the initial primitive state (3 x C).
+ * geometry (on the host what the plan positions give, on the device what the bed
+ * enters) and uploads the initial primitive state (3 x C).
  * Replaces Topology(...) + Domain(...) + SpaceDisc(fluxer, domain, v0, cor, tau)
  * + TimeDisc(&sd) (include/TriangMesh.h:27-40, src/Bathymetry.cpp:6-8,
  * src/SpaceDisc.cpp:4-13, include/TimeDisc.h:6-7). */
@@ -318,9 +319,11 @@ swe_status swe_adjoint_dts(swe_ctx* ctx, double* dts_out);
  * of the discrete forward.  Takes effect at the next backward. */
 swe_status swe_adjoint_set_regularisation(swe_ctx* ctx, double depth);
 /* Builds the adjoint's one-time tables and work arrays (the cells around each
- * node, the twin slots of each edge, the plane-point adjoints of every cell;
- * built from the bed, so swe_set_bathymetry drops them) ahead of the first
- * taped run, which otherwise builds them itself.  No reference counterpart. */
+ * node, the twin slots of each edge, the plane-point adjoints of every cell)
+ * ahead of the first taped run, which otherwise builds them itself.  They stay
+ * with the context; swe_set_bathymetry rewrites those that the bed enters.  The
+ * tape's arrays and up to 1 GiB of a backward pass's workspace stay too, for the
+ * next run of the same shape.  No reference counterpart. */
 swe_status swe_adjoint_prepare(swe_ctx* ctx);
 /* swe_adjoint_forward / swe_adjoint_backward with every array in device memory
  * (gauge_cells stays on the host): traces_out, trace_grads, grad_prim0 (3 x C
@@ -340,12 +343,13 @@ swe_status swe_adjoint_backward_device(swe_ctx* ctx, const double* trace_grads, 
 swe_status swe_run_traces(swe_ctx* ctx, int32_t scheme, int64_t n_steps, const double* dts, int32_t n_gauges,
                           const int64_t* gauge_cells, int64_t obs_every, double* traces_out);
 /* Replaces the node bathymetry (N values, the caller's node order, host) of a
- * context: every mesh record that depends on it is recomputed with the
- * reference's operation order and re-uploaded in place (device order, tuning
- * and captured graphs kept); the state is kept and the adjoint's tape is
- * dropped.  The reference's geometry is a caller array (include/Bathymetry.h:
- * 42-43), so writing its z row and stepping again is the reference-side
- * equivalent.  Call swe_prime afterwards for a CFLdt() of the new bed. */
+ * context: every mesh record that depends on it is recomputed on the device
+ * with the reference's operation order, in place (device order, tuning and
+ * captured graphs kept); the state and the interface values of the last
+ * reconstruction are kept and the adjoint's tape is dropped.  The reference's
+ * geometry is a caller array (include/Bathymetry.h:42-43), so writing its z row
+ * and stepping again is the reference-side equivalent.  Call swe_prime
+ * afterwards for a CFLdt() of the new bed. */
 swe_status swe_set_bathymetry(swe_ctx* ctx, const double* z);
 /* Recomputes the flux pass of the current state (SpaceDisc::
  * ComputeInterfaceValues + ComputeFluxes, src/SpaceDisc.cpp:33-74) so that
@@ -421,7 +425,7 @@ swe_status swe_batch_adjoint_backward_device(swe_batch* b, const double* trace_g
 swe_status swe_batch_run_traces(swe_batch* b, int32_t scheme, int64_t n_steps, const double* dts, int32_t n_gauges,
                                 const int64_t* gauge_cells, int64_t obs_every, double* traces_out);
 /* swe_set_bathymetry for a batch: z[q] (N_q values, host) for every instance
- * whose bed changes, NULL for the others; one recompute and re-upload. */
+ * whose bed changes, NULL for the others; one recompute. */
 swe_status swe_batch_set_bathymetry(swe_batch* b, const double* const* z);
 /* swe_prime for every instance of a batch. */
 swe_status swe_batch_prime(swe_batch* b);

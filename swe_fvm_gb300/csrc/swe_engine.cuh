@@ -6,8 +6,9 @@
 //   "slot" (i, k) = interface value of cell i on its local edge k, stored at
 //   k * C + i, so a warp writes and reads its own cells' slots coalesced.
 // Static per-cell records hold every quantity of the reference step that
-// depends on the mesh alone (precomputed once on the host with the reference's
-// operation order); the kernels do only state-dependent arithmetic.
+// depends on the mesh alone, evaluated once with the reference's operation order:
+// on the host what only the plan positions enter, on the device what the bed enters
+// (again for every new bed); the kernels do only state-dependent arithmetic.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -283,8 +284,8 @@ class Engine {
   // Replaces the node bathymetry of the instances whose pointer is not null
   // (each in the caller's node order, N_q values) and recomputes the mesh
   // records that depend on it on the device, in the same buffers (the captured
-  // step graphs stay valid); drops the adjoint's tape.  The state is kept; the
-  // caller re-primes the flux pass.
+  // step graphs stay valid); drops the adjoint's tape.  The state and the
+  // interface values are kept; the caller re-primes the flux pass.
   std::string set_bathymetry(const std::vector<const double*>& z);
   // Mean ms of one graph-replayed step of `scheme` (CFL dt) over n steps after
   // one warm-up replay, run from the current state, which is then restored
@@ -301,9 +302,9 @@ class Engine {
   void set_stream(cudaStream_t s);
   cudaStream_t stream() const { return stream_; }
 
-  // Resets the node maxima and the part-wet list (done by k_drain at the end
-  // of every stage; needed before a standalone reconstruction).
-  // list: the part-wet list too.
+  // Resets the node maxima and, with list, the part-wet list, before a standalone
+  // reconstruction.  (In a step k_drain empties the list at the end of every stage;
+  // the node maxima that PartWet2 reads are written by each stage.)
   cudaError_t reset_pass(bool list = true);
   // The state in buffer 0 was written from outside: its part-wet list is to be
   // made before the next step (a step leaves the next one's).
@@ -319,9 +320,9 @@ class Engine {
   // values, and one flux pass from them.
   cudaError_t interface_values(const double* W, const double* U, const double* V, List list = kStepList);
   cudaError_t fluxes(const double* W);
-  // The full interface values as of the last reconstruction: a step of several
-  // stages leaves only what its own kernels read, and the rest is written here
-  // from the last stage's input, which the step keeps.
+  // The full interface values as of the last reconstruction: the last of several
+  // stages leaves only what the step's own kernels read, and the rest is written
+  // here from its input, which the step keeps.
   cudaError_t refresh_slots();
   // One whole step of `scheme`; latch_mode 1 = CFL dt, 2 = fixed dt from
   // work.fixed_dt.  Enqueued on the engine's stream.

@@ -1283,8 +1283,9 @@ cudaError_t Engine::launch_stage(const Stage& st, const double* const* in, const
                                  double* const* out, bool first_stage_of_step, int latch_mode, bool full, cudaEvent_t* ev) {
   const int b = blk_[2];
   const int lm = first_stage_of_step ? latch_mode : 0;
-  // a stage that overwrites its own input leaves the full interface values now
-  // (refresh_slots could not make them later)
+  // a last stage that overwrites its own input (Euler) leaves the full interface
+  // values now: refresh_slots could not make them later.  Inner stages in buffer 1
+  // (SSPRK3's second) take this form too, although the next one replaces the values.
   const bool slots = full || in[0] == out[0];
   // (the input's partially-wet cells are listed: by the update before, or ensure_list)
   if (ev) {

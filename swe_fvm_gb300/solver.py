@@ -352,7 +352,7 @@ class SpaceDisc:
 
     def set_bathymetry(self, z) -> None:
         """Replaces the node bathymetry (N values, the caller's node order):
-        the mesh records are recomputed and re-uploaded in place."""
+        the mesh records that depend on it are recomputed on the device, in place."""
         a = np.ascontiguousarray(z, dtype=np.float64).reshape(self.num_nodes)
         self._check(_lib.load().swe_set_bathymetry(self.ctx, a.ctypes.data))
 
